@@ -288,7 +288,9 @@ int scafes_gpu_set_border_time_basis(scafes_handle* h, double t_center,
 /* Advances the unknown field by n_steps time steps (one step = the update
  * phase of one iteration of iterateOverTime, src/ScaFES_Problem.hpp:
  * 2596-2603, including the border pass and the old/new swap).  Asynchronous
- * on the handle's stream. */
+ * on the handle's stream.  With the default tile (cfg.tile 0) and no depth
+ * set, several steps of a small grid, or of any grid with a rule-table
+ * border, run as one cooperative launch (same results bit for bit). */
 int scafes_gpu_step(scafes_handle* h, int n_steps);
 
 /* Copies the current iterate (or another slot) back to the host; n as for
@@ -325,7 +327,8 @@ int scafes_gpu_autotune(scafes_handle* h, int n_steps, int* chosen,
  * intermediate step on a one-node halo in shared memory, so the field is
  * read and written once per two steps; same results bit for bit).  Depth 2
  * applies to Dirichlet problems with one border layer and no F_B; other
- * problems, and an odd last step, run depth 1.  Default 1;
+ * problems, and an odd last step, run depth 1.  Setting a depth also fixes
+ * one launch per pass.  Default 1;
  * scafes_gpu_autotune keeps depth 2 when it is faster.  _temporal_depth
  * gives the depth that scafes_gpu_step will use. */
 int scafes_gpu_set_temporal_depth(scafes_handle* h, int depth);
@@ -345,7 +348,8 @@ int scafes_gpu_err_linf(scafes_handle* h, double* err, double* max_ref);
  * on the handle's stream by the last scafes_gpu_step call. */
 int scafes_gpu_last_step_ms(const scafes_handle* h, float* ms);
 
-/* Number of kernel launches issued by the last scafes_gpu_step call. */
+/* Number of kernel launches issued by the last scafes_gpu_step call (one per
+ * pass over the grid, or one per 1024 steps of a one-launch loop). */
 int scafes_gpu_last_step_launches(const scafes_handle* h, int* launches);
 
 const char* scafes_gpu_last_error(const scafes_handle* h);

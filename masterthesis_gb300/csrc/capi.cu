@@ -35,6 +35,11 @@ int fail(std::string* where, int code, const char* fmt, ...) {
     return code;
 }
 
+// Steps per launch of the one-launch time loop: the step times of one
+// launch (48 bytes each) stay within the 64 KB that a copy from pageable
+// memory takes without waiting for the stream.
+constexpr int kLoopSteps = 1024;
+
 // Bytes of host staging used for precision conversions (per slab).
 constexpr size_t kStageBytes = 64ull << 20;
 
@@ -54,6 +59,12 @@ struct scafes_handle {
     scafes_border_node_rule* nodes = nullptr;  // per-node border rules (SCAFES_BORDER_NODES)
     int tile = 0;                         // tile variant of the sweep
     int depth = 1;                        // temporal blocking depth (1 or 2)
+    bool schedule_set = false;            // the caller chose the tile or the depth: one launch per pass
+    // One-launch time loop of small grids: the grid barrier's counter and
+    // the times of up to kLoopSteps steps (made on first use).
+    unsigned* arrivals = nullptr;
+    StepTimes* times = nullptr;
+    int sms = 1;
     CUtensorMap tm_tb[2];                 // TMA descriptors of u[0], u[1] for depth-2 passes
     bool tm_tb_ok[2] = {};
     int* status = nullptr;                // device status word of the kernels
@@ -176,6 +187,8 @@ extern "C" void scafes_gpu_destroy(scafes_handle* h) {
     cudaFree(h->stage);
     cudaFree(h->table);
     cudaFree(h->nodes);
+    cudaFree(h->arrivals);
+    cudaFree(h->times);
     cudaFree(h->snap_dev);
     for (int i = 0; i < 2; ++i) {
         if (h->snap_host[i]) cudaFreeHost(h->snap_host[i]);
@@ -233,6 +246,8 @@ extern "C" int scafes_gpu_create(const scafes_cfg* cfg, scafes_handle** out) {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     h->red_blocks = sms * 4;
+    h->sms = sms;
+    h->schedule_set = cfg->tile > 0;
     if ((e = cudaMalloc(&h->red, sizeof(double) * 2 * (h->red_blocks + 1))) != cudaSuccess)
         return bail(SCAFES_ERR_NOMEM, "cudaMalloc(scratch)", e);
     if ((e = cudaMallocHost(&h->red_host, sizeof(double) * 2)) != cudaSuccess)
@@ -515,7 +530,69 @@ static const CUtensorMap* tb_map(scafes_handle* h, int buf) {
     return &h->tm_tb[buf];
 }
 
-static int step_impl(scafes_handle* h, int n_steps, int tile, bool timed, int depth) {
+// Whether the steps run as one-launch time loops: a small grid, the default
+// schedule, several steps, and not under stream capture (the step times are
+// copied from host memory that a replay would find gone).
+static bool takes_loop(scafes_handle* h, const Star7Launch& a, int n_steps) {
+    if (h->schedule_set || n_steps < 3) return false;
+    if ((long long)n_nodes(h) > star7_loop_max_nodes(a)) return false;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(h->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+}
+
+// time(t), time(t+1) and the mirror correction of the step from iterate t.
+static void step_times(const scafes_handle* h, int t, double& t_old, double& t_new, double& corr) {
+    t_old = h->cfg.t_start + t * h->cfg.tau;
+    t_new = h->cfg.t_start + (t + 1) * h->cfg.tau;
+    corr = ldexp(1.0, t);  // 2^(t_new - 1)
+}
+
+// Runs the steps as one-launch loops; *done counts them (fewer than n_steps,
+// and h->schedule_set from then on, where the device cannot hold the loop's
+// CTAs at once).
+static int loop_steps(scafes_handle* h, const Star7Launch& a, int n_steps, int* done, int* launches) {
+    const bool timed = a.fb || a.gb || a.border == SCAFES_BORDER_TABLE || a.border == SCAFES_BORDER_MIRROR_POW2;
+    if (!h->arrivals) CUDA_TRY(h, cudaMalloc(&h->arrivals, sizeof(unsigned)));
+    if (timed && !h->times) CUDA_TRY(h, cudaMalloc(&h->times, sizeof(StepTimes) * kLoopSteps));
+    std::vector<StepTimes> st;
+    Star7Loop q;
+    q.step = a;
+    q.u[0] = h->u[0];
+    q.u[1] = h->u[1];
+    q.times = timed ? h->times : nullptr;
+    q.arrivals = h->arrivals;
+    q.c0 = h->fld[SCAFES_FIELD_C0];
+    q.ca = h->fld[SCAFES_FIELD_CA];
+    q.sms = h->sms;
+    for (*done = 0; *done < n_steps; *done += q.n_steps) {
+        q.first = h->cur;
+        q.n_steps = n_steps - *done < kLoopSteps ? n_steps - *done : kLoopSteps;
+        if (timed) {
+            st.resize(q.n_steps);
+            for (int i = 0; i < q.n_steps; ++i) {
+                double t_old, t_new, corr;
+                step_times(h, h->t + i, t_old, t_new, corr);
+                st[i] = StepTimes{make_split(t_old), make_split(t_new), make_split(corr)};
+            }
+            CUDA_TRY(h, cudaMemcpyAsync(h->times, st.data(), sizeof(StepTimes) * st.size(), cudaMemcpyHostToDevice,
+                                        h->stream));
+        }
+        const cudaError_t e = launch_star7_loop(q, h->stream);
+        if (e == cudaErrorCooperativeLaunchTooLarge) {
+            cudaGetLastError();
+            h->schedule_set = true;
+            return SCAFES_OK;
+        }
+        if (e != cudaSuccess)
+            return fail(&h->err, SCAFES_ERR_CUDA, "scafes_gpu_step: launch failed: %s", cudaGetErrorString(e));
+        h->cur ^= q.n_steps & 1;
+        h->t += q.n_steps;
+        ++*launches;
+    }
+    return SCAFES_OK;
+}
+
+static int step_impl(scafes_handle* h, int n_steps, int tile, bool timed, int depth, bool loop = false) {
     if (h->L.nl != 1) tile = STAR7_MULTI_LAYER_TILE;  // the only variant built for several layers
     Star7Launch a;
     a.precision = h->cfg.precision;
@@ -590,14 +667,18 @@ static int step_impl(scafes_handle* h, int n_steps, int tile, bool timed, int de
     if (timed) CUDA_TRY(h, cudaEventRecord(h->ev0, h->stream));
     a.status = h->status;
     int launches = 0;
-    for (int s = 0; s < n_steps;) {
+    int first = 0;
+    if (loop && takes_loop(h, a, n_steps)) {
+        const int rc = loop_steps(h, a, n_steps, &first, &launches);
+        if (rc != SCAFES_OK) return rc;
+    }
+    for (int s = first; s < n_steps;) {
         a.tm_uo = &h->tm[h->cur][tile];
         a.uo = h->u[h->cur];
         a.un = h->u[h->cur ^ 1];
-        a.time_old = h->cfg.t_start + h->t * h->cfg.tau;          // time(t)
-        a.time_new = h->cfg.t_start + (h->t + 1) * h->cfg.tau;    // time(t+1)
-        a.time_new2 = h->cfg.t_start + (h->t + 2) * h->cfg.tau;   // time(t+2)
-        a.mirror_corr = ldexp(1.0, h->t);                          // 2^(t_new - 1)
+        double corr2;
+        step_times(h, h->t + 1, a.time_new, a.time_new2, corr2);  // time(t+1), time(t+2)
+        step_times(h, h->t, a.time_old, a.time_new, a.mirror_corr);
         const int adv = (tb && n_steps - s >= 2) ? 2 : 1;
         a.tm_tb = adv == 2 ? &h->tm_tb[h->cur] : nullptr;
         cudaError_t e = adv == 2 ? launch_star7_tb(a, h->stream) : launch_star7(a, h->stream);
@@ -629,6 +710,7 @@ extern "C" int scafes_gpu_set_temporal_depth(scafes_handle* h, int depth) {
     if (depth != 1 && depth != 2)
         return fail(&h->err, SCAFES_ERR_ARG, "scafes_gpu_set_temporal_depth: depth %d (1 or 2)", depth);
     h->depth = depth;
+    h->schedule_set = true;
     return SCAFES_OK;
 }
 
@@ -793,7 +875,7 @@ extern "C" int scafes_gpu_step(scafes_handle* h, int n_steps) {
     if (n_steps < 0) return fail(&h->err, SCAFES_ERR_ARG, "scafes_gpu_step: n_steps=%d < 0", n_steps);
     if (!h->uploaded)
         return fail(&h->err, SCAFES_ERR_STATE, "scafes_gpu_step: upload the unknown field first");
-    return step_impl(h, n_steps, h->tile, true, h->depth);
+    return step_impl(h, n_steps, h->tile, true, h->depth, true);
 }
 
 // ---- snapshots ----------------------------------------------------------------
@@ -897,11 +979,11 @@ extern "C" int scafes_gpu_step_snapshots(scafes_handle* h, int n_steps, int inte
     for (long long t = t0 + 1; t <= t1 && rc == SCAFES_OK; ++t) {
         const bool at = (interval > 0 && t % interval == 0) || (t == t1 && (flags & SCAFES_SNAP_END));
         if (!at) continue;
-        rc = step_impl(h, (int)(t - done), h->tile, false, h->depth);
+        rc = step_impl(h, (int)(t - done), h->tile, false, h->depth, true);
         done = t;
         if (rc == SCAFES_OK) rc = snap(t);
     }
-    if (rc == SCAFES_OK && done < t1) rc = step_impl(h, (int)(t1 - done), h->tile, false, h->depth);
+    if (rc == SCAFES_OK && done < t1) rc = step_impl(h, (int)(t1 - done), h->tile, false, h->depth, true);
     if (rc == SCAFES_OK) {
         cudaError_t e = cudaEventRecord(h->ev1, h->stream);
         if (e != cudaSuccess) rc = fail(&h->err, SCAFES_ERR_CUDA, "scafes_gpu_step_snapshots: %s", cudaGetErrorString(e));

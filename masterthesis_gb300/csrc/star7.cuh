@@ -141,6 +141,28 @@ void star7_tb_box(int precision, int* width, int* rows);
 // Whether a problem can take depth-2 passes.
 bool star7_tb_eligible(const Star7Launch& a);
 
+// The times of one step of a one-launch time loop.
+struct StepTimes {
+    Split t_old, t_new, corr;  // time(t), time(t+1), mirror correction
+};
+
+// n_steps time steps in one cooperative launch (star7_loop.cuh), for grids
+// of at most star7_loop_max_nodes nodes.  cudaErrorCooperativeLaunchTooLarge
+// when the CTAs do not fit the device at once (nothing ran).
+struct Star7Loop {
+    Star7Launch step;        // border, layout, coefficients, known fields, rules, status
+    void* u[2];              // both iterates
+    int first;               // the old iterate of the first step
+    int n_steps;
+    const StepTimes* times;  // device, n_steps entries; null when nothing reads the time
+    unsigned* arrivals;      // device, the barrier's counter
+    const void* c0;          // variable coefficients
+    const void* ca;
+    int sms;
+};
+cudaError_t launch_star7_loop(const Star7Loop& q, cudaStream_t stream);
+long long star7_loop_max_nodes(const Star7Launch& a);
+
 // Conversions between host-layout doubles (dense, x fastest) staged on the
 // device and the padded device layout of each precision.
 cudaError_t convert_to_device(int precision, const double* dense, void* field,

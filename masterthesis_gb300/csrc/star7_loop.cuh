@@ -1,0 +1,254 @@
+// The time loop of a small star7 problem in one cooperative launch.
+//
+// A sweep of a small grid by the tile engine (star7_tile.cuh) is a chain of
+// latencies -- launch, barrier set-up, the first TMA planes, one plane after
+// the other -- on a handful of CTAs: 8.2 us a step at 17 x 15 x 16, 17.4 us
+// with rule-table borders at 40 x 31 x 27, 10.3 us at 64^3, of which the
+// FP64 pipe needs 0.1, 0.5 and 1.7 us.  Here the grid is dealt out node by
+// node over all SMs and stays in L2: a thread loads its node's neighbours
+// (plain loads, L1 within a step), stores the new value, and one grid-wide
+// barrier (a counter in global memory) ends the step.  The inner nodes and
+// the border nodes are numbered separately, so a warp holds one kind and the
+// border rules (a chain of FP64 operations) run in full warps instead of in
+// one or two lanes of every warp at a face.  A step now takes 2.15, 3.5 and
+// 5.2 us on those three; of the 2.1 us of an almost empty step, most is the
+// round trips to L2 (neighbours, store and release, counter, acquire).  Two
+// warps per CTA and up to one CTA per SM: 1, 2 and 4 warps measure the same
+// within 2 %, 16 warps 20 % slower at 17 x 15 x 16.
+//
+// Every node takes the operations of the tile engine in the same order
+// (PolX::star / star_vc, table_rule, node_rule, mirror): same bits.
+// Co-residency, which the barrier needs, comes from the cooperative launch;
+// the barrier's wait is bounded like every other wait (status word, return).
+#pragma once
+
+#include <algorithm>
+
+#include "node_order.cuh"
+#include "star7_tile.cuh"
+
+namespace scafes {
+
+template <class T>
+struct LoopArgs {
+    T* u[2];                 // iterates; u[first] is the old one of the first step
+    int first, n_steps;
+    const T* fa;
+    const T* fb;
+    const T* ga;
+    const T* gb;
+    T gval;
+    const T* c0;             // variable coefficients
+    const T* ca;
+    Layout L;
+    NodeOrder o;
+    Star7Coeffs c;
+    const BorderTable* table;
+    const scafes_border_node_rule* nodes;
+    const StepTimes* times;  // n_steps entries, or null when nothing reads the time
+    uint32_t in_cta, bd_cta; // inner and border nodes per CTA
+    unsigned* arrivals;      // barrier counter, 0 at launch
+    int* status;
+};
+
+// Ends a step for the whole grid: returns false (status set) when the other
+// CTAs did not arrive in time.  The release of thread 0 after the block
+// barrier publishes the block's stores; its acquire makes the others' stores
+// visible to the block's loads after the second block barrier.
+__device__ __forceinline__ bool grid_barrier(unsigned* arrivals, unsigned target, int* status) {
+    bool ok = true;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrivals) : "memory");
+        unsigned v;
+        uint64_t t0 = 0;
+        for (unsigned polls = 0;; ++polls) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(arrivals) : "memory");
+            if ((int)(v - target) >= 0) break;
+            if ((polls & 255u) == 255u) {
+                const uint64_t t = global_timer_ns();
+                if (t0 == 0) t0 = t;
+                if (t - t0 > kWaitLimitNs) {
+                    ok = false;
+                    atomicExch(status, SCAFES_ERR_TIMEOUT);
+                    break;
+                }
+            }
+        }
+    }
+    return __syncthreads_and(ok);
+}
+
+constexpr int LOOP_MAX_THREADS = 1024;
+constexpr uint32_t LOOP_MIN_WARPS = 2;
+
+template <class P, int SRC, int BORDER, bool VC>
+__global__ void __launch_bounds__(LOOP_MAX_THREADS, 1)
+star7_loop(const __grid_constant__ LoopArgs<typename P::T> A) {
+    using T = typename P::T;
+    constexpr bool HAS_F = SRC != SRC_NONE;
+    constexpr bool has_fb = SRC == SRC_AB;
+    if (__syncthreads_or(threadIdx.x == 0 && *(volatile int*)A.status != 0)) return;
+    const Layout& L = A.L;
+    const long long py = L.pitch, pz = L.plane;
+    // This CTA's inner and border nodes; the border nodes start at a warp.
+    const uint32_t i0 = blockIdx.x * A.in_cta, i1 = min(i0 + A.in_cta, A.o.n_inner);
+    const uint32_t b0 = blockIdx.x * A.bd_cta, b1 = min(b0 + A.bd_cta, A.o.n_border);
+    const uint32_t ni = i1 > i0 ? i1 - i0 : 0, nb = b1 > b0 ? b1 - b0 : 0;
+    const uint32_t split = (ni + 31) & ~31u;
+    TileJob<T> J{nullptr, nullptr, nullptr, A.fa, A.fb, A.ga, A.gb, A.gval, L};
+    J.table = A.table;
+    J.nodes = A.nodes;
+    for (int s = 0; s < A.n_steps; ++s) {
+        const T* uo = A.u[(A.first + s) & 1];
+        T* un = A.u[(A.first + s + 1) & 1];
+        if (A.times) {
+            J.time_old = A.times[s].t_old;
+            J.time_new = A.times[s].t_new;
+            J.corr = A.times[s].corr;
+        }
+        for (uint32_t j = threadIdx.x; j < split + nb; j += blockDim.x) {
+            int x, y, z;
+            if (j < split) {
+                if (j >= ni) continue;
+                inner_node(A.o, i0 + j, x, y, z);
+                const long long o = L.idx(x, y, z);
+                const T w = uo[o - 1], e = uo[o + 1], sn = uo[o - py], n = uo[o + py], b = uo[o - pz], t = uo[o + pz];
+                const T u = uo[o];
+                T f = P::zero();
+                if (HAS_F) f = P::src(A.fa[o], has_fb ? A.fb[o] : P::zero(), J.time_old, has_fb);
+                if constexpr (VC)
+                    un[o] = P::template star_vc<HAS_F>(A.c, u, w, e, sn, n, b, t, f, A.c0[o], A.ca[o]);
+                else
+                    un[o] = P::template star<HAS_F>(A.c, u, w, e, sn, n, b, t, f);
+            } else {
+                border_node(A.o, b0 + (j - split), x, y, z);
+                const long long o = L.idx(x, y, z);
+                T v;
+                if constexpr (BORDER == SCAFES_BORDER_DIRICHLET) {
+                    v = A.ga ? A.ga[o] : A.gval;
+                    if (A.gb) v = P::src(v, A.gb[o], J.time_new, true);
+                } else {
+                    // A neighbour outside the grid reads 0, as from the TMA halo.
+                    const T u = uo[o];
+                    const T w = x > 0 ? uo[o - 1] : P::zero(), e = x < L.nx - 1 ? uo[o + 1] : P::zero();
+                    const T sn = y > 0 ? uo[o - py] : P::zero(), n = y < L.ny - 1 ? uo[o + py] : P::zero();
+                    const T b = z > 0 ? uo[o - pz] : P::zero(), t = z < L.nz - 1 ? uo[o + pz] : P::zero();
+                    if constexpr (BORDER == SCAFES_BORDER_NODES) {
+                        v = node_rule<P>(J, x, y, z, u, w, e, sn, n, b, t);
+                    } else if constexpr (BORDER == SCAFES_BORDER_TABLE) {
+                        const int mask = (x == 0) | ((x == L.nx - 1) << 1) | ((y == 0) << 2) |
+                                         ((y == L.ny - 1) << 3) | ((z == 0) << 4) | ((z == L.nz - 1) << 5);
+                        v = table_rule<P, HAS_F, has_fb>(J, mask, o, u, w, e, sn, n, b, t);
+                    } else {
+                        T opp;
+                        bool minus;
+                        if (z == L.nz - 1)      { opp = b; minus = true; }
+                        else if (z == 0)        { opp = t; minus = false; }
+                        else if (y == L.ny - 1) { opp = sn; minus = true; }
+                        else if (y == 0)        { opp = n; minus = false; }
+                        else if (x == L.nx - 1) { opp = w; minus = true; }
+                        else                    { opp = e; minus = false; }
+                        v = P::mirror(u, opp, minus ? negated(J.corr) : J.corr);
+                    }
+                }
+                un[o] = v;
+            }
+        }
+        if (s + 1 < A.n_steps && !grid_barrier(A.arrivals, (unsigned)(s + 1) * gridDim.x, A.status)) return;
+    }
+}
+
+// ---- host side ---------------------------------------------------------------
+
+template <class T>
+static T loop_elem(double d) {
+    if constexpr (std::is_same<T, float2>::value) {
+        const f2 p = split_double(d);
+        return make_float2(p.hi, p.lo);
+    } else {
+        return (T)d;
+    }
+}
+
+template <class P, int SRC, int BORDER, bool VC>
+static cudaError_t launch_loop_typed(const Star7Loop& q, cudaStream_t stream) {
+    using T = typename P::T;
+    const Star7Launch& a = q.step;
+    LoopArgs<T> A;
+    A.u[0] = (T*)q.u[0];
+    A.u[1] = (T*)q.u[1];
+    A.first = q.first;
+    A.n_steps = q.n_steps;
+    A.fa = (const T*)a.fa;
+    A.fb = (const T*)a.fb;
+    A.ga = (const T*)a.ga;
+    A.gb = (const T*)a.gb;
+    A.gval = loop_elem<T>(a.gconst);
+    A.c0 = (const T*)q.c0;
+    A.ca = (const T*)q.ca;
+    A.L = a.L;
+    A.o = make_node_order(a.L.nx, a.L.ny, a.L.nz, a.L.nl);
+    A.c = a.c;
+    A.table = a.table;
+    A.nodes = a.nodes;
+    A.times = q.times;
+    A.arrivals = q.arrivals;
+    A.status = a.status;
+    // Two warps per CTA at least: fewer CTAs make the barrier cheaper, more
+    // spread the FP64 pipe's work; all SMs from 2 * 32 * SMs nodes on.
+    const uint32_t wi = (A.o.n_inner + 31) / 32, wb = (A.o.n_border + 31) / 32;
+    const uint32_t ctas = std::max(1u, std::min((uint32_t)q.sms, (wi + wb) / LOOP_MIN_WARPS));
+    A.in_cta = (A.o.n_inner + ctas - 1) / ctas;
+    A.bd_cta = (A.o.n_border + ctas - 1) / ctas;
+    const uint32_t want = ((A.in_cta + 31) / 32 + (A.bd_cta + 31) / 32) * 32;
+    const uint32_t rounds = (want + LOOP_MAX_THREADS - 1) / LOOP_MAX_THREADS;
+    const uint32_t threads = ((want / 32 + rounds - 1) / rounds) * 32;
+    cudaError_t e = cudaMemsetAsync(q.arrivals, 0, sizeof(unsigned), stream);
+    if (e != cudaSuccess) return e;
+    void* args[] = {&A};
+    e = cudaLaunchCooperativeKernel((const void*)star7_loop<P, SRC, BORDER, VC>, dim3(ctas), dim3(threads), args, 0,
+                                    stream);
+    return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+template <class P, int BORDER>
+static cudaError_t launch_loop_src(const Star7Loop& q, cudaStream_t stream) {
+    const Star7Launch& a = q.step;
+    if (a.fa == nullptr || a.c.cf == 0.0) return launch_loop_typed<P, SRC_NONE, BORDER, false>(q, stream);
+    if (a.fb == nullptr) return launch_loop_typed<P, SRC_A, BORDER, false>(q, stream);
+    return launch_loop_typed<P, SRC_AB, BORDER, false>(q, stream);
+}
+
+template <class P, int BORDER>
+static cudaError_t launch_loop_vc(const Star7Loop& q, cudaStream_t stream) {
+    if constexpr (std::is_same<P, PolF32x2>::value) {
+        return cudaErrorInvalidValue;
+    } else {
+        const Star7Launch& a = q.step;
+        if (a.fb != nullptr) return cudaErrorInvalidValue;
+        if (a.fa == nullptr || a.c.cf == 0.0) return launch_loop_typed<P, SRC_NONE, BORDER, true>(q, stream);
+        return launch_loop_typed<P, SRC_A, BORDER, true>(q, stream);
+    }
+}
+
+template <class P>
+cudaError_t launch_loop_prec(const Star7Loop& q, cudaStream_t stream) {
+    const Star7Launch& a = q.step;
+    if (a.vc) {
+        switch (a.border) {
+            case SCAFES_BORDER_DIRICHLET: return launch_loop_vc<P, SCAFES_BORDER_DIRICHLET>(q, stream);
+            case SCAFES_BORDER_TABLE: return launch_loop_vc<P, SCAFES_BORDER_TABLE>(q, stream);
+            case SCAFES_BORDER_NODES: return launch_loop_vc<P, SCAFES_BORDER_NODES>(q, stream);
+            default: return cudaErrorInvalidValue;
+        }
+    }
+    switch (a.border) {
+        case SCAFES_BORDER_DIRICHLET: return launch_loop_src<P, SCAFES_BORDER_DIRICHLET>(q, stream);
+        case SCAFES_BORDER_MIRROR_POW2: return launch_loop_src<P, SCAFES_BORDER_MIRROR_POW2>(q, stream);
+        case SCAFES_BORDER_TABLE: return launch_loop_src<P, SCAFES_BORDER_TABLE>(q, stream);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+}  // namespace scafes

@@ -86,6 +86,42 @@ cudaError_t launch_star7_tb_prepare(int precision) {
     }
 }
 
+cudaError_t launch_star7_loop_f64(const Star7Loop& q, cudaStream_t stream);
+cudaError_t launch_star7_loop_f32(const Star7Loop& q, cudaStream_t stream);
+cudaError_t launch_star7_loop_f32x2(const Star7Loop& q, cudaStream_t stream);
+
+// Largest grid whose steps run faster as a one-launch loop than as tile
+// sweeps (both measured on cubes, us per step, loop / sweeps):
+//   rule-table border: at every size; the sweeps evaluate the rules in one or
+//     two lanes of every warp at a face (f64 64^3 7.5 / 26, 448^3 1210 / 1908;
+//     f32 448^3 584 / 1462; pairs 448^3 781 / 1941);
+//   FP64, bound by the FP64 pipe in both forms: 96^3 12 / 18, 201 x 181 x 163
+//     61 / 78, 256^3 171 / 176, 320^3 320 / 315; with node coefficients 96^3
+//     12 / 31, 256^3 227 / 234, 320^3 424 / 411;
+//   FP32 and pairs: while the iterates and the source (and the coefficients)
+//     stay in the 126 MB L2, since the loop reads neighbours through L1 only:
+//     f32 201 x 181 x 163 20 / 23, 224^3 (90 MB) 35 / 34.5, with a source
+//     (135 MB) 52 / 39; pairs 201 x 181 x 163 (106 MB) 32 / 35, 224^3 (180
+//     MB) 75 / 55.  Node coefficients and rules: f32 224^3 69 / 85, 256^3
+//     106 / 96.
+long long star7_loop_max_nodes(const Star7Launch& a) {
+    const long long all = (1LL << 31) - 1;  // node numbers are 32-bit
+    if (a.border == SCAFES_BORDER_TABLE) return all;
+    if (a.precision == SCAFES_PREC_F64) return 256LL * 256 * 256;
+    if (a.vc) return 224LL * 224 * 224;
+    const int fields = 2 + (a.fa ? 1 : 0) + (a.fb ? 1 : 0);
+    return 100000000LL / (fields * (long long)element_size(a.precision));
+}
+
+cudaError_t launch_star7_loop(const Star7Loop& q, cudaStream_t stream) {
+    switch (q.step.precision) {
+        case SCAFES_PREC_F64: return launch_star7_loop_f64(q, stream);
+        case SCAFES_PREC_F32: return launch_star7_loop_f32(q, stream);
+        case SCAFES_PREC_F32X2: return launch_star7_loop_f32x2(q, stream);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
 cudaError_t launch_star7(const Star7Launch& a, cudaStream_t stream) {
     switch (a.precision) {
         case SCAFES_PREC_F64: return launch_star7_f64(a, stream);
