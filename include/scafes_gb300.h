@@ -181,9 +181,10 @@ typedef struct scafes_cfg {
     int precision;           /* enum scafes_precision */
     int border;              /* enum scafes_border */
     int tile;                /* sweep tile variant 1..4 (see
-                                scafes_gpu_autotune), 0 = default: 1 for
-                                FP64, else 3 on grids of at least 256 x 256
-                                columns and 1 below */
+                                scafes_gpu_autotune), 0 = the default
+                                schedule: one-launch loops on small grids, a
+                                sweep by plain loads for FP64, rule tables
+                                and border layers, a tile for the others */
     double c0;               /* centre coefficient */
     double cp[3];            /* pair coefficient per axis */
     double cf;               /* source coefficient (0 disables F) */
@@ -289,8 +290,8 @@ int scafes_gpu_set_border_time_basis(scafes_handle* h, double t_center,
  * phase of one iteration of iterateOverTime, src/ScaFES_Problem.hpp:
  * 2596-2603, including the border pass and the old/new swap).  Asynchronous
  * on the handle's stream.  With the default tile (cfg.tile 0) and no depth
- * set, several steps of a small grid, or of any grid with a rule-table
- * border, run as one cooperative launch (same results bit for bit). */
+ * set, several steps of a small grid run as one cooperative launch (same
+ * results bit for bit). */
 int scafes_gpu_step(scafes_handle* h, int n_steps);
 
 /* Copies the current iterate (or another slot) back to the host; n as for
@@ -314,7 +315,8 @@ int scafes_gpu_synchronize(scafes_handle* h);
  * n_steps sweeps with each tile variant of the sweep kernel (32 x BY CTA
  * tile, R rows per thread) on the uploaded problem, keeps the fastest for
  * later scafes_gpu_step calls and returns it (1-based) in *chosen and the
- * per-variant ms per step in ms_per_tile[4] (may be NULL); then times
+ * per-variant ms per step in ms_per_tile[4] (may be NULL); a sweep by plain
+ * loads is timed too and takes the tile's place if it is faster; then times
  * temporal blocking depth 2 where the problem allows it and keeps it if it
  * is faster per step (scafes_gpu_temporal_depth).  The iterate and the step
  * counter are restored afterwards.  Allocates one temporary copy of the

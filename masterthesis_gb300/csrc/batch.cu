@@ -675,10 +675,7 @@ extern "C" int scafes_batch_step_looped(scafes_batch* b, int n_steps) {
             Star7Launch a;
             a.precision = b->precision;
             a.border = SCAFES_BORDER_DIRICHLET;
-            a.tile = star7_default_tile(I.L, b->precision);
             a.L = I.L;
-            a.tm_uo = &b->hmaps[((size_t)i * 3 + b->cur) * STAR7_NUM_TILES + a.tile];
-            a.tm_f = &b->hmaps[((size_t)i * 3 + 2) * STAR7_NUM_TILES + a.tile];
             a.table = nullptr;
             a.status = b->status;
             a.uo = (char*)b->pool + (size_t)I.off_u[b->cur] * b->esz;
@@ -690,6 +687,12 @@ extern "C" int scafes_batch_step_looped(scafes_batch* b, int n_steps) {
             a.gconst = I.gconst;
             a.c = I.c;
             a.time_old = a.time_new = a.mirror_corr = 0.0;
+            a.tile = star7_default_tile(a);
+            a.tm_uo = a.tm_f = nullptr;
+            if (a.tile != STAR7_MARCH) {
+                a.tm_uo = &b->hmaps[((size_t)i * 3 + b->cur) * STAR7_NUM_TILES + a.tile];
+                a.tm_f = &b->hmaps[((size_t)i * 3 + 2) * STAR7_NUM_TILES + a.tile];
+            }
             cudaError_t e = launch_star7(a, b->stream);
             if (e != cudaSuccess)
                 return bfail(b, SCAFES_ERR_CUDA, "scafes_batch_step_looped: %s", cudaGetErrorString(e));

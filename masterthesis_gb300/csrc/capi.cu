@@ -57,7 +57,7 @@ struct scafes_handle {
     CUtensorMap tmc[2][STAR7_NUM_TILES];  // TMA descriptors of C0 and CA (box 32 x BY) per tile
     bool tmc_ok[2][STAR7_NUM_TILES] = {};
     scafes_border_node_rule* nodes = nullptr;  // per-node border rules (SCAFES_BORDER_NODES)
-    int tile = 0;                         // tile variant of the sweep
+    int tile = -1;                        // schedule of the sweep (tile variant or STAR7_MARCH), -1 the default
     int depth = 1;                        // temporal blocking depth (1 or 2)
     bool schedule_set = false;            // the caller chose the tile or the depth: one launch per pass
     // One-launch time loop of small grids: the grid barrier's counter and
@@ -235,7 +235,7 @@ extern "C" int scafes_gpu_create(const scafes_cfg* cfg, scafes_handle** out) {
         if ((e = cudaMemsetAsync(h->u[i], 0, bytes, h->stream)) != cudaSuccess)
             return bail(SCAFES_ERR_CUDA, "cudaMemset(u)", e);
     }
-    h->tile = cfg->tile > 0 ? cfg->tile - 1 : star7_default_tile(h->L, cfg->precision);
+    h->tile = cfg->tile - 1;
     if ((e = cudaMalloc(&h->status, sizeof(int))) != cudaSuccess)
         return bail(SCAFES_ERR_NOMEM, "cudaMalloc(status)", e);
     if ((e = cudaMemsetAsync(h->status, 0, sizeof(int), h->stream)) != cudaSuccess)
@@ -561,8 +561,6 @@ static int loop_steps(scafes_handle* h, const Star7Launch& a, int n_steps, int* 
     q.u[1] = h->u[1];
     q.times = timed ? h->times : nullptr;
     q.arrivals = h->arrivals;
-    q.c0 = h->fld[SCAFES_FIELD_C0];
-    q.ca = h->fld[SCAFES_FIELD_CA];
     q.sms = h->sms;
     for (*done = 0; *done < n_steps; *done += q.n_steps) {
         q.first = h->cur;
@@ -593,13 +591,9 @@ static int loop_steps(scafes_handle* h, const Star7Launch& a, int n_steps, int* 
 }
 
 static int step_impl(scafes_handle* h, int n_steps, int tile, bool timed, int depth, bool loop = false) {
-    if (h->L.nl != 1) tile = STAR7_MULTI_LAYER_TILE;  // the only variant built for several layers
     Star7Launch a;
     a.precision = h->cfg.precision;
     a.border = h->cfg.border;
-    a.tile = tile;
-    for (int b = 0; b < 2; ++b)
-        if (!tensor_map(h, b, tile)) return SCAFES_ERR_CUDA;
     a.L = h->L;
     a.fa = h->has[SCAFES_FIELD_F_A] ? h->fld[SCAFES_FIELD_F_A] : nullptr;
     a.fb = h->has[SCAFES_FIELD_F_B] ? h->fld[SCAFES_FIELD_F_B] : nullptr;
@@ -608,8 +602,17 @@ static int step_impl(scafes_handle* h, int n_steps, int tile, bool timed, int de
     a.gconst = 0.0;
     a.c = make_star7_coeffs(h->cfg.c0, h->cfg.cp, h->cfg.cf);
     a.table = h->table;
-    a.tm_f = nullptr;
-    if (a.fa && !a.fb && h->cfg.cf != 0.0 && !(a.tm_f = source_map(h, tile))) return SCAFES_ERR_CUDA;
+    a.vc = var_coeffs(h);
+    a.c0 = h->fld[SCAFES_FIELD_C0];
+    a.ca = h->fld[SCAFES_FIELD_CA];
+    if (tile < 0) tile = star7_default_tile(a);
+    if (h->L.nl != 1 && tile != STAR7_MARCH) tile = STAR7_MULTI_LAYER_TILE;  // the only tile built for several layers
+    a.tile = tile;
+    const bool tma = tile != STAR7_MARCH;
+    a.tm_uo = a.tm_f = nullptr;
+    for (int b = 0; b < 2; ++b)
+        if (tma && !tensor_map(h, b, tile)) return SCAFES_ERR_CUDA;
+    if (tma && a.fa && !a.fb && h->cfg.cf != 0.0 && !(a.tm_f = source_map(h, tile))) return SCAFES_ERR_CUDA;
     if (!h->has[SCAFES_FIELD_F_A] && h->has[SCAFES_FIELD_F_B])
         return fail(&h->err, SCAFES_ERR_UNSUPPORTED,
                     "scafes_gpu_step: upload F_A (possibly zeros) when F_B is used");
@@ -627,7 +630,6 @@ static int step_impl(scafes_handle* h, int n_steps, int tile, bool timed, int de
             return fail(&h->err, SCAFES_ERR_STATE,
                         "scafes_gpu_step: a border rule reads the source F, but no F_A is uploaded or cf == 0");
     }
-    a.vc = var_coeffs(h);
     if (h->has[SCAFES_FIELD_C0] != h->has[SCAFES_FIELD_CA])
         return fail(&h->err, SCAFES_ERR_STATE,
                     "scafes_gpu_step: the variable-coefficient update needs both slots C0 and CA uploaded");
@@ -657,7 +659,7 @@ static int step_impl(scafes_handle* h, int n_steps, int tile, bool timed, int de
         if (h->cfg.border == SCAFES_BORDER_MIRROR_POW2)
             return fail(&h->err, SCAFES_ERR_UNSUPPORTED,
                         "scafes_gpu_step: the variable-coefficient update takes the Dirichlet, table or per-node border");
-        if (!(a.tm_c0 = coeff_map(h, 0, tile)) || !(a.tm_ca = coeff_map(h, 1, tile))) return SCAFES_ERR_CUDA;
+        if (tma && (!(a.tm_c0 = coeff_map(h, 0, tile)) || !(a.tm_ca = coeff_map(h, 1, tile)))) return SCAFES_ERR_CUDA;
     }
     a.tm_tb = nullptr;
     const bool tb = depth == 2 && star7_tb_eligible(a);
@@ -673,7 +675,7 @@ static int step_impl(scafes_handle* h, int n_steps, int tile, bool timed, int de
         if (rc != SCAFES_OK) return rc;
     }
     for (int s = first; s < n_steps;) {
-        a.tm_uo = &h->tm[h->cur][tile];
+        if (tma) a.tm_uo = &h->tm[h->cur][tile];
         a.uo = h->u[h->cur];
         a.un = h->u[h->cur ^ 1];
         double corr2;
@@ -1049,9 +1051,9 @@ extern "C" int scafes_gpu_autotune(scafes_handle* h, int n_steps, int* chosen, f
     CUDA_TRY(h, cudaMalloc(&save, bytes));
     const int t_save = h->t, cur_save = h->cur;
     cudaError_t e = cudaMemcpyAsync(save, h->u[h->cur], bytes, cudaMemcpyDeviceToDevice, h->stream);
-    int best = h->tile, rc = SCAFES_OK;
+    int best = 0, best_tile = 0, rc = SCAFES_OK;
     float best_ms = 0.f;
-    for (int tile = 0; tile < STAR7_NUM_TILES && e == cudaSuccess && rc == SCAFES_OK; ++tile) {
+    for (int tile = 0; tile <= STAR7_MARCH && e == cudaSuccess && rc == SCAFES_OK; ++tile) {
         rc = step_impl(h, 1, tile, false, 1);  // warm-up (and first-use setup)
         if (rc == SCAFES_OK) rc = step_impl(h, n_steps, tile, true, 1);
         float ms = 0.f;
@@ -1059,13 +1061,14 @@ extern "C" int scafes_gpu_autotune(scafes_handle* h, int n_steps, int* chosen, f
             e = cudaEventSynchronize(h->ev1);
             if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, h->ev0, h->ev1);
         }
-        if (ms_per_tile) ms_per_tile[tile] = ms / n_steps;
+        if (ms_per_tile && tile < STAR7_NUM_TILES) ms_per_tile[tile] = ms / n_steps;
         if (rc == SCAFES_OK && e == cudaSuccess && (tile == 0 || ms < best_ms)) {
             best_ms = ms;
             best = tile;
+            if (tile < STAR7_NUM_TILES) best_tile = tile;
         }
     }
-    // Temporal blocking: depth 2 (its own tile) against the best depth-1 tile.
+    // Temporal blocking: depth 2 (its own tile) against the best depth-1 schedule.
     int best_depth = 1;
     int dep = 0;
     const int n2 = n_steps + (n_steps & 1);
@@ -1099,7 +1102,7 @@ extern "C" int scafes_gpu_autotune(scafes_handle* h, int n_steps, int* chosen, f
     if (rc) return rc;
     h->tile = best;
     h->depth = best_depth;
-    if (chosen) *chosen = best + 1;
+    if (chosen) *chosen = best_tile + 1;
     return SCAFES_OK;
 }
 

@@ -15,6 +15,9 @@ constexpr int STAR7_NUM_TILES = 4;
 // The one tile variant built for more than one border layer; a launch with
 // L.nl != 1 must use it (its TMA descriptors are encoded for that tile).
 constexpr int STAR7_MULTI_LAYER_TILE = 1;
+// The schedule that no tile variant stands for: the sweep by plain loads
+// (star7_march.cuh), for any border, source and number of border layers.
+constexpr int STAR7_MARCH = STAR7_NUM_TILES;
 
 // Coefficients of u_new = c0*u + sum_p cp*(u_{p-}+u_{p+}) + cf*F, in double
 // and split into FP32 triples (hi + lo + lo2, ~72 bits) for the
@@ -58,9 +61,8 @@ __host__ __device__ inline Split negated(const Split& s) {
 int star7_box_width(int precision);
 // Height (rows) of the TMA box of tile variant `tile`.
 int star7_box_height(int tile);
-// Tile variant used when none is chosen: {8,1} for FP64; otherwise {32,4}
-// on large grids and {8,1} else.
-int star7_default_tile(const Layout& L, int precision);
+// Schedule used when none is chosen: a tile variant or STAR7_MARCH.
+int star7_default_tile(const struct Star7Launch& a);
 
 // Device block of a SCAFES_BORDER_TABLE problem: the rule of each border
 // class and the border field's higher time orders and time variable
@@ -97,7 +99,7 @@ __host__ __device__ inline long long border_node_index(const Layout& L, int x, i
 struct Star7Launch {
     int precision;        // enum scafes_precision
     int border;           // enum scafes_border
-    int tile;             // tile variant 0 .. STAR7_NUM_TILES-1
+    int tile;             // tile variant 0 .. STAR7_NUM_TILES-1, or STAR7_MARCH
     Layout L;
     const CUtensorMap* tm_uo;  // TMA descriptor of the old iterate
     const CUtensorMap* tm_f;   // TMA descriptor of F_A, box 32 x BY of the tile (F_A-only sources)
@@ -121,6 +123,8 @@ struct Star7Launch {
     bool vc = false;
     const CUtensorMap* tm_c0 = nullptr;
     const CUtensorMap* tm_ca = nullptr;
+    const void* c0 = nullptr;  // the fields themselves
+    const void* ca = nullptr;
     const scafes_border_node_rule* nodes = nullptr;  // SCAFES_BORDER_NODES rules
 };
 
@@ -156,8 +160,6 @@ struct Star7Loop {
     int n_steps;
     const StepTimes* times;  // device, n_steps entries; null when nothing reads the time
     unsigned* arrivals;      // device, the barrier's counter
-    const void* c0;          // variable coefficients
-    const void* ca;
     int sms;
 };
 cudaError_t launch_star7_loop(const Star7Loop& q, cudaStream_t stream);

@@ -25,7 +25,7 @@
 #include <algorithm>
 
 #include "node_order.cuh"
-#include "star7_tile.cuh"
+#include "star7_border.cuh"
 
 namespace scafes {
 
@@ -123,36 +123,7 @@ star7_loop(const __grid_constant__ LoopArgs<typename P::T> A) {
                     un[o] = P::template star<HAS_F>(A.c, u, w, e, sn, n, b, t, f);
             } else {
                 border_node(A.o, b0 + (j - split), x, y, z);
-                const long long o = L.idx(x, y, z);
-                T v;
-                if constexpr (BORDER == SCAFES_BORDER_DIRICHLET) {
-                    v = A.ga ? A.ga[o] : A.gval;
-                    if (A.gb) v = P::src(v, A.gb[o], J.time_new, true);
-                } else {
-                    // A neighbour outside the grid reads 0, as from the TMA halo.
-                    const T u = uo[o];
-                    const T w = x > 0 ? uo[o - 1] : P::zero(), e = x < L.nx - 1 ? uo[o + 1] : P::zero();
-                    const T sn = y > 0 ? uo[o - py] : P::zero(), n = y < L.ny - 1 ? uo[o + py] : P::zero();
-                    const T b = z > 0 ? uo[o - pz] : P::zero(), t = z < L.nz - 1 ? uo[o + pz] : P::zero();
-                    if constexpr (BORDER == SCAFES_BORDER_NODES) {
-                        v = node_rule<P>(J, x, y, z, u, w, e, sn, n, b, t);
-                    } else if constexpr (BORDER == SCAFES_BORDER_TABLE) {
-                        const int mask = (x == 0) | ((x == L.nx - 1) << 1) | ((y == 0) << 2) |
-                                         ((y == L.ny - 1) << 3) | ((z == 0) << 4) | ((z == L.nz - 1) << 5);
-                        v = table_rule<P, HAS_F, has_fb>(J, mask, o, u, w, e, sn, n, b, t);
-                    } else {
-                        T opp;
-                        bool minus;
-                        if (z == L.nz - 1)      { opp = b; minus = true; }
-                        else if (z == 0)        { opp = t; minus = false; }
-                        else if (y == L.ny - 1) { opp = sn; minus = true; }
-                        else if (y == 0)        { opp = n; minus = false; }
-                        else if (x == L.nx - 1) { opp = w; minus = true; }
-                        else                    { opp = e; minus = false; }
-                        v = P::mirror(u, opp, minus ? negated(J.corr) : J.corr);
-                    }
-                }
-                un[o] = v;
+                un[L.idx(x, y, z)] = border_value<P, SRC, BORDER>(J, uo, x, y, z);
             }
         }
         if (s + 1 < A.n_steps && !grid_barrier(A.arrivals, (unsigned)(s + 1) * gridDim.x, A.status)) return;
@@ -185,8 +156,8 @@ static cudaError_t launch_loop_typed(const Star7Loop& q, cudaStream_t stream) {
     A.ga = (const T*)a.ga;
     A.gb = (const T*)a.gb;
     A.gval = loop_elem<T>(a.gconst);
-    A.c0 = (const T*)q.c0;
-    A.ca = (const T*)q.ca;
+    A.c0 = (const T*)a.c0;
+    A.ca = (const T*)a.ca;
     A.L = a.L;
     A.o = make_node_order(a.L.nx, a.L.ny, a.L.nz, a.L.nl);
     A.c = a.c;

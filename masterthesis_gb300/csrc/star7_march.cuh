@@ -1,0 +1,235 @@
+// One time step by plain loads: a warp owns R rows of 32 columns and marches
+// z, with below, current and above in registers and the x and y neighbours
+// through L1 (which holds them from their own "above" loads a plane
+// earlier).  The border nodes are left to CTAs of their own at the front of
+// the grid, in full warps (star7_border.cuh); the marching threads compute
+// inner nodes only, so every border kind, source and layer count is one
+// kernel and no warp at a face runs a rule for one or two lanes.
+//
+// The FP64 sweep is bound by the FP64 pipe (16 clocks of an SM per warp
+// instruction, 4 per node) and by the integer sums; the tile engine
+// (star7_tile.cuh) spends as many instructions again on its ring -- barrier
+// waits, block barriers, addresses -- as on the node: 268 issued per 32
+// nodes against 175 here, which the memory path does not need, since FP64
+// asks it for 2 TB/s.  512^3: 1178 -> 1077 us (124.6 GLUP/s, FP64 pipe 82 %
+// busy, integer ALU 55 %); 256^3: 175 -> 145 us.  Six CTAs of 256 threads (40
+// registers, nothing spilled): 4, 5 and 8 CTAs measure 2 % to 0.2 % slower.
+// FP32 and pairs are bound by the memory path, where the tile engine's ring
+// keeps more bytes in flight (f32 400^3 89 against 123 us); they come here
+// with rule tables and several border layers only.
+#pragma once
+
+#include <algorithm>
+
+#include "node_order.cuh"
+#include "star7_border.cuh"
+
+namespace scafes {
+
+template <class T>
+struct MarchArgs {
+    const T* uo;
+    T* un;
+    const T* fa;
+    const T* fb;
+    const T* ga;
+    const T* gb;
+    T gval;
+    const T* c0;
+    const T* ca;
+    Layout L;
+    NodeOrder o;
+    Star7Coeffs c;
+    const BorderTable* table;
+    const scafes_border_node_rule* nodes;
+    StepTimes t;
+    uint32_t border_ctas;
+    FastDiv tx, txy;  // tiles along x, tiles of a layer
+    int zchunk;
+    const int* status;
+};
+
+constexpr int MARCH_Y = 8;  // warps of a CTA
+
+template <class P, int SRC, int BORDER, bool VC, int R, int MINB>
+__global__ void __launch_bounds__(32 * MARCH_Y, MINB)
+star7_march(const __grid_constant__ MarchArgs<typename P::T> A) {
+    using T = typename P::T;
+    constexpr bool HAS_F = SRC != SRC_NONE;
+    constexpr bool has_fb = SRC == SRC_AB;
+    const Layout& L = A.L;
+    if (*(const volatile int*)A.status != 0) return;  // an earlier sweep gave up
+    if (blockIdx.x < A.border_ctas) {
+        const uint32_t m = blockIdx.x * (32 * MARCH_Y) + threadIdx.x;
+        if (m >= A.o.n_border) return;
+        TileJob<T> J{nullptr, nullptr, nullptr, A.fa, A.fb, A.ga, A.gb, A.gval, L, A.t.t_old, A.t.t_new, A.t.corr};
+        J.table = A.table;
+        J.nodes = A.nodes;
+        int x, y, z;
+        border_node(A.o, m, x, y, z);
+        A.un[L.idx(x, y, z)] = border_value<P, SRC, BORDER>(J, A.uo, x, y, z);
+        return;
+    }
+    const uint32_t q = blockIdx.x - A.border_ctas;
+    const uint32_t k = fastdiv(q, A.txy), r = q - k * A.txy.d, j = fastdiv(r, A.tx);
+    const int x = (int)(r - j * A.tx.d) * 32 + (threadIdx.x & 31);
+    const int y = (int)(j * MARCH_Y + (threadIdx.x >> 5)) * R + L.nl;
+    if (x < L.nl || x >= L.nx - L.nl || y >= L.ny - L.nl) return;
+    const int z0 = (int)k * A.zchunk + L.nl, z1 = min(z0 + A.zchunk, L.nz - L.nl);
+    const long long py = L.pitch, pz = L.plane;
+    long long o = L.idx(x, y, z0);
+    const T* __restrict__ uo = A.uo;
+    T* __restrict__ un = A.un;
+    // Rows that are border rows are computed but not stored; a row beyond the
+    // grid reads the last one.
+    unsigned skip = 0u;
+    long long ro[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        ro[i] = (min(y + i, L.ny - 1) - y) * py;
+        if (y + i >= L.ny - L.nl) skip |= 1u << i;
+    }
+    const long long rn = (min(y + R, L.ny - 1) - y) * py;
+    T below[R], cur[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        below[i] = uo[o + ro[i] - pz];
+        cur[i] = uo[o + ro[i]];
+    }
+#pragma unroll 2
+    for (int z = z0; z < z1; ++z, o += pz) {
+        T above[R], w[R], e[R], f[R], v[R];
+        const T ym = uo[o - py], yp = uo[o + rn];
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            above[i] = uo[o + ro[i] + pz];
+            w[i] = uo[o + ro[i] - 1];
+            e[i] = uo[o + ro[i] + 1];
+            f[i] = P::zero();
+            if (HAS_F) f[i] = P::src(A.fa[o + ro[i]], has_fb ? A.fb[o + ro[i]] : P::zero(), A.t.t_old, has_fb);
+        }
+        if constexpr (VC) {
+            T c0[R], ca[R];
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                c0[i] = A.c0[o + ro[i]];
+                ca[i] = A.ca[o + ro[i]];
+            }
+            P::template star_vc_rows<HAS_F, R>(A.c, below, cur, above, ym, yp, w, e, f, c0, ca, 1, v, skip);
+        } else {
+            P::template star_rows<HAS_F, R>(A.c, below, cur, above, ym, yp, w, e, f, v, skip);
+        }
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+            if (R == 1 || !((skip >> i) & 1u)) un[o + i * py] = v[i];
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            below[i] = cur[i];
+            cur[i] = above[i];
+        }
+    }
+}
+
+// ---- host side ---------------------------------------------------------------
+
+template <class T>
+static T march_elem(double d) {
+    if constexpr (std::is_same<T, float2>::value) {
+        const f2 p = split_double(d);
+        return make_float2(p.hi, p.lo);
+    } else {
+        return (T)d;
+    }
+}
+
+// Rows per thread and resident CTAs: pairs work on two rows at once (the
+// paired FP32 instructions), the others on one.
+template <class P>
+constexpr int march_rows() {
+    return std::is_same<P, PolF32x2>::value ? 2 : 1;
+}
+template <class P>
+constexpr int march_ctas() {
+    return std::is_same<P, PolF32x2>::value ? 4 : 6;
+}
+
+template <class P, int SRC, int BORDER, bool VC>
+static cudaError_t launch_march_typed(const Star7Launch& a, cudaStream_t stream) {
+    using T = typename P::T;
+    constexpr int R = march_rows<P>();
+    MarchArgs<T> A;
+    A.uo = (const T*)a.uo;
+    A.un = (T*)a.un;
+    A.fa = (const T*)a.fa;
+    A.fb = (const T*)a.fb;
+    A.ga = (const T*)a.ga;
+    A.gb = (const T*)a.gb;
+    A.gval = march_elem<T>(a.gconst);
+    A.c0 = (const T*)a.c0;
+    A.ca = (const T*)a.ca;
+    A.L = a.L;
+    A.o = make_node_order(a.L.nx, a.L.ny, a.L.nz, a.L.nl);
+    A.c = a.c;
+    A.table = a.table;
+    A.nodes = a.nodes;
+    A.t = StepTimes{make_split(a.time_old), make_split(a.time_new), make_split(a.mirror_corr)};
+    A.status = a.status;
+    const int nl = a.L.nl, iy = a.L.ny - 2 * nl, iz = a.L.nz - 2 * nl;
+    A.border_ctas = (A.o.n_border + 32 * MARCH_Y - 1) / (32 * MARCH_Y);
+    // 8 planes per CTA (16 for pairs), 4 while that leaves under two rounds
+    // of resident CTAs: 256^3 f64 145, 150, 163 us with 8, 16, 32 planes;
+    // 160^3 40.4 with 4, 41.9 with 8; pairs 300 x 280 x 260 108, 104.5, 112
+    // with 8, 16, 32.
+    int sms = 1, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const long long tx = (a.L.nx + 31) / 32, ty = std::max(0, (iy + MARCH_Y * R - 1) / (MARCH_Y * R));
+    int zc = R == 2 ? 16 : 8;
+    while (zc > 4 && tx * ty * ((iz + zc - 1) / zc) < 12LL * sms) zc >>= 1;
+    const long long tz = std::max(0, (iz + zc - 1) / zc);
+    A.zchunk = zc;
+    A.tx = make_fastdiv((uint32_t)tx);
+    A.txy = make_fastdiv((uint32_t)std::max(1LL, tx * ty));
+    const long long ctas = A.border_ctas + (A.o.n_inner ? tx * ty * tz : 0);
+    if (ctas > 0x7fffffffLL) return cudaErrorInvalidValue;
+    star7_march<P, SRC, BORDER, VC, R, march_ctas<P>()><<<(unsigned)ctas, 32 * MARCH_Y, 0, stream>>>(A);
+    return cudaGetLastError();
+}
+
+template <class P, int BORDER>
+static cudaError_t launch_march_src(const Star7Launch& a, cudaStream_t stream) {
+    if (a.fa == nullptr || a.c.cf == 0.0) return launch_march_typed<P, SRC_NONE, BORDER, false>(a, stream);
+    if (a.fb == nullptr) return launch_march_typed<P, SRC_A, BORDER, false>(a, stream);
+    return launch_march_typed<P, SRC_AB, BORDER, false>(a, stream);
+}
+
+template <class P, int BORDER>
+static cudaError_t launch_march_vc(const Star7Launch& a, cudaStream_t stream) {
+    if constexpr (std::is_same<P, PolF32x2>::value) {
+        return cudaErrorInvalidValue;
+    } else {
+        if (a.fb != nullptr) return cudaErrorInvalidValue;
+        if (a.fa == nullptr || a.c.cf == 0.0) return launch_march_typed<P, SRC_NONE, BORDER, true>(a, stream);
+        return launch_march_typed<P, SRC_A, BORDER, true>(a, stream);
+    }
+}
+
+template <class P>
+cudaError_t launch_march_prec(const Star7Launch& a, cudaStream_t stream) {
+    if (a.vc) {
+        switch (a.border) {
+            case SCAFES_BORDER_DIRICHLET: return launch_march_vc<P, SCAFES_BORDER_DIRICHLET>(a, stream);
+            case SCAFES_BORDER_TABLE: return launch_march_vc<P, SCAFES_BORDER_TABLE>(a, stream);
+            case SCAFES_BORDER_NODES: return launch_march_vc<P, SCAFES_BORDER_NODES>(a, stream);
+            default: return cudaErrorInvalidValue;
+        }
+    }
+    switch (a.border) {
+        case SCAFES_BORDER_DIRICHLET: return launch_march_src<P, SCAFES_BORDER_DIRICHLET>(a, stream);
+        case SCAFES_BORDER_MIRROR_POW2: return launch_march_src<P, SCAFES_BORDER_MIRROR_POW2>(a, stream);
+        case SCAFES_BORDER_TABLE: return launch_march_src<P, SCAFES_BORDER_TABLE>(a, stream);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+}  // namespace scafes

@@ -39,13 +39,22 @@ int star7_box_height(int tile) {
     return kTiles[tile].by + 2;
 }
 
-int star7_default_tile(const Layout& L, int precision) {
-    // FP64: one row per thread (the integer-pipe sums want resident warps,
-    // not registers; the autotuner's choice at every size measured).  Else
-    // four rows per thread once the grid has enough tiles to fill the GPU.
-    if (precision == SCAFES_PREC_F64) return 0;
-    const long long cols = (long long)L.nx * L.ny;
-    return cols >= 256LL * 256LL ? 2 : 0;
+// Measured in us per step (cubes unless given):
+//   FP64: the march (star7_march.cuh) at every size;
+//   rule tables, several border layers: the march, whose border rules run in
+//     full warps (256^3 with a rule table: f64 226 against 500 with the best
+//     tile, f32 85 / 369, pairs 144 / 586);
+//   pairs: with a source the {32,4} tile (201 x 181 x 163: 40.5, {8,1} 41.9;
+//     300 x 280 x 260: 104.7, {16,4} 108.5), without one the {16,4} tile
+//     (256^3: 64.7, {32,4} 81.2);
+//   FP32: the {16,4} tile (400^3 89 - 94, {32,4} 94 - 95, {8,1} 154; with
+//     node coefficients 256^3 88, {32,4} 95, the march 96; 448^3 345, 354, 439);
+//   FP32 and pairs below 128 x 128 columns: the {8,1} tile, which has the
+//     most CTAs (several steps of these grids run as a one-launch loop).
+int star7_default_tile(const Star7Launch& a) {
+    if (a.precision == SCAFES_PREC_F64 || a.L.nl != 1 || a.border == SCAFES_BORDER_TABLE) return STAR7_MARCH;
+    if ((long long)a.L.nx * a.L.ny < 128LL * 128LL) return 0;
+    return a.precision == SCAFES_PREC_F32X2 && a.fa ? 2 : 3;
 }
 
 cudaError_t launch_star7_f64(const Star7Launch& a, cudaStream_t stream);
@@ -90,27 +99,22 @@ cudaError_t launch_star7_loop_f64(const Star7Loop& q, cudaStream_t stream);
 cudaError_t launch_star7_loop_f32(const Star7Loop& q, cudaStream_t stream);
 cudaError_t launch_star7_loop_f32x2(const Star7Loop& q, cudaStream_t stream);
 
-// Largest grid whose steps run faster as a one-launch loop than as tile
-// sweeps (both measured on cubes, us per step, loop / sweeps):
-//   rule-table border: at every size; the sweeps evaluate the rules in one or
-//     two lanes of every warp at a face (f64 64^3 7.5 / 26, 448^3 1210 / 1908;
-//     f32 448^3 584 / 1462; pairs 448^3 781 / 1941);
-//   FP64, bound by the FP64 pipe in both forms: 96^3 12 / 18, 201 x 181 x 163
-//     61 / 78, 256^3 171 / 176, 320^3 320 / 315; with node coefficients 96^3
-//     12 / 31, 256^3 227 / 234, 320^3 424 / 411;
+// Largest grid whose steps run faster as a one-launch loop than as sweeps
+// (both measured, us per step, loop / default sweep):
+//   FP64, and rule tables in any type: f64 96^3 11.4 / 14.4, 201 x 181 x 163
+//     60 / 64, 256^3 161 / 148; node coefficients 96^3 12 / 16, 201 x 181 x
+//     163 75 / 78, 256^3 221 / 178; rule table 96^3 16 / 21, 201 x 181 x 163
+//     95 / 98, 256^3 270 / 226; f32 rule table 201 x 181 x 163 40 / 39, 256^3
+//     122 / 85; pairs 63 / 66, 169 / 144;
 //   FP32 and pairs: while the iterates and the source (and the coefficients)
 //     stay in the 126 MB L2, since the loop reads neighbours through L1 only:
-//     f32 201 x 181 x 163 20 / 23, 224^3 (90 MB) 35 / 34.5, with a source
+//     f32 201 x 181 x 163 19 / 23, 224^3 (90 MB) 35 / 34.5, with a source
 //     (135 MB) 52 / 39; pairs 201 x 181 x 163 (106 MB) 32 / 35, 224^3 (180
-//     MB) 75 / 55.  Node coefficients and rules: f32 224^3 69 / 85, 256^3
-//     106 / 96.
+//     MB) 75 / 55; f32 node coefficients 201 x 181 x 163 (122 MB) 37 / 47.
 long long star7_loop_max_nodes(const Star7Launch& a) {
-    const long long all = (1LL << 31) - 1;  // node numbers are 32-bit
-    if (a.border == SCAFES_BORDER_TABLE) return all;
-    if (a.precision == SCAFES_PREC_F64) return 256LL * 256 * 256;
-    if (a.vc) return 224LL * 224 * 224;
-    const int fields = 2 + (a.fa ? 1 : 0) + (a.fb ? 1 : 0);
-    return 100000000LL / (fields * (long long)element_size(a.precision));
+    if (a.precision == SCAFES_PREC_F64 || a.border == SCAFES_BORDER_TABLE) return 200LL * 200 * 200;
+    const int fields = 2 + (a.fa ? 1 : 0) + (a.fb ? 1 : 0) + (a.vc ? 2 : 0);
+    return 120000000LL / (fields * (long long)element_size(a.precision));
 }
 
 cudaError_t launch_star7_loop(const Star7Loop& q, cudaStream_t stream) {
@@ -122,7 +126,19 @@ cudaError_t launch_star7_loop(const Star7Loop& q, cudaStream_t stream) {
     }
 }
 
+cudaError_t launch_star7_march_f64(const Star7Launch& a, cudaStream_t stream);
+cudaError_t launch_star7_march_f32(const Star7Launch& a, cudaStream_t stream);
+cudaError_t launch_star7_march_f32x2(const Star7Launch& a, cudaStream_t stream);
+
 cudaError_t launch_star7(const Star7Launch& a, cudaStream_t stream) {
+    if (a.tile == STAR7_MARCH) {
+        switch (a.precision) {
+            case SCAFES_PREC_F64: return launch_star7_march_f64(a, stream);
+            case SCAFES_PREC_F32: return launch_star7_march_f32(a, stream);
+            case SCAFES_PREC_F32X2: return launch_star7_march_f32x2(a, stream);
+            default: return cudaErrorInvalidValue;
+        }
+    }
     switch (a.precision) {
         case SCAFES_PREC_F64: return launch_star7_f64(a, stream);
         case SCAFES_PREC_F32: return launch_star7_f32(a, stream);

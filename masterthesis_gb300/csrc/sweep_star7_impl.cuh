@@ -150,11 +150,13 @@ static int num_sms() {
 }
 
 // z-chunk length: 16 planes keep ~8 CTAs per SM streaming with two halo
-// planes per chunk; shorter chunks give enough CTAs on small grids.
-static int choose_zchunk(const Layout& L, int by) {
+// planes per chunk; shorter chunks give enough CTAs on small grids.  The
+// {16,4} tile takes 8 planes in FP32: 89.4 against 93.9 us at 400^3, 37.6
+// against 40.8 at 320 x 256 x 256.
+static int choose_zchunk(const Layout& L, int by, int most = 16) {
     const long long tiles = (long long)((L.nx + BX - 1) / BX) * ((L.ny + by - 1) / by);
     const long long want = (long long)num_sms() * 16;
-    int zc = 16;
+    int zc = most;
     while (zc > 4 && tiles * ((L.nz + zc - 1) / zc) < want) zc >>= 1;
     while ((L.nz + zc - 1) / zc > 65535) zc <<= 1;  // grid.z limit
     return zc;
@@ -188,7 +190,7 @@ static cudaError_t launch_typed(const Star7Launch& a, cudaStream_t stream) {
     }
     T gval;
     to_elem(a.gconst, gval);
-    const int zchunk = choose_zchunk(L, BY);
+    const int zchunk = choose_zchunk(L, BY, std::is_same<P, PolF32>::value && BY == 16 && R == 4 ? 8 : 16);
     dim3 block(BX, BY / R, 1);
     dim3 grid((L.nx + BX - 1) / BX, (L.ny + BY - 1) / BY, (L.nz + zchunk - 1) / zchunk);
     kern<<<grid, block, G::SMEM, stream>>>(*a.tm_uo, FS ? *a.tm_f : *a.tm_uo, (T*)a.un, (const T*)a.fa, (const T*)a.fb, (const T*)a.ga,

@@ -1,8 +1,8 @@
 """The one-launch time loop of small grids (star7_loop.cuh).
 
 CPU: the numbering of inner and border nodes against plain loops.  GPU: the
-loop gives the bits of the launch-per-step sweeps (an explicitly set depth
-keeps those) for every border kind, source, element type and layer count it
+loop, the sweep by plain loads (star7_march.cuh) and the tile sweeps give the
+same bits (an explicitly set depth or tile keeps one launch per step) for every border kind, source, element type and layer count it
 accepts, on grids with no inner node, one node, and remainders of warps and
 CTAs, over more steps than one launch takes.
 """
@@ -25,7 +25,7 @@ def test_node_numbers_walk_the_grid(tmp_path):
     assert res.returncode == 0, res.stdout
 
 
-def _problem(M, n, prec, border, source, layers, rng):
+def _problem(M, n, prec, border, source, layers, rng, tile):
     """A handle with every field the problem reads, and its initial iterate."""
     shape = (n[2], n[1], n[0])
     tau = 0.4 / (2.0 * sum((m - 1) ** 2 for m in n))
@@ -33,7 +33,7 @@ def _problem(M, n, prec, border, source, layers, rng):
              "radiation": M.BORDER_TABLE, "nodes": M.BORDER_NODES, "vc": M.BORDER_DIRICHLET}
     variable = border in ("nodes", "vc")
     heat = dict(c0=1.0, cp=[(m - 1) ** 2 * 1.0 for m in n], cf=1.0) if variable else dict(heat=(1.0, 1.0, 0.3))
-    cfg = M.make_cfg(n, tau=tau, t_start=0.25, precision=prec, border=kinds[border], n_layers=layers, **heat)
+    cfg = M.make_cfg(n, tau=tau, t_start=0.25, precision=prec, border=kinds[border], n_layers=layers, tile=tile, **heat)
     p = M.Plain(cfg)
     if source != "none":
         p.upload(M.FIELD_F_A, rng.uniform(0.5, 1.0, shape))
@@ -74,19 +74,21 @@ CASES = [(prec, border, source, layers)
 @pytest.mark.gpu
 @pytest.mark.parametrize("prec,border,source,layers", CASES)
 @pytest.mark.parametrize("n,steps", [((4, 4, 4), 3), ((5, 7, 4), 1030), ((33, 18, 11), 5), ((70, 66, 68), 4)])
-def test_loop_gives_the_bits_of_the_sweeps(gpu, prec, border, source, layers, n, steps):
+def test_loop_and_sweeps_give_the_same_bits(gpu, prec, border, source, layers, n, steps):
     M = gpu
     got = []
-    for pinned in (False, True):
-        p, u0 = _problem(M, n, prec, border, source, layers, np.random.default_rng(n[0] + steps))
+    for schedule in ("loop", "default sweep", "tile"):
+        tile = 2 if schedule == "tile" else 0
+        p, u0 = _problem(M, n, prec, border, source, layers, np.random.default_rng(n[0] + steps), tile)
         with p:
-            if pinned:
+            if schedule == "default sweep":
                 p.set_temporal_depth(1)
             p.upload(M.FIELD_U, u0)
             p.step(1)  # the loop starts at a later step and from the other buffer
             p.step(steps)
-            assert p.last_step_launches() == (steps if pinned else (steps + 1023) // 1024)
+            assert p.last_step_launches() == ((steps + 1023) // 1024 if schedule == "loop" else steps)
             assert p.timestep() == steps + 1
             got.append(p.download())
     assert np.all(np.isfinite(got[1])) or border == "mirror"
     assert np.array_equal(got[0], got[1], equal_nan=True)
+    assert np.array_equal(got[2], got[1], equal_nan=True)
