@@ -405,8 +405,10 @@ int scafes_batch_upload(scafes_batch* b, int inst, int field,
 int scafes_batch_download(scafes_batch* b, int inst, int field,
                           double* host, size_t n);
 
-/* Advances every instance by n_steps: one persistent launch per step, the
- * whole loop recorded once per (n_steps, schedule) into a CUDA graph and
+/* Advances every instance by n_steps: one launch per step (FP64, and small
+ * ensembles: a sweep by plain loads, one CTA per short work item; else the
+ * persistent kernel, which scafes_batch_set_schedule also selects), the whole
+ * loop recorded once per (n_steps, schedule) into a CUDA graph and
  * replayed.  Asynchronous on the batch's stream. */
 int scafes_batch_step(scafes_batch* b, int n_steps);
 
@@ -419,7 +421,9 @@ int scafes_batch_step_looped(scafes_batch* b, int n_steps);
  * depth 1, then depth 2 (two steps per pass over each instance with the
  * plain sweep's depth-2 kernel, one launch per instance and pass on 16
  * parallel chains of the graph), for n_steps (rounded up to even) batched
- * steps, and keeps the fastest (iterates restored afterwards). */
+ * steps, and the sweep by plain loads, and keeps the fastest (iterates
+ * restored afterwards).  *tile and *ctas_per_sm report the best persistent
+ * schedule. */
 int scafes_batch_autotune(scafes_batch* b, int n_steps, int* tile,
                           int* ctas_per_sm);
 /* Sets the schedule directly: tile 1..4, ctas_per_sm 0 (= occupancy) .. 16. */
@@ -434,8 +438,8 @@ int scafes_batch_temporal_depth(const scafes_batch* b, int* depth, float* ms_dep
 
 /* ms of the last scafes_batch_step / _step_looped call (CUDA events). */
 int scafes_batch_last_ms(const scafes_batch* b, float* ms);
-/* Work items per step, kernel launches of the last step call, schedule and
- * total nodes of the ensemble. */
+/* Work items per step, kernel launches of the last step call, schedule (tile 0
+ * is the sweep by plain loads) and total nodes of the ensemble. */
 int scafes_batch_info(const scafes_batch* b, int* n_items, int* launches,
                       int* tile, int* ctas_per_sm, long long* n_nodes);
 const char* scafes_batch_last_error(const scafes_batch* b);

@@ -26,6 +26,7 @@
 #include <string>
 #include <vector>
 
+#include "star7_march.cuh"
 #include "star7_tile.cuh"
 
 using namespace scafes;
@@ -37,6 +38,7 @@ void set_last_error(const char* msg);
 namespace {
 
 constexpr int kZChunk = 32;  // planes per work item
+constexpr long long kMarchNodes = 4000000;  // FP32 and pairs: larger ensembles take the persistent kernel
 constexpr int kSideStreams = 16;  // parallel launch chains of a depth-2 step
 
 struct BatchInst {
@@ -52,6 +54,7 @@ struct BatchInst {
     // A field near a large constant value then keeps its pair precision
     // for the deviation.  FP64 keeps shift = 0: the reference's arithmetic.
     double shift, fshift;
+    ColumnTile ct;  // of the steps by plain loads
 };
 
 __global__ void k_add_scalar(double* __restrict__ a, size_t n, double v) {
@@ -64,6 +67,50 @@ struct BatchItem {
     short tx, ty;  // tile indices
     short z0, z1;  // planes [z0, z1)
 };
+
+// One CTA of a step by plain loads: a column tile over the inner planes
+// [z0, z1) of an instance, or (z1 == 0) 256 of its border nodes from
+// number z0 on.
+struct MarchItem {
+    int inst;
+    short tx, ty;
+    int z0, z1;
+};
+
+// One step of the ensemble by plain loads (star7_march.cuh), a CTA per item:
+// with thousands of items of 8 planes or fewer the block scheduler balances
+// the step, where the persistent kernel's 32-plane items leave SMs idle at
+// its end (and almost all of them on a small ensemble), and the column tiles
+// follow each instance's width.  us per step, this / the persistent kernel's
+// best tile: FP64, 32 instances of 32 to 160 nodes an axis 327 / 396, 12 of 20
+// to 60 11.9 / 63; pairs 226 / 163 and 9.8 / 30, FP32 155 / 76 and 7.9 / 14:
+// the memory-bound types keep the TMA ring (and its {16,4} tile) from
+// kMarchNodes nodes on, about where the fields outgrow L2.  FP64 takes 5 CTAs
+// per SM (48 registers): 4 (64, no spills) 350, 6 (40) 338.
+template <class P, int R, int MINB>
+__global__ void __launch_bounds__(MARCH_THREADS, MINB)
+batch_march(const BatchInst* __restrict__ inst, const NodeOrder* __restrict__ order,
+            const MarchItem* __restrict__ items, typename P::T* __restrict__ pool, int cur,
+            const int* __restrict__ status) {
+    if (*(const volatile int*)status != 0) return;
+    const MarchItem w = items[blockIdx.x];
+    const BatchInst& I = inst[w.inst];
+    const Layout L = I.L;
+    if (w.z1 == 0) {
+        const uint32_t m = (uint32_t)w.z0 + threadIdx.x;
+        if (m >= order[w.inst].n_border) return;
+        int x, y, z;
+        border_node(order[w.inst], m, x, y, z);
+        pool[I.off_u[cur ^ 1] + L.idx(x, y, z)] = P::from_double(I.gconst);
+        return;
+    }
+    const uint32_t row = fastdiv(threadIdx.x, I.ct.w), col = threadIdx.x - row * I.ct.w.d;
+    const int x = w.tx * (int)I.ct.w.d + (int)col + 1, y = (w.ty * I.ct.h + (int)row) * R + 1;
+    if ((int)row >= I.ct.h || x >= L.nx - 1 || y >= L.ny - 1) return;
+    const Star7Coeffs c = I.c;
+    march_rows_of<P, SRC_A, false, R>(L, c, pool + I.off_u[cur], pool + I.off_u[cur ^ 1], pool + I.off_f, nullptr,
+                                      nullptr, nullptr, Split{0.0, 0.f, 0.f}, x, y, w.z0, w.z1);
+}
 
 // The persistent loop: pull work items until the step's queue is empty.
 template <class P, int BY, int R, int NS>
@@ -157,13 +204,17 @@ struct scafes_batch {
     // Work items per tile variant.
     std::vector<BatchItem> hitems[STAR7_NUM_TILES];
     BatchItem* ditems[STAR7_NUM_TILES] = {};
+    // Items and node numbers of the steps by plain loads.
+    std::vector<MarchItem> hmarch;
+    MarchItem* dmarch = nullptr;
+    NodeOrder* dorder = nullptr;
     int* counters = nullptr;
     int n_counters = 0;
     int* status = nullptr;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    int tile = 1;
+    int tile = STAR7_MARCH;  // tile variant of the persistent kernel, or STAR7_MARCH
     int ctas_per_sm = 0;  // 0 = occupancy limit
     int depth = 1;        // temporal-blocking depth of scafes_batch_step (1 or 2)
     float depth_ms[2] = {-1.f, -1.f};  // the autotuner's best time per depth
@@ -258,8 +309,23 @@ int grid_size(scafes_batch* b, const KernelInfo& k) {
     return num_sms_dev() * per_sm;
 }
 
-// Enqueues one step of the whole ensemble (one persistent launch).
+template <class P>
+void launch_march(scafes_batch* b, int cur) {
+    batch_march<P, march_rows<P>(), march_ctas<P, SRC_A, false>()><<<(unsigned)b->hmarch.size(), MARCH_THREADS, 0, b->stream>>>(
+        b->dinst, b->dorder, b->dmarch, (typename P::T*)b->pool, cur, b->status);
+}
+
+// Enqueues one step of the whole ensemble (one launch).
 int enqueue_step(scafes_batch* b, int cur, int* counter) {
+    if (b->tile == STAR7_MARCH) {
+        switch (b->precision) {
+            case SCAFES_PREC_F32: launch_march<PolF32>(b, cur); break;
+            case SCAFES_PREC_F32X2: launch_march<PolF32x2>(b, cur); break;
+            default: launch_march<PolF64>(b, cur); break;
+        }
+        BTRY(b, cudaGetLastError());
+        return SCAFES_OK;
+    }
     const KernelInfo k = kinfo(b->precision, b->tile);
     const int grid = grid_size(b, k);
     const int n_items = (int)b->hitems[b->tile].size();
@@ -381,6 +447,29 @@ void build_items(scafes_batch* b) {
     }
 }
 
+void build_march_items(scafes_batch* b) {
+    const long long slots = 12LL * num_sms_dev();
+    for (int zc = 8;; zc >>= 1) {
+        auto& v = b->hmarch;
+        v.clear();
+        for (int i = 0; i < (int)b->hinst.size(); ++i) {
+            const Layout& L = b->hinst[i].L;
+            const long long border = border_node_count(L.nx, L.ny, L.nz, 1);
+            for (long long m = 0; m < border; m += MARCH_THREADS) v.push_back({i, 0, 0, (int)m, 0});
+        }
+        const size_t borders = v.size();
+        for (int i = 0; i < (int)b->hinst.size(); ++i) {
+            const Layout& L = b->hinst[i].L;
+            const ColumnTile& ct = b->hinst[i].ct;
+            for (int z0 = 1; z0 < L.nz - 1; z0 += zc)
+                for (int ty = 0; ty < ct.ny; ++ty)
+                    for (int tx = 0; tx < ct.nx; ++tx)
+                        v.push_back({i, (short)tx, (short)ty, z0, std::min(z0 + zc, L.nz - 1)});
+        }
+        if (zc <= 2 || (long long)(v.size() - borders) >= slots) break;
+    }
+}
+
 }  // namespace
 
 extern "C" int scafes_batch_star7_coeffs(scafes_batch_instance* in, double coeff_a, double rho_c, double perf) {
@@ -409,6 +498,8 @@ extern "C" void scafes_batch_destroy(scafes_batch* b) {
     cudaFree(b->pool);
     cudaFree(b->dmaps);
     for (int i = 0; i < STAR7_NUM_TILES; ++i) cudaFree(b->ditems[i]);
+    cudaFree(b->dmarch);
+    cudaFree(b->dorder);
     cudaFree(b->counters);
     cudaFree(b->status);
     if (b->ev0) cudaEventDestroy(b->ev0);
@@ -459,6 +550,8 @@ extern "C" int scafes_batch_create(const scafes_batch_instance* in, int n_inst, 
         I.off_u[1] = (long long)total; total += sz;
         I.off_f = (long long)total; total += sz;
         I.c = make_star7_coeffs(in[i].c0, in[i].cp, in[i].cf);
+        I.ct = make_column_tile(I.L.nx - 2, I.L.ny - 2,
+                                precision == SCAFES_PREC_F32X2 ? march_rows<PolF32x2>() : march_rows<PolF64>());
         I.gconst = in[i].g_value;
         I.shift = I.fshift = 0.0;
         const double k = in[i].c0 + 2.0 * (in[i].cp[0] + in[i].cp[1] + in[i].cp[2]) - 1.0;
@@ -553,7 +646,19 @@ extern "C" int scafes_batch_create(const scafes_batch_instance* in, int n_inst, 
             return bail(SCAFES_ERR_CUDA);
         }
     }
-    if ((e = cudaStreamSynchronize(b->stream)) != cudaSuccess) {
+    long long nodes = 0;
+    for (const BatchInst& I : b->hinst) nodes += (long long)I.L.nx * I.L.ny * I.L.nz;
+    b->tile = precision == SCAFES_PREC_F64 || nodes <= kMarchNodes ? STAR7_MARCH : 3;
+    build_march_items(b);
+    std::vector<NodeOrder> order;
+    for (const BatchInst& I : b->hinst) order.push_back(make_node_order(I.L.nx, I.L.ny, I.L.nz, 1));
+    if ((e = cudaMalloc(&b->dmarch, sizeof(MarchItem) * b->hmarch.size())) != cudaSuccess ||
+        (e = cudaMemcpyAsync(b->dmarch, b->hmarch.data(), sizeof(MarchItem) * b->hmarch.size(),
+                             cudaMemcpyHostToDevice, b->stream)) != cudaSuccess ||
+        (e = cudaMalloc(&b->dorder, sizeof(NodeOrder) * order.size())) != cudaSuccess ||
+        (e = cudaMemcpyAsync(b->dorder, order.data(), sizeof(NodeOrder) * order.size(), cudaMemcpyHostToDevice,
+                             b->stream)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(b->stream)) != cudaSuccess) {
         bfail(nullptr, SCAFES_ERR_CUDA, "scafes_batch_create: %s", cudaGetErrorString(e));
         return bail(SCAFES_ERR_CUDA);
     }
@@ -618,8 +723,7 @@ extern "C" int scafes_batch_step(scafes_batch* b, int n_steps) {
     if (n_steps == 0) return SCAFES_OK;
     int rc = ensure_counters(b, n_steps);
     if (rc) return rc;
-    const KernelInfo k = kinfo(b->precision, b->tile);
-    grid_size(b, k);  // sets the smem attribute outside any capture
+    if (b->tile != STAR7_MARCH) grid_size(b, kinfo(b->precision, b->tile));  // sets the smem attribute outside any capture
     // Depth 2: n_steps / 2 passes, an odd last step by the persistent kernel.
     const int pairs = b->depth == 2 ? n_steps / 2 : 0;
     const int singles = n_steps - 2 * pairs;
@@ -719,9 +823,10 @@ extern "C" int scafes_batch_last_ms(const scafes_batch* b, float* ms) {
 extern "C" int scafes_batch_info(const scafes_batch* b, int* n_items, int* launches, int* tile, int* ctas_per_sm,
                                  long long* n_nodes) {
     if (!b) return bfail(nullptr, SCAFES_ERR_ARG, "scafes_batch_info: batch is NULL");
-    if (n_items) *n_items = (int)b->hitems[b->tile].size();
+    const bool march = b->tile == STAR7_MARCH;
+    if (n_items) *n_items = (int)(march ? b->hmarch.size() : b->hitems[b->tile].size());
     if (launches) *launches = b->launches;
-    if (tile) *tile = b->tile + 1;
+    if (tile) *tile = march ? 0 : b->tile + 1;
     if (ctas_per_sm) *ctas_per_sm = b->ctas_per_sm;
     if (n_nodes) {
         long long s = 0;
@@ -740,7 +845,7 @@ extern "C" int scafes_batch_autotune(scafes_batch* b, int n_steps, int* tile_out
     BTRY(b, cudaMalloc(&save, bytes));
     cudaError_t e = cudaMemcpyAsync(save, b->pool, bytes, cudaMemcpyDeviceToDevice, b->stream);
     const int cur0 = b->cur, t0 = b->t;
-    int best_tile = b->tile, best_ctas = b->ctas_per_sm, best_depth = 1, rc = SCAFES_OK;
+    int best_tile = 0, best_ctas = 0, best_depth = 1, rc = SCAFES_OK;
     float best = -1.f;
     const int ctas_opts[] = {0, 1, 2, 4};
     // Depth 1: every tile x CTAs per SM; then depth 2 (its own kernel, no
@@ -762,11 +867,25 @@ extern "C" int scafes_batch_autotune(scafes_batch* b, int n_steps, int* tile_out
             }
         }
     }
+    // The step by plain loads, which has no tile or CTA choice.
+    int best_schedule = best_tile;
+    if (rc == SCAFES_OK && e == cudaSuccess) {
+        b->tile = STAR7_MARCH;
+        b->ctas_per_sm = 0;
+        rc = scafes_batch_step(b, trial);
+        if (rc == SCAFES_OK) rc = scafes_batch_step(b, trial);
+        float ms = 0.f;
+        if (rc == SCAFES_OK) rc = scafes_batch_last_ms(b, &ms);
+        if (rc == SCAFES_OK && ms < best) {
+            best = ms;
+            best_schedule = STAR7_MARCH;
+        }
+    }
     b->depth_ms[0] = best;
     b->depth_ms[1] = -1.f;
     if (rc == SCAFES_OK && e == cudaSuccess) {
         b->depth = 2;
-        b->tile = best_tile;
+        b->tile = best_schedule;
         b->ctas_per_sm = best_ctas;
         rc = scafes_batch_step(b, trial);
         if (rc == SCAFES_OK) rc = scafes_batch_step(b, trial);
@@ -785,7 +904,7 @@ extern "C" int scafes_batch_autotune(scafes_batch* b, int n_steps, int* tile_out
     cudaFree(save);
     b->cur = cur0;
     b->t = t0;
-    b->tile = best_tile;
+    b->tile = best_schedule;
     b->ctas_per_sm = best_ctas;
     b->depth = best_depth;
     b->timed = false;

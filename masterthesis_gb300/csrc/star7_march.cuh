@@ -1,4 +1,4 @@
-// One time step by plain loads: a warp owns R rows of 32 columns and marches
+// One time step by plain loads: a thread owns R rows of a column and marches
 // z, with below, current and above in registers and the x and y neighbours
 // through L1 (which holds them from their own "above" loads a plane
 // earlier).  The border nodes are left to CTAs of their own at the front of
@@ -26,6 +26,37 @@
 
 namespace scafes {
 
+constexpr int MARCH_THREADS = 256;
+
+// The columns of a CTA: w x h threads (h R rows), w h <= MARCH_THREADS.
+// FP64 pays for every warp whatever its active lanes, and 32 columns at a
+// time leave up to a quarter of them idle (98 inner columns: 98 of 128), so
+// the width follows the grid: the (w, h) with the fewest idle threads, w
+// from 16 to 64 (sectors; rows that share their y neighbours in L1).
+struct ColumnTile {
+    FastDiv w;
+    int h, nx, ny;  // rows of threads; tiles along x and y
+};
+inline ColumnTile make_column_tile(int ix, int iy, int rows) {
+    ColumnTile t;
+    t.h = t.nx = t.ny = 0;
+    long long best = 0;
+    const int ty = (iy + rows - 1) / rows;  // rows of threads
+    for (int n = (ix + 63) / 64; n <= (ix + 15) / 16 || n == (ix + 63) / 64; ++n) {
+        if (n == 0) break;
+        const int w = (ix + n - 1) / n, h = MARCH_THREADS / w, m = (ty + h - 1) / h;
+        const long long threads = (long long)n * m * MARCH_THREADS;
+        if (t.h == 0 || threads < best || (threads == best && h > t.h)) {
+            best = threads;
+            t.w = make_fastdiv((uint32_t)w);
+            t.h = h;
+            t.nx = n;
+            t.ny = m;
+        }
+    }
+    return t;
+}
+
 template <class T>
 struct MarchArgs {
     const T* uo;
@@ -44,42 +75,26 @@ struct MarchArgs {
     const scafes_border_node_rule* nodes;
     StepTimes t;
     uint32_t border_ctas;
+    ColumnTile ct;
     FastDiv tx, txy;  // tiles along x, tiles of a layer
     int zchunk;
     const int* status;
 };
 
-constexpr int MARCH_Y = 8;  // warps of a CTA
-
-template <class P, int SRC, int BORDER, bool VC, int R, int MINB>
-__global__ void __launch_bounds__(32 * MARCH_Y, MINB)
-star7_march(const __grid_constant__ MarchArgs<typename P::T> A) {
+// The R rows from row y of column x, planes [z0, z1), all of them inner
+// planes and (row y, column x) an inner one.
+template <class P, int SRC, bool VC, int R>
+__device__ __forceinline__ void march_rows_of(const Layout& L, const Star7Coeffs& c, const typename P::T* __restrict__ uo,
+                                              typename P::T* __restrict__ un, const typename P::T* __restrict__ fa,
+                                              const typename P::T* __restrict__ fb,
+                                              const typename P::T* __restrict__ c0f,
+                                              const typename P::T* __restrict__ caf, const Split& t_old, int x, int y,
+                                              int z0, int z1) {
     using T = typename P::T;
     constexpr bool HAS_F = SRC != SRC_NONE;
     constexpr bool has_fb = SRC == SRC_AB;
-    const Layout& L = A.L;
-    if (*(const volatile int*)A.status != 0) return;  // an earlier sweep gave up
-    if (blockIdx.x < A.border_ctas) {
-        const uint32_t m = blockIdx.x * (32 * MARCH_Y) + threadIdx.x;
-        if (m >= A.o.n_border) return;
-        TileJob<T> J{nullptr, nullptr, nullptr, A.fa, A.fb, A.ga, A.gb, A.gval, L, A.t.t_old, A.t.t_new, A.t.corr};
-        J.table = A.table;
-        J.nodes = A.nodes;
-        int x, y, z;
-        border_node(A.o, m, x, y, z);
-        A.un[L.idx(x, y, z)] = border_value<P, SRC, BORDER>(J, A.uo, x, y, z);
-        return;
-    }
-    const uint32_t q = blockIdx.x - A.border_ctas;
-    const uint32_t k = fastdiv(q, A.txy), r = q - k * A.txy.d, j = fastdiv(r, A.tx);
-    const int x = (int)(r - j * A.tx.d) * 32 + (threadIdx.x & 31);
-    const int y = (int)(j * MARCH_Y + (threadIdx.x >> 5)) * R + L.nl;
-    if (x < L.nl || x >= L.nx - L.nl || y >= L.ny - L.nl) return;
-    const int z0 = (int)k * A.zchunk + L.nl, z1 = min(z0 + A.zchunk, L.nz - L.nl);
     const long long py = L.pitch, pz = L.plane;
     long long o = L.idx(x, y, z0);
-    const T* __restrict__ uo = A.uo;
-    T* __restrict__ un = A.un;
     // Rows that are border rows are computed but not stored; a row beyond the
     // grid reads the last one.
     unsigned skip = 0u;
@@ -106,18 +121,18 @@ star7_march(const __grid_constant__ MarchArgs<typename P::T> A) {
             w[i] = uo[o + ro[i] - 1];
             e[i] = uo[o + ro[i] + 1];
             f[i] = P::zero();
-            if (HAS_F) f[i] = P::src(A.fa[o + ro[i]], has_fb ? A.fb[o + ro[i]] : P::zero(), A.t.t_old, has_fb);
+            if (HAS_F) f[i] = P::src(fa[o + ro[i]], has_fb ? fb[o + ro[i]] : P::zero(), t_old, has_fb);
         }
         if constexpr (VC) {
             T c0[R], ca[R];
 #pragma unroll
             for (int i = 0; i < R; ++i) {
-                c0[i] = A.c0[o + ro[i]];
-                ca[i] = A.ca[o + ro[i]];
+                c0[i] = c0f[o + ro[i]];
+                ca[i] = caf[o + ro[i]];
             }
-            P::template star_vc_rows<HAS_F, R>(A.c, below, cur, above, ym, yp, w, e, f, c0, ca, 1, v, skip);
+            P::template star_vc_rows<HAS_F, R>(c, below, cur, above, ym, yp, w, e, f, c0, ca, 1, v, skip);
         } else {
-            P::template star_rows<HAS_F, R>(A.c, below, cur, above, ym, yp, w, e, f, v, skip);
+            P::template star_rows<HAS_F, R>(c, below, cur, above, ym, yp, w, e, f, v, skip);
         }
 #pragma unroll
         for (int i = 0; i < R; ++i)
@@ -128,6 +143,33 @@ star7_march(const __grid_constant__ MarchArgs<typename P::T> A) {
             cur[i] = above[i];
         }
     }
+}
+
+template <class P, int SRC, int BORDER, bool VC, int R, int MINB>
+__global__ void __launch_bounds__(MARCH_THREADS, MINB)
+star7_march(const __grid_constant__ MarchArgs<typename P::T> A) {
+    using T = typename P::T;
+    const Layout& L = A.L;
+    if (*(const volatile int*)A.status != 0) return;  // an earlier sweep gave up
+    if (blockIdx.x < A.border_ctas) {
+        const uint32_t m = blockIdx.x * (MARCH_THREADS) + threadIdx.x;
+        if (m >= A.o.n_border) return;
+        TileJob<T> J{nullptr, nullptr, nullptr, A.fa, A.fb, A.ga, A.gb, A.gval, L, A.t.t_old, A.t.t_new, A.t.corr};
+        J.table = A.table;
+        J.nodes = A.nodes;
+        int x, y, z;
+        border_node(A.o, m, x, y, z);
+        A.un[L.idx(x, y, z)] = border_value<P, SRC, BORDER>(J, A.uo, x, y, z);
+        return;
+    }
+    const uint32_t q = blockIdx.x - A.border_ctas;
+    const uint32_t k = fastdiv(q, A.txy), r = q - k * A.txy.d, j = fastdiv(r, A.tx);
+    const uint32_t row = fastdiv(threadIdx.x, A.ct.w), col = threadIdx.x - row * A.ct.w.d;
+    const int x = (int)((r - j * A.tx.d) * A.ct.w.d + col) + L.nl;
+    const int y = ((int)j * A.ct.h + (int)row) * R + L.nl;
+    if ((int)row >= A.ct.h || x >= L.nx - L.nl || y >= L.ny - L.nl) return;
+    const int z0 = (int)k * A.zchunk + L.nl, z1 = min(z0 + A.zchunk, L.nz - L.nl);
+    march_rows_of<P, SRC, VC, R>(L, A.c, A.uo, A.un, A.fa, A.fb, A.c0, A.ca, A.t.t_old, x, y, z0, z1);
 }
 
 // ---- host side ---------------------------------------------------------------
@@ -148,9 +190,10 @@ template <class P>
 constexpr int march_rows() {
     return std::is_same<P, PolF32x2>::value ? 2 : 1;
 }
-template <class P>
+template <class P, int SRC, bool VC>
 constexpr int march_ctas() {
-    return std::is_same<P, PolF32x2>::value ? 4 : 6;
+    if (std::is_same<P, PolF32x2>::value) return 4;
+    return std::is_same<P, PolF64>::value && (SRC != SRC_NONE || VC) ? 5 : 6;
 }
 
 template <class P, int SRC, int BORDER, bool VC>
@@ -175,7 +218,7 @@ static cudaError_t launch_march_typed(const Star7Launch& a, cudaStream_t stream)
     A.t = StepTimes{make_split(a.time_old), make_split(a.time_new), make_split(a.mirror_corr)};
     A.status = a.status;
     const int nl = a.L.nl, iy = a.L.ny - 2 * nl, iz = a.L.nz - 2 * nl;
-    A.border_ctas = (A.o.n_border + 32 * MARCH_Y - 1) / (32 * MARCH_Y);
+    A.border_ctas = (A.o.n_border + MARCH_THREADS - 1) / (MARCH_THREADS);
     // 8 planes per CTA (16 for pairs), 4 while that leaves under two rounds
     // of resident CTAs: 256^3 f64 145, 150, 163 us with 8, 16, 32 planes;
     // 160^3 40.4 with 4, 41.9 with 8; pairs 300 x 280 x 260 108, 104.5, 112
@@ -183,16 +226,17 @@ static cudaError_t launch_march_typed(const Star7Launch& a, cudaStream_t stream)
     int sms = 1, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const long long tx = (a.L.nx + 31) / 32, ty = std::max(0, (iy + MARCH_Y * R - 1) / (MARCH_Y * R));
+    A.ct = make_column_tile(a.L.nx - 2 * nl, iy, R);
+    const long long tx = A.ct.nx, ty = A.ct.ny;
     int zc = R == 2 ? 16 : 8;
     while (zc > 4 && tx * ty * ((iz + zc - 1) / zc) < 12LL * sms) zc >>= 1;
     const long long tz = std::max(0, (iz + zc - 1) / zc);
     A.zchunk = zc;
-    A.tx = make_fastdiv((uint32_t)tx);
+    A.tx = make_fastdiv((uint32_t)std::max(1LL, tx));
     A.txy = make_fastdiv((uint32_t)std::max(1LL, tx * ty));
     const long long ctas = A.border_ctas + (A.o.n_inner ? tx * ty * tz : 0);
     if (ctas > 0x7fffffffLL) return cudaErrorInvalidValue;
-    star7_march<P, SRC, BORDER, VC, R, march_ctas<P>()><<<(unsigned)ctas, 32 * MARCH_Y, 0, stream>>>(A);
+    star7_march<P, SRC, BORDER, VC, R, march_ctas<P, SRC, VC>()><<<(unsigned)ctas, MARCH_THREADS, 0, stream>>>(A);
     return cudaGetLastError();
 }
 

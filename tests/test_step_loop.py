@@ -92,3 +92,31 @@ def test_loop_and_sweeps_give_the_same_bits(gpu, prec, border, source, layers, n
     assert np.all(np.isfinite(got[1])) or border == "mirror"
     assert np.array_equal(got[0], got[1], equal_nan=True)
     assert np.array_equal(got[2], got[1], equal_nan=True)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", ["f64", "f32", "f32x2"])
+def test_ensemble_schedules_give_the_same_bits(gpu, prec):
+    """The ensemble's step by plain loads against the persistent kernel, on
+    instances with one inner row, widths around the column tiles' limits and
+    a remainder of planes."""
+    M = gpu
+    rng = np.random.default_rng(4)
+    sizes = [(3, 3, 3), (3, 9, 12), (18, 3, 11), (66, 65, 10), (67, 21, 20), (131, 7, 5)]
+    specs = [M.batch_instance(n, 0.3 / sum((m - 1) ** 2 for m in n), 0.5, 1.0, 1e-3, 37.0) for n in sizes]
+    data = [(37.0 + rng.uniform(0.0, 1.0, n[::-1]), rng.uniform(0.0, 10.0, n[::-1])) for n in sizes]
+    got = []
+    for tile in (0, 1, 4):
+        with M.Batch(specs, prec) as b:
+            for i, (u, f) in enumerate(data):
+                b.upload(i, M.FIELD_F_A, f)
+                b.upload(i, M.FIELD_U, u)
+            if tile:
+                b.set_schedule(tile)
+            else:
+                assert b.info()["tile"] == 0
+            b.step(5)
+            got.append([b.download(i) for i in range(len(sizes))])
+    for other in got[1:]:
+        for a, c in zip(got[0], other):
+            assert np.array_equal(a, c)
