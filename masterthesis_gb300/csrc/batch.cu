@@ -646,13 +646,24 @@ extern "C" int scafes_batch_create(const scafes_batch_instance* in, int n_inst, 
             return bail(SCAFES_ERR_CUDA);
         }
     }
-    long long nodes = 0;
-    for (const BatchInst& I : b->hinst) nodes += (long long)I.L.nx * I.L.ny * I.L.nz;
-    b->tile = precision == SCAFES_PREC_F64 || nodes <= kMarchNodes ? STAR7_MARCH : 3;
+    long long nodes = 0, most = 0;
+    for (const BatchInst& I : b->hinst) {
+        const long long n = (long long)I.L.nx * I.L.ny * I.L.nz;
+        nodes += n;
+        most = std::max(most, n);
+    }
+    const bool f64 = precision == SCAFES_PREC_F64;
+    b->tile = f64 || nodes <= kMarchNodes ? STAR7_MARCH : 3;
     build_march_items(b);
+    // The steps by plain loads number an instance's nodes, and the items, in
+    // 32 bits.
+    if (most >= (1LL << 31) || b->hmarch.size() >= (1ull << 31)) {
+        b->hmarch.clear();
+        if (b->tile == STAR7_MARCH) b->tile = f64 ? 0 : 3;
+    }
     std::vector<NodeOrder> order;
     for (const BatchInst& I : b->hinst) order.push_back(make_node_order(I.L.nx, I.L.ny, I.L.nz, 1));
-    if ((e = cudaMalloc(&b->dmarch, sizeof(MarchItem) * b->hmarch.size())) != cudaSuccess ||
+    if ((e = cudaMalloc(&b->dmarch, sizeof(MarchItem) * std::max<size_t>(1, b->hmarch.size()))) != cudaSuccess ||
         (e = cudaMemcpyAsync(b->dmarch, b->hmarch.data(), sizeof(MarchItem) * b->hmarch.size(),
                              cudaMemcpyHostToDevice, b->stream)) != cudaSuccess ||
         (e = cudaMalloc(&b->dorder, sizeof(NodeOrder) * order.size())) != cudaSuccess ||
@@ -869,7 +880,7 @@ extern "C" int scafes_batch_autotune(scafes_batch* b, int n_steps, int* tile_out
     }
     // The step by plain loads, which has no tile or CTA choice.
     int best_schedule = best_tile;
-    if (rc == SCAFES_OK && e == cudaSuccess) {
+    if (rc == SCAFES_OK && e == cudaSuccess && !b->hmarch.empty()) {
         b->tile = STAR7_MARCH;
         b->ctas_per_sm = 0;
         rc = scafes_batch_step(b, trial);

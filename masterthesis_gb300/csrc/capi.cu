@@ -1053,7 +1053,8 @@ extern "C" int scafes_gpu_autotune(scafes_handle* h, int n_steps, int* chosen, f
     cudaError_t e = cudaMemcpyAsync(save, h->u[h->cur], bytes, cudaMemcpyDeviceToDevice, h->stream);
     int best = 0, best_tile = 0, rc = SCAFES_OK;
     float best_ms = 0.f;
-    for (int tile = 0; tile <= STAR7_MARCH && e == cudaSuccess && rc == SCAFES_OK; ++tile) {
+    const int schedules = n_nodes(h) < (1ull << 31) ? STAR7_MARCH + 1 : STAR7_NUM_TILES;  // 32-bit node numbers
+    for (int tile = 0; tile < schedules && e == cudaSuccess && rc == SCAFES_OK; ++tile) {
         rc = step_impl(h, 1, tile, false, 1);  // warm-up (and first-use setup)
         if (rc == SCAFES_OK) rc = step_impl(h, n_steps, tile, true, 1);
         float ms = 0.f;

@@ -1,6 +1,6 @@
 // Numbers of the inner and the border nodes of a grid and back, by
-// multiplications instead of divisions: how the kernels that work through a
-// grid node by node (star7_loop.cuh) deal it out.
+// multiplications instead of divisions, and column tiles that fit a grid: how
+// the kernels without a TMA ring deal a grid out.
 #pragma once
 
 #include <stdint.h>
@@ -88,6 +88,39 @@ SCAFES_HD void border_node(const NodeOrder& o, uint32_t m, int& x, int& y, int& 
     const uint32_t j = fastdiv(r, o.pair), i = r - j * 2 * o.nl;
     y = (int)(j + o.nl);
     x = (int)(i < o.nl ? i : o.nx - 2 * o.nl + i);
+}
+
+constexpr int MARCH_THREADS = 256;
+
+// The columns of a CTA: w x h threads (h R rows), w h <= MARCH_THREADS.
+// FP64 pays for every warp whatever its active lanes, and 32 columns at a
+// time leave up to a quarter of them idle (98 inner columns: 98 of 128), so
+// the width follows the grid: the (w, h) with the fewest idle threads, w
+// at most 64 and at
+// least 16 where the grid has them, h at most 16 (sectors; rows that share
+// their y neighbours in L1; the halos that callers keep in shared memory).
+struct ColumnTile {
+    FastDiv w;
+    int h, nx, ny;  // rows of threads; tiles along x and y
+};
+inline ColumnTile make_column_tile(int ix, int iy, int rows) {
+    ColumnTile t;
+    t.h = t.nx = t.ny = 0;
+    long long best = 0;
+    const int ty = (iy + rows - 1) / rows;  // rows of threads
+    for (int n = (ix + 63) / 64; n <= (ix + 15) / 16 || n == (ix + 63) / 64; ++n) {
+        if (n == 0) break;
+        const int w = (ix + n - 1) / n, h = MARCH_THREADS / w < 16 ? MARCH_THREADS / w : 16, m = (ty + h - 1) / h;
+        const long long threads = (long long)n * m * MARCH_THREADS;
+        if (t.h == 0 || threads < best || (threads == best && h > t.h)) {
+            best = threads;
+            t.w = make_fastdiv((uint32_t)w);
+            t.h = h;
+            t.nx = n;
+            t.ny = m;
+        }
+    }
+    return t;
 }
 
 }  // namespace scafes

@@ -26,37 +26,6 @@
 
 namespace scafes {
 
-constexpr int MARCH_THREADS = 256;
-
-// The columns of a CTA: w x h threads (h R rows), w h <= MARCH_THREADS.
-// FP64 pays for every warp whatever its active lanes, and 32 columns at a
-// time leave up to a quarter of them idle (98 inner columns: 98 of 128), so
-// the width follows the grid: the (w, h) with the fewest idle threads, w
-// from 16 to 64 (sectors; rows that share their y neighbours in L1).
-struct ColumnTile {
-    FastDiv w;
-    int h, nx, ny;  // rows of threads; tiles along x and y
-};
-inline ColumnTile make_column_tile(int ix, int iy, int rows) {
-    ColumnTile t;
-    t.h = t.nx = t.ny = 0;
-    long long best = 0;
-    const int ty = (iy + rows - 1) / rows;  // rows of threads
-    for (int n = (ix + 63) / 64; n <= (ix + 15) / 16 || n == (ix + 63) / 64; ++n) {
-        if (n == 0) break;
-        const int w = (ix + n - 1) / n, h = MARCH_THREADS / w, m = (ty + h - 1) / h;
-        const long long threads = (long long)n * m * MARCH_THREADS;
-        if (t.h == 0 || threads < best || (threads == best && h > t.h)) {
-            best = threads;
-            t.w = make_fastdiv((uint32_t)w);
-            t.h = h;
-            t.nx = n;
-            t.ny = m;
-        }
-    }
-    return t;
-}
-
 template <class T>
 struct MarchArgs {
     const T* uo;
@@ -200,6 +169,7 @@ template <class P, int SRC, int BORDER, bool VC>
 static cudaError_t launch_march_typed(const Star7Launch& a, cudaStream_t stream) {
     using T = typename P::T;
     constexpr int R = march_rows<P>();
+    if ((long long)a.L.nx * a.L.ny * a.L.nz >= (1LL << 31)) return cudaErrorInvalidValue;  // 32-bit node numbers
     MarchArgs<T> A;
     A.uo = (const T*)a.uo;
     A.un = (T*)a.un;

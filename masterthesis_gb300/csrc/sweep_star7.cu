@@ -52,8 +52,11 @@ int star7_box_height(int tile) {
 //   FP32 and pairs below 128 x 128 columns: the {8,1} tile, which has the
 //     most CTAs (several steps of these grids run as a one-launch loop).
 int star7_default_tile(const Star7Launch& a) {
-    if (a.precision == SCAFES_PREC_F64 || a.L.nl != 1 || a.border == SCAFES_BORDER_TABLE) return STAR7_MARCH;
-    if ((long long)a.L.nx * a.L.ny < 128LL * 128LL) return 0;
+    // The march numbers nodes in 32 bits.
+    const bool march = (long long)a.L.nx * a.L.ny * a.L.nz < (1LL << 31);
+    if (march && (a.precision == SCAFES_PREC_F64 || a.L.nl != 1 || a.border == SCAFES_BORDER_TABLE))
+        return STAR7_MARCH;
+    if (a.precision == SCAFES_PREC_F64 || (long long)a.L.nx * a.L.ny < 128LL * 128LL) return 0;
     return a.precision == SCAFES_PREC_F32X2 && a.fa ? 2 : 3;
 }
 
