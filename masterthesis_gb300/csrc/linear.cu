@@ -10,8 +10,8 @@
 // evalUpdatePhase, pointer swap, evalUpdate2Phase, src/ScaFES_Problem.hpp:
 // 2596-2619, 2829-2918; every node of the new iterate starts as a copy of
 // the old one, :5078-5082, which a recorded rule already contains).
-// FP64, plain loads: a correctness path for the problems the fused kernels
-// (Lame-Navier, Yee) do not cover as recorded callbacks.  Each field has its
+// FP64, plain loads: the path of the problems the fused kernels (Lame-Navier,
+// Yee) do not cover as recorded callbacks.  Each field has its
 // own pair of buffers; a field that a phase leaves alone on every node (its
 // rule the identity) is neither copied nor swapped in that phase.
 #include <cuda_runtime.h>
@@ -22,6 +22,7 @@
 #include <string>
 #include <vector>
 
+#include "node_order.cuh"
 #include "scafes_common.cuh"
 #include "../../include/scafes_gb300.h"
 
@@ -54,7 +55,79 @@ struct FieldPtrs {
     double* out[SCAFES_LIN_MAX_FIELDS];
 };
 
-__global__ void k_linear(FieldPtrs P, const Rule* __restrict__ rules, const Term* __restrict__ terms, int n_fields,
+// One node per thread, the inner nodes first (every one of them class 0), the
+// border nodes in CTAs after them, numbered densely (node_order.cuh).  The
+// FP64 pipe bounds it (a DFMA per term and node), so what counts is that the
+// rest keeps out of its way: the inner rules come as kernel parameters with
+// their sources resolved to addresses, so a term is two constant loads, one
+// load of the field and the DFMA, without a table to fetch first (us per step
+// of the Yee cavity at 96 x 81 x 73: the table in memory, read by every node,
+// 52.8, in shared memory 51, this 37.7); and a rule that starts with a field's own
+// value, weight 1 and no constant, starts from that value instead of
+// multiplying it.
+struct Resolved {
+    const double* p;  // the source's buffer, moved by the term's offset
+    double w;
+};
+
+struct LinArgs {
+    FieldPtrs P;
+    const Rule* rules;
+    const Term* terms;
+    int n_fields;
+    Layout L;
+    NodeOrder o;
+    uint32_t inner_ctas;
+    // The inner rules of the fields this phase writes, one after the other.
+    int n_written;
+    struct Written {
+        double* out;
+        double cst;
+        int first, end;  // terms
+        bool own;        // starts from its first term's value itself
+    } written[SCAFES_LIN_MAX_FIELDS];
+    Resolved term[SCAFES_LIN_MAX_FIELDS * SCAFES_LIN_MAX_TERMS];
+};
+
+__global__ void __launch_bounds__(MARCH_THREADS) k_linear(const __grid_constant__ LinArgs A) {
+    const Layout& L = A.L;
+    int x, y, z;
+    if (blockIdx.x < A.inner_ctas) {
+        const uint32_t m = blockIdx.x * MARCH_THREADS + threadIdx.x;
+        if (m >= A.o.n_inner) return;
+        inner_node(A.o, m, x, y, z);
+        const long long o = L.idx(x, y, z);
+        for (int f = 0; f < A.n_written; ++f) {
+            const LinArgs::Written& w = A.written[f];
+            int k = w.first;
+            double v = w.cst;
+            if (w.own) v = __ldg(A.term[k++].p + o);
+#pragma unroll 4
+            for (; k < w.end; ++k) v = fma(A.term[k].w, __ldg(A.term[k].p + o), v);
+            w.out[o] = v;
+        }
+        return;
+    }
+    const uint32_t m = (blockIdx.x - A.inner_ctas) * MARCH_THREADS + threadIdx.x;
+    if (m >= A.o.n_border) return;
+    border_node(A.o, m, x, y, z);
+    const int cls = (x == 0) | ((x == L.nx - 1) << 1) | ((y == 0) << 2) | ((y == L.ny - 1) << 3) | ((z == 0) << 4) |
+                    ((z == L.nz - 1) << 5);
+    const long long o = L.idx(x, y, z);
+    for (int f = 0; f < A.n_fields; ++f) {
+        if (A.P.out[f] == nullptr) continue;
+        const Rule r = A.rules[f * kClasses + cls];
+        double v = r.cst;
+        for (int k = r.off; k < r.off + r.n; ++k) {
+            const Term t = A.terms[k];
+            v = fma(t.w, A.P.in[t.src][o + t.d], v);
+        }
+        A.P.out[f][o] = v;
+    }
+}
+
+// Grids of 2^31 nodes and more, which 32-bit node numbers do not cover.
+__global__ void k_linear_big(FieldPtrs P, const Rule* __restrict__ rules, const Term* __restrict__ terms, int n_fields,
                          Layout L) {
     const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y, z = blockIdx.z;
     if (x >= L.nx || y >= L.ny) return;
@@ -275,6 +348,20 @@ extern "C" int scafes_lin_step(scafes_lin* h, int n_steps) {
     if (int rc = sync_rules(h)) return rc;
     const Layout& L = h->L;
     const dim3 grid((L.nx + 31) / 32, (L.ny + 7) / 8, L.nz), block(32, 8);
+    const bool numbered = (long long)L.nx * L.ny * L.nz < (1LL << 31);
+    NodeOrder o{};
+    uint32_t inner_ctas = 0, border_ctas = 0;
+    if (numbered) {
+        o = make_node_order(L.nx, L.ny, L.nz, 1);
+        inner_ctas = (o.n_inner + MARCH_THREADS - 1) / MARCH_THREADS;
+        border_ctas = (o.n_border + MARCH_THREADS - 1) / MARCH_THREADS;
+    }
+    LinArgs A;
+    A.terms = h->terms;
+    A.n_fields = h->n_fields;
+    A.L = L;
+    A.o = o;
+    A.inner_ctas = inner_ctas;
     const size_t per_phase = (size_t)h->n_fields * kClasses;
     LTRY(h, cudaEventRecord(h->e0, h->stream));
     for (int s = 0; s < n_steps; ++s)
@@ -289,7 +376,26 @@ extern "C" int scafes_lin_step(scafes_lin* h, int n_steps) {
                 P.in[f] = h->buf[h->cur[f]] + fo;
                 if (!h->ident[(size_t)ph * h->n_fields + f]) P.out[f] = h->buf[h->cur[f] ^ 1] + fo;
             }
-            k_linear<<<grid, block, 0, h->stream>>>(P, h->rules + ph * per_phase, h->terms, h->n_fields, L);
+            const Rule* rules = h->rules + ph * per_phase;
+            if (numbered) {
+                A.P = P;
+                A.rules = rules;
+                A.n_written = 0;
+                int n = 0;
+                for (int f = 0; f < h->n_fields; ++f) {
+                    if (!P.out[f]) continue;
+                    const size_t sl = slot(h, ph, f, 0);
+                    const auto& tl = h->host_terms[sl];
+                    const double cst = h->host_cst[sl];
+                    const int first = n;
+                    for (const auto& t : tl) A.term[n++] = Resolved{P.in[t.src] + L.idx(t.dx, t.dy, t.dz), t.w};
+                    A.written[A.n_written++] = {P.out[f], cst, first, n,
+                                                !tl.empty() && cst == 0.0 && tl[0].w == 1.0};
+                }
+                k_linear<<<inner_ctas + border_ctas, MARCH_THREADS, 0, h->stream>>>(A);
+            } else {
+                k_linear_big<<<grid, block, 0, h->stream>>>(P, rules, h->terms, h->n_fields, L);
+            }
             LTRY(h, cudaGetLastError());
             for (int f = 0; f < h->n_fields; ++f)
                 if (P.out[f]) h->cur[f] ^= 1;
