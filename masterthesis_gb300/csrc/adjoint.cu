@@ -21,6 +21,7 @@
 // in device memory; the split points follow the optimal binomial schedule
 // (Griewank & Walther, "Algorithm 799: revolve", ACM TOMS 26(1), 2000),
 // computed here by dynamic programming over (steps, free snapshots).
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -31,6 +32,7 @@
 #include <vector>
 
 #include "adjoint.cuh"
+#include "node_order.cuh"
 #include "scafes_common.cuh"
 #include "tma.cuh"
 #include "../../include/scafes_gb300.h"
@@ -72,28 +74,54 @@ __global__ void k_faces(const double* __restrict__ k, double* __restrict__ kx, d
 // form u'_i = d_i u_i + sum_f K_f u_nb: 7 FP64 operations per node (the
 // flux form takes 12), summed in the order diagonal, +x, -x, +y, -y, +z,
 // -z, which the reverse sweep's recomputation repeats bit for bit.
-__global__ void __launch_bounds__(AX * AY)
+__device__ __forceinline__ double forward_node(const double* __restrict__ u, const double* __restrict__ kx,
+                                               const double* __restrict__ ky, const double* __restrict__ kz,
+                                               const double* __restrict__ dg, const Layout& L, long long o) {
+    double v = dg[o] * u[o];
+    v = fma(kx[o], u[o + 1], v);
+    v = fma(kx[o - 1], u[o - 1], v);
+    v = fma(ky[o], u[o + L.pitch], v);
+    v = fma(ky[o - L.pitch], u[o - L.pitch], v);
+    v = fma(kz[o], u[o + L.plane], v);
+    return fma(kz[o - L.plane], u[o - L.plane], v);
+}
+
+// Inner nodes numbered densely, one per thread, then the border nodes
+// (node_order.cuh): thousands of short CTAs without idle lanes.  Columns of 16
+// planes per CTA left most SMs with two CTAs at 97 x 90 x 83 (20.2 us a step
+// against 12.3 here; the FP64 pipe needs 8).
+__global__ void __launch_bounds__(MARCH_THREADS)
 k_forward(const double* __restrict__ u, double* __restrict__ un, const double* __restrict__ kx,
-          const double* __restrict__ ky, const double* __restrict__ kz, const double* __restrict__ dg, Layout L) {
+          const double* __restrict__ ky, const double* __restrict__ kz, const double* __restrict__ dg, Layout L,
+          const __grid_constant__ NodeOrder order, uint32_t inner_ctas) {
+    int x, y, z;
+    if (blockIdx.x < inner_ctas) {
+        const uint32_t m = blockIdx.x * MARCH_THREADS + threadIdx.x;
+        if (m >= order.n_inner) return;
+        inner_node(order, m, x, y, z);
+        const long long o = L.idx(x, y, z);
+        un[o] = forward_node(u, kx, ky, kz, dg, L, o);
+    } else {
+        const uint32_t m = (blockIdx.x - inner_ctas) * MARCH_THREADS + threadIdx.x;
+        if (m >= order.n_border) return;
+        border_node(order, m, x, y, z);
+        const long long o = L.idx(x, y, z);
+        un[o] = u[o];
+    }
+}
+
+// The same by columns, for grids of 2^31 nodes and more (node numbers are
+// 32-bit).
+__global__ void __launch_bounds__(AX * AY)
+k_forward_big(const double* __restrict__ u, double* __restrict__ un, const double* __restrict__ kx,
+              const double* __restrict__ ky, const double* __restrict__ kz, const double* __restrict__ dg, Layout L) {
     const int x = blockIdx.x * AX + threadIdx.x, y = blockIdx.y * AY + threadIdx.y;
     if (x >= L.nx || y >= L.ny) return;
     const bool colb = x == 0 || y == 0 || x == L.nx - 1 || y == L.ny - 1;
     const int zb = blockIdx.z * 16, ze = min(zb + 16, L.nz);
     for (int z = zb; z < ze; ++z) {
         const long long o = L.idx(x, y, z);
-        const double uc = u[o];
-        if (colb || z == 0 || z == L.nz - 1) {
-            un[o] = uc;
-            continue;
-        }
-        double v = dg[o] * uc;
-        v = fma(kx[o], u[o + 1], v);
-        v = fma(kx[o - 1], u[o - 1], v);
-        v = fma(ky[o], u[o + L.pitch], v);
-        v = fma(ky[o - L.pitch], u[o - L.pitch], v);
-        v = fma(kz[o], u[o + L.plane], v);
-        v = fma(kz[o - L.plane], u[o - L.plane], v);
-        un[o] = v;
+        un[o] = colb || z == 0 || z == L.nz - 1 ? u[o] : forward_node(u, kx, ky, kz, dg, L, o);
     }
 }
 
@@ -238,7 +266,7 @@ __global__ void k_prep_x2(const double* __restrict__ k, float2* __restrict__ kx,
 // faces (border nodes copied), with every operand staged through TMA: a
 // column-per-thread kernel with plain loads stalled on their latency (ncu:
 // long-scoreboard stalls, 0.63 of HBM).  A CTA owns an FTX x FTY column tile
-// and marches FZ_ planes; per plane one mbarrier covers five boxes -- u with
+// and marches a chunk of planes; per plane one mbarrier covers five boxes -- u with
 // a one-node halo (x from x0-2 for 16-byte alignment), the x faces from
 // x0-2, the y faces from row y0-1, the z faces and the diagonal of the tile
 // -- in a ring of four planes (planes z, z+1 in use, z+2, z+3 in flight).
@@ -246,7 +274,7 @@ __global__ void k_prep_x2(const double* __restrict__ k, float2* __restrict__ kx,
 // products are accumulated in a fixed order (diagonal, +x, -x, +y, -y, +z,
 // -z), which the reverse sweep's recomputation repeats bit for bit.  Every
 // wait is bounded (status word, drain, return).
-constexpr int FTX = 32, FTY = 8, FZ_ = 32, FNS = 4;
+constexpr int FTX = 32, FTY = 8, FNS = 4;
 constexpr int FUW = FTX + 4, FUH = FTY + 2;             // u box: x0-2 .. x0+33, y0-1 .. y0+8
 constexpr int FXW = FTX + 4, FXH = FTY;                 // x faces: x0-2 .. x0+33, own rows
 constexpr int FYW = FTX, FYH = FTY + 1;                 // y faces: own columns, y0-1 .. y0+7
@@ -262,12 +290,12 @@ __global__ void __launch_bounds__(FTX * FTY)
 k_forward_x2_tma(const __grid_constant__ CUtensorMap tu, const __grid_constant__ CUtensorMap tkx,
                  const __grid_constant__ CUtensorMap tky, const __grid_constant__ CUtensorMap tkz,
                  const __grid_constant__ CUtensorMap tdg, float2* __restrict__ un, Layout L,
-                 int* __restrict__ status) {
+                 int zchunk, int* __restrict__ status) {
     extern __shared__ __align__(128) float2 fsm[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(fsm + FNS * FSLOT);
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * FTX + tx;
     const int x0 = blockIdx.x * FTX, y0 = blockIdx.y * FTY;
-    const int z0 = blockIdx.z * FZ_, z1 = min(z0 + FZ_, L.nz);
+    const int z0 = blockIdx.z * zchunk, z1 = min(z0 + zchunk, L.nz);
     if (__syncthreads_or(tid == 0 && *(volatile int*)status != 0)) return;
     if (tid == 0) {
         for (int b = 0; b < FNS; ++b) scafes::mbar_init(&bar[b], 1);
@@ -359,7 +387,7 @@ k_forward_x2_tma(const __grid_constant__ CUtensorMap tu, const __grid_constant__
 // node instead of 104).  A face to a node outside the grid or between two
 // border nodes contributes nothing: lambda is zero there.
 // The operands are staged through TMA on the forward step's tile (RTX x
-// RTY columns, RZ_ planes, a ring of four planes on four mbarriers).  Per
+// RTY columns, a chunk of planes, a ring of four planes on four mbarriers).  Per
 // plane one mbarrier covers six boxes: lambda and u with a one-node halo
 // (x from x0-2), the x faces from x0-2, the y faces from row y0-1, the z
 // faces and the diagonal.  lambda, u and the z face of the plane below and
@@ -367,7 +395,7 @@ k_forward_x2_tma(const __grid_constant__ CUtensorMap tu, const __grid_constant__
 // read with plain loads one plane ahead and written in place.
 // Out-of-range box elements read as zero.  Every wait is bounded (status
 // word, drain, return).
-constexpr int RTX = FTX, RTY = FTY, RZ_ = FZ_, RNS = FNS;
+constexpr int RTX = FTX, RTY = FTY, RNS = FNS;
 constexpr int RLW = FUW, RLH = FUH;                       // lambda and u boxes: the forward's u box
 constexpr int RO_L = 0, RO_U = pad16(RLW * RLH), RO_X = RO_U + pad16(RLW * RLH);
 constexpr int RO_Y = RO_X + pad16(FXW * FXH), RO_Z = RO_Y + pad16(FYW * FYH), RO_D = RO_Z + pad16(FKW * FKH);
@@ -421,7 +449,7 @@ k_adjoint_x2_tma(const __grid_constant__ CUtensorMap tl, const __grid_constant__
                  const __grid_constant__ CUtensorMap tkx, const __grid_constant__ CUtensorMap tky,
                  const __grid_constant__ CUtensorMap tkz, const __grid_constant__ CUtensorMap tdg,
                  E* __restrict__ lamn, float2* __restrict__ g, E* __restrict__ bnd, float2 hx2,
-                 float2 hy2, float2 hz2, Layout L, int* __restrict__ status) {
+                 float2 hy2, float2 hz2, Layout L, int zchunk, int* __restrict__ status) {
     constexpr bool F64 = std::is_same<E, double>::value;
     extern __shared__ __align__(128) unsigned char rsm_raw[];
     E* rsm = reinterpret_cast<E*>(rsm_raw);
@@ -429,7 +457,7 @@ k_adjoint_x2_tma(const __grid_constant__ CUtensorMap tl, const __grid_constant__
     uint64_t* bar = reinterpret_cast<uint64_t*>(rsm + RNS * RSLOT + (F64 ? 4 * RPAIR : 0));
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * RTX + tx;
     const int x0 = blockIdx.x * RTX, y0 = blockIdx.y * RTY;
-    const int z0 = blockIdx.z * RZ_, z1 = min(z0 + RZ_, L.nz);
+    const int z0 = blockIdx.z * zchunk, z1 = min(z0 + zchunk, L.nz);
     if (__syncthreads_or(tid == 0 && *(volatile int*)status != 0)) return;
     if (tid == 0) {
         for (int b = 0; b < RNS; ++b) scafes::mbar_init(&bar[b], 1);
@@ -737,13 +765,28 @@ int coefficient_maps(scafes_adj* a) {
     return SCAFES_OK;
 }
 
+// Planes per CTA of the TMA steps: 32, which amortise the two halo planes,
+// fewer while the grid would not fill the SMs with `per_sm` CTAs each (at 97 x
+// 90 x 83, 32 planes were 144 CTAs of 8 warps for 152 SMs).
+int chunk_planes(const Layout& L, int per_sm) {
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const long long tiles = (long long)((L.nx + FTX - 1) / FTX) * ((L.ny + FTY - 1) / FTY);
+    const long long chunks = std::max(1LL, (long long)sms * per_sm / tiles);
+    long long zc = std::min(32LL, std::max(4LL, (L.nz + chunks - 1) / chunks));
+    while ((L.nz + zc - 1) / zc > 65535) zc <<= 1;  // grid.z limit
+    return (int)zc;
+}
+
 int fwd_x2_tma(scafes_adj* a, const double* src, double* dst) {
     if (int rc = coefficient_maps(a)) return rc;
     CUtensorMap mu;
     if (int rc = state_map(a, src, BOX_HALO, &mu)) return rc;
-    const dim3 grid((a->L.nx + FTX - 1) / FTX, (a->L.ny + FTY - 1) / FTY, (a->L.nz + FZ_ - 1) / FZ_);
+    const int zc = chunk_planes(a->L, (int)(227 * 1024 / FSMEM));
+    const dim3 grid((a->L.nx + FTX - 1) / FTX, (a->L.ny + FTY - 1) / FTY, (a->L.nz + zc - 1) / zc);
     k_forward_x2_tma<<<grid, dim3(FTX, FTY), FSMEM, a->stream>>>(mu, a->cmaps[0], a->cmaps[1], a->cmaps[2],
-                                                                  a->cmaps[3], P2(dst), a->L, a->status);
+                                                                  a->cmaps[3], P2(dst), a->L, zc, a->status);
     return SCAFES_OK;
 }
 
@@ -762,8 +805,14 @@ int fwd(scafes_adj* a, const double* src, double* dst) {
     if (pairs(a)) {
         const int rc = fwd_x2_tma(a, src, dst);
         if (rc) return rc;
-    } else
-        k_forward<<<grid3(a->L), dim3(AX, AY), 0, a->stream>>>(src, dst, a->kx, a->ky, a->kz, a->dg, a->L);
+    } else if ((long long)a->L.nx * a->L.ny * a->L.nz < (1LL << 31)) {
+        const NodeOrder o = make_node_order(a->L.nx, a->L.ny, a->L.nz, 1);
+        const uint32_t inner = (o.n_inner + MARCH_THREADS - 1) / MARCH_THREADS;
+        k_forward<<<inner + (o.n_border + MARCH_THREADS - 1) / MARCH_THREADS, MARCH_THREADS, 0, a->stream>>>(
+            src, dst, a->kx, a->ky, a->kz, a->dg, a->L, o, inner);
+    } else {
+        k_forward_big<<<grid3(a->L), dim3(AX, AY), 0, a->stream>>>(src, dst, a->kx, a->ky, a->kz, a->dg, a->L);
+    }
     ATRY(a, cudaGetLastError());
     ++a->fwd_steps;
     return SCAFES_OK;
@@ -867,7 +916,8 @@ int adj_step(Rev& R, const double* u_t) {
     CUtensorMap ml, mu;
     if (int rc = state_map(a, a->lam[R.cur], BOX_HALO, &ml)) return rc;
     if (int rc = state_map(a, u_t, BOX_HALO, &mu)) return rc;
-    const dim3 grid((a->L.nx + RTX - 1) / RTX, (a->L.ny + RTY - 1) / RTY, (a->L.nz + RZ_ - 1) / RZ_);
+    const int zc = chunk_planes(a->L, (int)(227 * 1024 / (pairs(a) ? RSMEM : RSMEM_F64)));
+    const dim3 grid((a->L.nx + RTX - 1) / RTX, (a->L.ny + RTY - 1) / RTY, (a->L.nz + zc - 1) / zc);
     auto half = [](double w) {
         const f2 p = split_double(0.5 * w);
         return make_float2(p.hi, p.lo);
@@ -875,11 +925,11 @@ int adj_step(Rev& R, const double* u_t) {
     if (pairs(a))
         k_adjoint_x2_tma<float2><<<grid, dim3(RTX, RTY), RSMEM, a->stream>>>(
             ml, mu, a->cmaps[0], a->cmaps[1], a->cmaps[2], a->cmaps[3], P2(a->lam[R.cur ^ 1]), P2(a->gx),
-            P2(a->bnd), half(a->w[0]), half(a->w[1]), half(a->w[2]), a->L, a->status);
+            P2(a->bnd), half(a->w[0]), half(a->w[1]), half(a->w[2]), a->L, zc, a->status);
     else
         k_adjoint_x2_tma<double><<<grid, dim3(RTX, RTY), RSMEM_F64, a->stream>>>(
             ml, mu, a->cmaps[0], a->cmaps[1], a->cmaps[2], a->cmaps[3], a->lam[R.cur ^ 1], P2(a->gx), a->bnd,
-            half(a->w[0]), half(a->w[1]), half(a->w[2]), a->L, a->status);
+            half(a->w[0]), half(a->w[1]), half(a->w[2]), a->L, zc, a->status);
     ATRY(a, cudaGetLastError());
     R.cur ^= 1;
     ++a->adj_steps;
