@@ -63,4 +63,49 @@ SCAFES_HD uint64_t dadd_same_sign_bits(uint64_t a, uint64_t b, bool& ok) {
     return ((uint64_t)((e + c - 1u) << 20) << 32) + r;
 }
 
+// a + b for operands of any signs: RN of the exact sum where `ok`, which
+// holds when the exponents are at most 9 apart or one operand is zero (or
+// subnormal, and then lost below the other's last bit), and the larger
+// exponent field is in [64, 2045] or the sum is zero.  For the differences of
+// neighbours in fields that change sign.  The significands are aligned to the
+// larger exponent with 9 guard bits (so nothing is shifted out), added as
+// signed 64-bit numbers, and the magnitude is normalised by its leading
+// zeros and rounded half to even.  (-0) + (-0) gives +0.
+SCAFES_HD uint64_t dadd_bits(uint64_t a, uint64_t b, bool& ok) {
+    const uint32_t ah = (uint32_t)(a >> 32), al = (uint32_t)a;
+    const uint32_t bh = (uint32_t)(b >> 32), bl = (uint32_t)b;
+    const uint32_t ta = ah & 0x7ff00000u, tb = bh & 0x7ff00000u;
+    const uint32_t e = ta > tb ? ta : tb, m = ta > tb ? tb : ta;
+    const uint32_t sa = (e - ta) >> 20, sb = (e - tb) >> 20;
+#if defined(__CUDA_ARCH__)
+    // PTX shifts clamp: 0 from 32 on.
+    uint32_t pa, pb;
+    asm("shr.u32 %0, 512, %1;" : "=r"(pa) : "r"(sa));
+    asm("shr.u32 %0, 512, %1;" : "=r"(pb) : "r"(sb));
+#else
+    const uint32_t pa = sa < 32 ? 512u >> sa : 0u, pb = sb < 32 ? 512u >> sb : 0u;
+#endif
+    // The hidden bit, absent with a zero exponent field.
+    const uint32_t mah = (ah & 0x000fffffu) | (ta < 0x00100000u ? ta : 0x00100000u);
+    const uint32_t mbh = (bh & 0x000fffffu) | (tb < 0x00100000u ? tb : 0x00100000u);
+    const uint64_t A = (uint64_t)al * pa + ((uint64_t)(mah * pa) << 32);
+    const uint64_t B = (uint64_t)bl * pb + ((uint64_t)(mbh * pb) << 32);
+    const int64_t d = (int32_t)(ah ^ bh) >> 31;  // all ones when the signs differ
+    const int64_t s = (int64_t)(A + ((B ^ (uint64_t)d) - (uint64_t)d));
+    const int64_t n = s >> 63;
+    const uint64_t mag = (uint64_t)((s ^ n) - n);
+#if defined(__CUDA_ARCH__)
+    const int lz = __clzll((long long)mag);
+#else
+    const int lz = mag ? __builtin_clzll(mag) : 64;
+#endif
+    uint64_t r = mag << ((lz - 1) & 63);  // leading bit at 62
+    r += (uint64_t)(0x1ffu + (((uint32_t)r >> 10) & 1u));
+    r >>= 10;
+    const uint32_t top = e - 0x04000000u;  // exponent field - 64
+    ok = (e - m <= 0x00900000u || m == 0u) && (top <= 0x7bd00000u || mag == 0u);
+    const uint32_t hi = ((uint32_t)(r >> 32) + e + ((uint32_t)(1 - lz) << 20)) | ((ah ^ (uint32_t)n) & 0x80000000u);
+    return mag ? ((uint64_t)hi << 32) | (uint32_t)r : 0u;
+}
+
 }  // namespace scafes

@@ -12,18 +12,22 @@
 // schemes here follow the textbook forms written out in the oracle
 // (orc_lame, orc_yee), which the tests use as the reference.
 //
-// Both are FP64-issue-bound on GB300 (Lame: ~57 FP64 operations per node,
-// Yee: ~24 per cell and step), so the kernels read neighbours straight from
-// global memory through L1 instead of staging tiles: one thread per (x, y)
-// column marches a chunk of 16 z-planes.  The FP32-pair Lame kernel
+// Both are bound by the FP64 pipe on GB300 in FP64 (Lame: 44 operations per
+// node, Yee: 24 per cell and step), so the kernels read neighbours straight
+// from global memory through L1 instead of staging tiles, and move part of
+// the sums to the integer pipe (dadd_int.cuh).  The FP32-pair Lame kernel
 // (k_lame_x2_tma) stages the three components through TMA instead (its
 // pair arithmetic needs the loads' latency hidden); FP32 and FP32-pair Yee
 // run the fused one-pass step (k_yee_tma) below.
-#include <cstdarg>
+#include <algorithm>
 #include <cmath>
+#include <cstdarg>
+#include <cstring>
 #include <cstdio>
 #include <string>
 
+#include "dadd_int.cuh"
+#include "node_order.cuh"
 #include "scafes_common.cuh"
 #include "star7.cuh"
 #include "tma.cuh"
@@ -44,7 +48,9 @@ struct LameCoef {
     double b[3][3];   // b[c][q]: weight of d_cq u_q (includes tau^2/rho/(4 h_c h_q))
 };
 
-// u_new (written over uprev) = 2u - uprev + sum ... on inner nodes; 0 on border.
+// u_new (written over uprev) = 2u - uprev + sum ... on inner nodes; 0 on
+// border.  For grids of 2^31 nodes and more only (k_lame_march numbers nodes
+// in 32 bits).
 __global__ void __launch_bounds__(MX * MY)
 k_lame(const double* __restrict__ u, double* __restrict__ up, LameCoef K, Layout L, long long comp) {
     const int x = blockIdx.x * MX + threadIdx.x, y = blockIdx.y * MY + threadIdx.y;
@@ -84,42 +90,260 @@ k_lame(const double* __restrict__ u, double* __restrict__ up, LameCoef K, Layout
     }
 }
 
-// Yee H half step (see orc_yee for the staggering).
-template <class T>
-__global__ void __launch_bounds__(MX * MY)
-k_yee_h(const T* __restrict__ ex, const T* __restrict__ ey, const T* __restrict__ ez, T* __restrict__ hx,
-        T* __restrict__ hy, T* __restrict__ hz, Layout L, T ch) {
-    const int x = blockIdx.x * MX + threadIdx.x, y = blockIdx.y * MY + threadIdx.y;
-    if (x >= L.nx || y >= L.ny) return;
-    const int z0 = blockIdx.z * MZ, z1 = min(z0 + MZ, L.nz);
-    for (int z = z0; z < z1; ++z) {
-        const long long m = L.idx(x, y, z);
-        const bool xi = x + 1 < L.nx, yi = y + 1 < L.ny, zi = z + 1 < L.nz;
-        if (yi && zi) hx[m] -= ch * ((ez[m + L.pitch] - ez[m]) - (ey[m + L.plane] - ey[m]));
-        if (xi && zi) hy[m] -= ch * ((ex[m + L.plane] - ex[m]) - (ez[m + 1] - ez[m]));
-        if (xi && yi) hz[m] -= ch * ((ey[m + 1] - ey[m]) - (ex[m + L.pitch] - ex[m]));
+// a + b and a - b as FMAs (same rounding).
+__device__ __forceinline__ double fadd(double a, double b, double one) { return fma(a, one, b); }
+__device__ __forceinline__ double fsub(double a, double b, double mone) { return fma(b, mone, a); }
+
+// N sums (NEG: differences) of a[i] and b[i]: the first NI on the integer pipe
+// (dadd_bits: the FP64 adder's result), the others as DFMAs.  A warp with a
+// lane outside the integer adder's range takes those NI in FP64 too, in a
+// call: predicated inline they would hold the FP64 pipe in every warp.
+template <int N>
+struct Doubles {
+    double v[N];
+};
+template <int N, bool NEG>
+__device__ __noinline__ Doubles<N> fp64_combine(Doubles<N> a, Doubles<N> b) {
+    Doubles<N> r;
+#pragma unroll
+    for (int i = 0; i < N; ++i) r.v[i] = NEG ? a.v[i] - b.v[i] : a.v[i] + b.v[i];
+    return r;
+}
+template <int NI, bool NEG, int N>
+__device__ __forceinline__ void combine(const double (&a)[N], const double (&b)[N], double (&d)[N], double one) {
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+        bool o;
+        const uint64_t r = dadd_bits((uint64_t)__double_as_longlong(a[i]),
+                                     (uint64_t)__double_as_longlong(b[i]) ^ (NEG ? 1ull << 63 : 0ull), o);
+        d[i] = __longlong_as_double((long long)r);
+        ok = ok && o;
+    }
+#pragma unroll
+    for (int i = NI; i < N; ++i) d[i] = NEG ? fma(b[i], -one, a[i]) : fma(b[i], one, a[i]);
+    if constexpr (NI > 0) {
+        if (__any_sync(__activemask(), !ok)) {
+            Doubles<NI> x, y;
+#pragma unroll
+            for (int i = 0; i < NI; ++i) x.v[i] = a[i], y.v[i] = b[i];
+            const Doubles<NI> r = fp64_combine<NI, NEG>(x, y);
+#pragma unroll
+            for (int i = 0; i < NI; ++i) d[i] = r.v[i];
+        }
     }
 }
 
-// Yee E step with PEC walls and the soft current source.
-template <class T>
-__global__ void __launch_bounds__(MX * MY)
-k_yee_e(T* __restrict__ ex, T* __restrict__ ey, T* __restrict__ ez, const T* __restrict__ hx,
-        const T* __restrict__ hy, const T* __restrict__ hz, Layout L, T ch, long long src, T src_val) {
-    const int x = blockIdx.x * MX + threadIdx.x, y = blockIdx.y * MY + threadIdx.y;
-    if (x >= L.nx || y >= L.ny) return;
-    const int z0 = blockIdx.z * MZ, z1 = min(z0 + MZ, L.nz);
-    const bool xin = x > 0 && x + 1 < L.nx, yin = y > 0 && y + 1 < L.ny;
-    for (int z = z0; z < z1; ++z) {
-        const long long m = L.idx(x, y, z);
-        const bool zin = z > 0 && z + 1 < L.nz;
-        if (x + 1 < L.nx && yin && zin) ex[m] += ch * ((hz[m] - hz[m - L.pitch]) - (hy[m] - hy[m - L.plane]));
-        if (y + 1 < L.ny && xin && zin) ey[m] += ch * ((hx[m] - hx[m - L.plane]) - (hz[m] - hz[m - 1]));
-        if (z + 1 < L.nz && xin && yin) {
-            T v = ez[m] + ch * ((hy[m] - hy[m - 1]) - (hx[m] - hx[m - L.pitch]));
-            if (m == src) v -= src_val;
-            ez[m] = v;
+// The FP64 step.  Written out per node it takes 54 FP64 operations, 24 of
+// them for the six mixed derivatives; but with D_q v = v(+q) - v(-q), the
+// mixed terms of component c are one difference along c of
+//   S_c = sum over q != c of k_q D_q u_q,
+// and the D_q are shared between the components: 14 operations (three D, two
+// products, S_x, S_y, S_z, and a difference and an FMA per component), 44 in
+// all.  S_z stays with its column; S_x and S_y go through shared memory, the
+// tile's threads also computing the S of the nodes around it.  The nine
+// second differences' sums u(+p) + u(-p) go to the integer pipe, which leaves
+// 35; the other sums and differences are FMAs with a one in a register: GB300
+// issues a DFMA in 16 clocks of an SM and a DADD or DMUL in 19.
+// A CTA marches a few planes of a column tile that fits the grid's width
+// (make_column_tile); CTAs in front zero the border nodes of u^{n+1}.
+// us per step at 129 x 111 x 101: columns of 16 planes, written out per node
+// 252; this split 141; with 3, 6, 9 integer sums 134, 127, 119 (FP64 pipe 79 %
+// busy, ALU 35 %); with integer D as well 119 - 124.  Error against a
+// 113-bit run (60 - 120 steps, three grids): 0.96 of the written-out form's.
+struct LameMarch {
+    const double* u;
+    double* up;
+    long long comp;
+    double a[3][3];  // as LameCoef
+    double k[3];     // k_q = tau^2/rho (lambda + mu) / (4 h_q)
+    double ih[3];    // 1 / h_c
+    double one;
+    Layout L;
+    NodeOrder o;
+    ColumnTile ct;
+    FastDiv tx, txy;
+    uint32_t border_ctas;
+    int zchunk;
+};
+
+constexpr int LSX = MARCH_THREADS + 2 * 16, LSY = MARCH_THREADS + 2 * 64;  // S with its halo: h <= 16, w <= 64
+
+__global__ void __launch_bounds__(MARCH_THREADS, 3) k_lame_march(const __grid_constant__ LameMarch A) {
+    __shared__ double sx[2][LSX], sy[2][LSY];
+    const Layout& L = A.L;
+    if (blockIdx.x < A.border_ctas) {
+        const uint32_t m = blockIdx.x * MARCH_THREADS + threadIdx.x;
+        if (m >= A.o.n_border) return;
+        int x, y, z;
+        border_node(A.o, m, x, y, z);
+        const long long o = L.idx(x, y, z);
+        for (int c = 0; c < 3; ++c) A.up[o + c * A.comp] = 0.0;
+        return;
+    }
+    const uint32_t q = blockIdx.x - A.border_ctas;
+    const uint32_t kz = fastdiv(q, A.txy), r = q - kz * A.txy.d, jt = fastdiv(r, A.tx);
+    const int W = (int)A.ct.w.d, H = A.ct.h;
+    const int x0 = (int)(r - jt * A.tx.d) * W + 1, y0 = (int)jt * H + 1;
+    const int row = (int)fastdiv(threadIdx.x, A.ct.w), col = (int)threadIdx.x - row * W;
+    const bool main = row < H;
+    // Threads beyond the grid compute on its last nodes and write nothing;
+    // those on its last column and row provide S only.
+    const int x = min(x0 + col, L.nx - 1), y = min(y0 + row, L.ny - 1);
+    const bool live = main && x0 + col < L.nx - 1 && y0 + row < L.ny - 1;
+    const int z0 = (int)kz * A.zchunk + 1, z1 = min(z0 + A.zchunk, L.nz - 1);
+    const long long py = L.pitch, pz = L.plane;
+    const int xp = x < L.nx - 1 ? 1 : 0;
+    const long long yp = y < L.ny - 1 ? py : 0;
+    // One S node around the tile per thread: columns -1 and W of its rows
+    // (S_x), then rows -1 and H of its columns (S_y).
+    const int h = (int)threadIdx.x;
+    const bool hx = h < 2 * H, hy = !hx && h < 2 * H + 2 * W;
+    const int g = h - 2 * H;
+    const int hcol = hx ? ((h & 1) ? W : -1) : g >> 1, hrow = hx ? h >> 1 : ((g & 1) ? H : -1);
+    const int hxx = min(x0 + hcol, L.nx - 1), hyy = min(y0 + hrow, L.ny - 1);
+    const int hdx = hxx < L.nx - 1 && hxx > 0 ? 1 : 0;
+    const long long hdy = hyy < L.ny - 1 && hyy > 0 ? py : 0;
+    const double one = A.one, mone = -one;
+    const double* u0 = A.u;
+    const double* u1 = A.u + A.comp;
+    const double* u2 = A.u + 2 * A.comp;
+    long long o = L.idx(x, y, z0), ho = (hx || hy) ? L.idx(hxx, hyy, z0) : 0;
+    // k_x D_x u, k_y D_y v and their sum S_z at a node.
+    auto dxy = [&](long long m, double& qx, double& qy) {
+        qx = A.k[0] * fsub(u0[m + xp], u0[m - 1], mone);
+        qy = A.k[1] * fsub(u1[m + yp], u1[m - py], mone);
+        return fadd(qx, qy, one);
+    };
+    double qx, qy, szb, szc, wb = u2[o - pz], wc = u2[o];
+    szb = dxy(o - pz, qx, qy);
+    szc = dxy(o, qx, qy);
+    int p = 0;
+    for (int z = z0; z < z1; ++z, o += pz, ho += pz, p ^= 1) {
+        const double wa = u2[o + pz];
+        const double dz = fsub(wa, wb, mone);
+        if (main) {
+            sx[p][row * (W + 2) + col + 1] = fma(A.k[2], dz, qy);
+            sy[p][(row + 1) * W + col] = fma(A.k[2], dz, qx);
         }
+        if (hx) {
+            const double d = fsub(u2[ho + pz], u2[ho - pz], mone);
+            const double e = fsub(u1[ho + hdy], u1[ho - hdy], mone);
+            sx[p][hrow * (W + 2) + hcol + 1] = fma(A.k[2], d, A.k[1] * e);
+        } else if (hy) {
+            const double d = fsub(u2[ho + pz], u2[ho - pz], mone);
+            const double e = fsub(u0[ho + hdx], u0[ho - hdx], mone);
+            sy[p][(hrow + 1) * W + hcol] = fma(A.k[2], d, A.k[0] * e);
+        }
+        const double sza = dxy(o + pz, qx, qy);
+        double acc[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double* uc = A.u + c * A.comp;
+            const double v = c == 2 ? wc : uc[o];
+            acc[c] = fma(2.0, v, -A.up[o + c * A.comp]);
+            const double sa[3] = {uc[o + yp], c == 2 ? wa : uc[o + pz], uc[o + xp]};
+            const double sb[3] = {uc[o - py], c == 2 ? wb : uc[o - pz], uc[o - 1]};
+            double s[3];
+            combine<3, false>(sa, sb, s, one);
+            const double lx = fma(-2.0, v, s[2]), ly = fma(-2.0, v, s[0]), lz = fma(-2.0, v, s[1]);
+            acc[c] = fma(A.a[c][0], lx, acc[c]);
+            acc[c] = fma(A.a[c][1], ly, acc[c]);
+            acc[c] = fma(A.a[c][2], lz, acc[c]);
+        }
+        __syncthreads();  // S of plane z is complete; the other buffer is free
+        if (live) {
+            const double* a = &sx[p][row * (W + 2) + col + 1];
+            const double* b = &sy[p][(row + 1) * W + col];
+            A.up[o] = fma(A.ih[0], fsub(a[1], a[-1], mone), acc[0]);
+            A.up[o + A.comp] = fma(A.ih[1], fsub(b[W], b[-W], mone), acc[1]);
+            A.up[o + 2 * A.comp] = fma(A.ih[2], fsub(sza, szb, mone), acc[2]);
+        }
+        wb = wc;
+        wc = wa;
+        szb = szc;
+        szc = sza;
+    }
+}
+
+// Yee steps in FP64 (see orc_yee for the staggering): one node per thread
+// over the dense numbering of the grid, so that no lane idles beyond a row's
+// end and thousands of short CTAs balance the SMs; the neighbours come
+// through L1.  Bound by the FP64 pipe: 12 operations per node and half step,
+// of which the kYeeInt differences along y and z go to the integer pipe (the
+// x differences change sign inside a warp more often than the others and
+// would send it to the fallback).  us per step at 128 x 120 x 113 (both
+// halves): columns of 16 planes 130; dense 84; with 2, 3, 4, 5, 6 integer
+// differences 74, 68, 64, 73, 82 (then both pipes are 55 - 60 % busy).
+constexpr int kYeeInt = 4;
+
+struct YeeFlat {
+    Layout L;
+    FastDiv nx, nxy;
+    uint32_t nodes;  // of this launch, from plane z0 on
+    int z0;
+    double ch, one;
+};
+
+__device__ __forceinline__ bool yee_node(const YeeFlat& A, int& x, int& y, int& z) {
+    const uint32_t m = blockIdx.x * (uint32_t)MARCH_THREADS + threadIdx.x;
+    const uint32_t k = fastdiv(m, A.nxy), r = m - k * A.nxy.d, j = fastdiv(r, A.nx);
+    x = (int)(r - j * A.nx.d);
+    y = (int)j;
+    z = (int)k + A.z0;
+    return m < A.nodes;
+}
+
+__global__ void __launch_bounds__(MARCH_THREADS, 6)
+k_yee_h(const double* __restrict__ ex, const double* __restrict__ ey, const double* __restrict__ ez,
+        double* __restrict__ hx, double* __restrict__ hy, double* __restrict__ hz,
+        const __grid_constant__ YeeFlat A) {
+    int x, y, z;
+    if (!yee_node(A, x, y, z)) return;
+    const Layout& L = A.L;
+    const long long m = L.idx(x, y, z);
+    const bool xi = x + 1 < L.nx, yi = y + 1 < L.ny, zi = z + 1 < L.nz;
+    // A neighbour beyond the grid reads the node itself; nothing is stored there.
+    const long long mx = m + (xi ? 1 : 0), my = m + (yi ? L.pitch : 0), mz = m + (zi ? L.plane : 0);
+    const double c = -A.ch, mone = -A.one;
+    const double ex0 = ex[m], ey0 = ey[m], ez0 = ez[m];
+    // The x differences last (see kYeeInt).
+    const double a[6] = {ez[my], ey[mz], ex[mz], ex[my], ez[mx], ey[mx]};
+    const double b[6] = {ez0, ey0, ex0, ex0, ez0, ey0};
+    double d[6];
+    combine<kYeeInt, true>(a, b, d, A.one);
+    if (yi && zi) hx[m] = fma(c, fsub(d[0], d[1], mone), hx[m]);
+    if (xi && zi) hy[m] = fma(c, fsub(d[2], d[4], mone), hy[m]);
+    if (xi && yi) hz[m] = fma(c, fsub(d[5], d[3], mone), hz[m]);
+}
+
+// Out of line: inline, the compiler would predicate the one node's
+// subtraction, and a predicated-off FP64 instruction holds the pipe as well.
+__device__ __noinline__ double yee_source(double v, double s) { return v - s; }
+
+// E step with PEC walls and the soft current source.
+__global__ void __launch_bounds__(MARCH_THREADS, 6)
+k_yee_e(double* __restrict__ ex, double* __restrict__ ey, double* __restrict__ ez, const double* __restrict__ hx,
+        const double* __restrict__ hy, const double* __restrict__ hz, const __grid_constant__ YeeFlat A,
+        long long src, double src_val) {
+    int x, y, z;
+    if (!yee_node(A, x, y, z)) return;
+    const Layout& L = A.L;
+    const long long m = L.idx(x, y, z);
+    const bool xin = x > 0 && x + 1 < L.nx, yin = y > 0 && y + 1 < L.ny, zin = z > 0 && z + 1 < L.nz;
+    const long long mx = m - (x > 0 ? 1 : 0), my = m - (y > 0 ? L.pitch : 0), mz = m - (z > 0 ? L.plane : 0);
+    const double c = A.ch, mone = -A.one;
+    const double hx0 = hx[m], hy0 = hy[m], hz0 = hz[m];
+    const double a[6] = {hz0, hy0, hx0, hx0, hz0, hy0};
+    const double b[6] = {hz[my], hy[mz], hx[mz], hx[my], hz[mx], hy[mx]};
+    double d[6];
+    combine<kYeeInt, true>(a, b, d, A.one);
+    if (x + 1 < L.nx && yin && zin) ex[m] = fma(c, fsub(d[0], d[1], mone), ex[m]);
+    if (y + 1 < L.ny && xin && zin) ey[m] = fma(c, fsub(d[2], d[4], mone), ey[m]);
+    if (z + 1 < L.nz && xin && yin) {
+        double v = fma(c, fsub(d[5], d[3], mone), ez[m]);
+        if (m == src) v = yee_source(v, src_val);
+        ez[m] = v;
     }
 }
 
@@ -198,7 +422,8 @@ __device__ __forceinline__ float2 pa_result(PAcc acc) {
 // + sum_q b_cq ((u_q(+c+q) - u_q(+c-q)) - (u_q(-c+q) - u_q(-c-q))) - u^{n-1},
 // the FP64 form rearranged with the centre weight d_c = 2 - 2 sum_p a_cp.
 // The three components of u^n are staged by TMA: a CTA owns an LX x LY
-// column tile (LX x LY/2 threads, two rows each) and marches LZ planes; per
+// column tile (LX x LY/2 threads, two rows each) and marches 32 planes (fewer
+// while the grid would not fill the SMs); per
 // input plane one mbarrier covers the three components' boxes with a
 // one-node halo in x and y (x from x0-2 for 16-byte alignment), in a ring
 // of LNS planes: planes z-1, z, z+1 are read from shared memory while the
@@ -206,7 +431,7 @@ __device__ __forceinline__ float2 pa_result(PAcc acc) {
 // written with plain coalesced accesses of the nodes themselves.  The terms
 // come in the order of the FP64 kernel's.  Every wait is bounded (status
 // word, drain, return).
-constexpr int LX = 32, LY = 8, LZ = 32, LNS = 6;
+constexpr int LX = 32, LY = 8, LNS = 6;
 constexpr int LBW = LX + 4, LBH = LY + 2;                     // box: x0-2 .. x0+33, y0-1 .. y0+8
 constexpr int LBOX = (LBW * LBH + 15) / 16 * 16;              // float2 per box, 128-byte multiple
 constexpr int LSLOT = 3 * LBOX;                               // float2 per ring slot
@@ -283,12 +508,12 @@ __device__ __forceinline__ void pa_result2(const PAcc2& acc, float2& o0, float2&
 __global__ void __launch_bounds__(LX * LY / 2)
 k_lame_x2_tma(const __grid_constant__ CUtensorMap t0, const __grid_constant__ CUtensorMap t1,
               const __grid_constant__ CUtensorMap t2, float2* __restrict__ up, LameCoefX2 K, Layout L,
-              long long comp, int* __restrict__ status) {
+              long long comp, int zchunk, int* __restrict__ status) {
     extern __shared__ __align__(128) float2 lsm[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(lsm + LNS * LSLOT);
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * LX + tx;
     const int x0 = blockIdx.x * LX, y0 = blockIdx.y * LY;
-    const int z0 = blockIdx.z * LZ, z1 = min(z0 + LZ, L.nz);
+    const int z0 = blockIdx.z * zchunk, z1 = min(z0 + zchunk, L.nz);
     if (__syncthreads_or(tid == 0 && *(volatile int*)status != 0)) return;
     if (tid == 0) {
         for (int b = 0; b < LNS; ++b) mbar_init(&bar[b], 1);
@@ -699,6 +924,24 @@ int mfail(scafes_mf* h, int code, const char* fmt, ...) {
                          __FILE__, __LINE__);                                                  \
     } while (0)
 
+// z-planes per CTA of the pair Lame step: 32, fewer while the grid would not
+// give every SM the CTAs it can hold.
+int sm_count() {
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms > 0 ? sms : 1;
+}
+
+int lame_zchunk(const Layout& L) {
+    const int sms = sm_count();
+    const long long tiles = (long long)((L.nx + LX - 1) / LX) * ((L.ny + LY - 1) / LY);
+    const long long chunks = std::max(1LL, sms * (long long)(227 * 1024 / LAME_SMEM) / tiles);
+    long long zc = std::min(32LL, std::max(4LL, (L.nz + chunks - 1) / chunks));
+    while ((L.nz + zc - 1) / zc > 65535) zc <<= 1;  // grid.z limit
+    return (int)zc;
+}
+
 // z-planes per CTA of the fused Yee step: long chunks (the plane below a
 // chunk is recomputed), shorter ones while the grid has few column tiles.
 int yee_zchunk(const Layout& L) {
@@ -715,6 +958,9 @@ int yee_zchunk(const Layout& L) {
     while ((L.nz + zc - 1) / zc > 65535) zc <<= 1;  // grid.z limit
     return zc;
 }
+
+// Nodes that 32-bit numbers and fastdiv cover.
+constexpr long long kMaxNumbered = (1LL << 31) - 1;
 
 dim3 mgrid(const Layout& L) { return dim3((L.nx + MX - 1) / MX, (L.ny + MY - 1) / MY, (L.nz + MZ - 1) / MZ); }
 
@@ -913,16 +1159,43 @@ extern "C" int scafes_mf_step(scafes_mf* h, int n_steps) {
             const int rc = lame_maps(h);
             if (rc) return rc;
         }
-        const dim3 lgrid((L.nx + LX - 1) / LX, (L.ny + LY - 1) / LY, (L.nz + LZ - 1) / LZ);
+        LameMarch F{};
+        unsigned lame_ctas = 0;
+        if (!x2 && (long long)L.nx * L.ny * L.nz <= kMaxNumbered) {
+            F.comp = comp;
+            memcpy(F.a, K.a, sizeof(F.a));
+            for (int p = 0; p < 3; ++p) {
+                F.k[p] = s * (lam + mu) / (4.0 * hh[p]);
+                F.ih[p] = 1.0 / hh[p];
+            }
+            F.one = 1.0;
+            F.L = L;
+            F.o = make_node_order(L.nx, L.ny, L.nz, 1);
+            F.ct = make_column_tile(L.nx - 2, L.ny - 2, 1);
+            F.tx = make_fastdiv((uint32_t)F.ct.nx);
+            F.txy = make_fastdiv((uint32_t)(F.ct.nx * F.ct.ny));
+            F.border_ctas = (F.o.n_border + MARCH_THREADS - 1) / MARCH_THREADS;
+            // 8 planes per CTA, fewer while that leaves under two rounds of
+            // resident CTAs (us per step at 129 x 111 x 101 with 4, 6, 8
+            // planes: 123, 119, 123).
+            const long long lt = (long long)F.ct.nx * F.ct.ny, want = 2LL * 3 * sm_count();
+            F.zchunk = (int)std::max(1LL, std::min(8LL, (L.nz - 2) * lt / want));
+            lame_ctas = F.border_ctas + F.ct.nx * F.ct.ny * ((L.nz - 2 + F.zchunk - 1) / F.zchunk);
+        }
+        const int lzc = lame_zchunk(L);
+        const dim3 lgrid((L.nx + LX - 1) / LX, (L.ny + LY - 1) / LY, (L.nz + lzc - 1) / lzc);
         for (int st = 0; st < n_steps; ++st) {
             void* u = field_ptr(h, 3 * h->cur);
             void* up = field_ptr(h, 3 * (h->cur ^ 1));
             if (x2) {
                 const CUtensorMap* t = h->ltm[h->cur];
                 k_lame_x2_tma<<<lgrid, dim3(LX, LY / 2), LAME_SMEM, h->stream>>>(t[0], t[1], t[2], (float2*)up, K2,
-                                                                                L, comp, h->status);
+                                                                                L, comp, lzc, h->status);
             } else {
-                k_lame<<<mgrid(L), dim3(MX, MY), 0, h->stream>>>((const double*)u, (double*)up, K, L, comp);
+                F.u = (const double*)u;
+                F.up = (double*)up;
+                if (lame_ctas) k_lame_march<<<lame_ctas, MARCH_THREADS, 0, h->stream>>>(F);
+                else k_lame<<<mgrid(L), dim3(MX, MY), 0, h->stream>>>((const double*)u, (double*)up, K, L, comp);
             }
             MTRY(h, cudaGetLastError());
             h->cur ^= 1;
@@ -933,6 +1206,14 @@ extern "C" int scafes_mf_step(scafes_mf* h, int n_steps) {
         const double ch = c.tau / hgrid;
         const long long src = L.idx(c.src[0], c.src[1], c.src[2]);
         const double amp = c.p[0], t0 = c.p[1], w = c.p[2], freq = c.p[3];
+        YeeFlat Y;
+        Y.L = L;
+        Y.nx = make_fastdiv((uint32_t)L.nx);
+        Y.nxy = make_fastdiv((uint32_t)L.nx * (uint32_t)L.ny);
+        // Planes per launch: all of them below 2^31 nodes.
+        const int slab = (int)std::min<long long>(L.nz, kMaxNumbered / ((long long)L.nx * L.ny));
+        Y.ch = ch;
+        Y.one = 1.0;
         for (int st = 0; st < n_steps; ++st) {
             const double time = c.t_start + (h->t + 1) * c.tau;
             const double a = (time - t0) / w;
@@ -953,9 +1234,16 @@ extern "C" int scafes_mf_step(scafes_mf* h, int n_steps) {
             } else if (h->esz == 8) {
                 double* f[6];
                 for (int i = 0; i < 6; ++i) f[i] = (double*)field_ptr(h, i);
-                k_yee_h<double><<<mgrid(L), dim3(MX, MY), 0, h->stream>>>(f[0], f[1], f[2], f[3], f[4], f[5], L, ch);
-                k_yee_e<double><<<mgrid(L), dim3(MX, MY), 0, h->stream>>>(f[0], f[1], f[2], f[3], f[4], f[5], L, ch,
-                                                                          src, sv);
+                for (int half = 0; half < 2; ++half)
+                    for (Y.z0 = 0; Y.z0 < L.nz; Y.z0 += slab) {
+                        Y.nodes = (uint32_t)((long long)L.nx * L.ny * std::min(slab, L.nz - Y.z0));
+                        const unsigned ctas = (Y.nodes + MARCH_THREADS - 1) / MARCH_THREADS;
+                        if (half == 0)
+                            k_yee_h<<<ctas, MARCH_THREADS, 0, h->stream>>>(f[0], f[1], f[2], f[3], f[4], f[5], Y);
+                        else
+                            k_yee_e<<<ctas, MARCH_THREADS, 0, h->stream>>>(f[0], f[1], f[2], f[3], f[4], f[5], Y, src,
+                                                                           sv);
+                    }
             } else {
                 const int rc = yee_maps(h);
                 if (rc) return rc;
