@@ -34,6 +34,7 @@
 #include "adjoint.cuh"
 #include "node_order.cuh"
 #include "scafes_common.cuh"
+#include "step_launch.cuh"
 #include "tma.cuh"
 #include "../../include/scafes_gb300.h"
 
@@ -94,20 +95,24 @@ __global__ void __launch_bounds__(MARCH_THREADS)
 k_forward(const double* __restrict__ u, double* __restrict__ un, const double* __restrict__ kx,
           const double* __restrict__ ky, const double* __restrict__ kz, const double* __restrict__ dg, Layout L,
           const __grid_constant__ NodeOrder order, uint32_t inner_ctas) {
+    scafes::step_wait();
     int x, y, z;
     if (blockIdx.x < inner_ctas) {
         const uint32_t m = blockIdx.x * MARCH_THREADS + threadIdx.x;
         if (m >= order.n_inner) return;
         inner_node(order, m, x, y, z);
-        const long long o = L.idx(x, y, z);
+        long long o = L.idx(x, y, z);
+        scafes::after_wait(o);
         un[o] = forward_node(u, kx, ky, kz, dg, L, o);
     } else {
         const uint32_t m = (blockIdx.x - inner_ctas) * MARCH_THREADS + threadIdx.x;
         if (m >= order.n_border) return;
         border_node(order, m, x, y, z);
-        const long long o = L.idx(x, y, z);
+        long long o = L.idx(x, y, z);
+        scafes::after_wait(o);
         un[o] = u[o];
     }
+    scafes::step_next();
 }
 
 // The same by columns, for grids of 2^31 nodes and more (node numbers are
@@ -296,6 +301,7 @@ k_forward_x2_tma(const __grid_constant__ CUtensorMap tu, const __grid_constant__
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * FTX + tx;
     const int x0 = blockIdx.x * FTX, y0 = blockIdx.y * FTY;
     const int z0 = blockIdx.z * zchunk, z1 = min(z0 + zchunk, L.nz);
+    scafes::step_wait();
     if (__syncthreads_or(tid == 0 && *(volatile int*)status != 0)) return;
     if (tid == 0) {
         for (int b = 0; b < FNS; ++b) scafes::mbar_init(&bar[b], 1);
@@ -374,6 +380,7 @@ k_forward_x2_tma(const __grid_constant__ CUtensorMap tu, const __grid_constant__
         uc = ua;
         kzb = kzc;
     }
+    scafes::step_next();
     if (!__syncthreads_and(ok)) fail(issued);
 }
 
@@ -458,6 +465,7 @@ k_adjoint_x2_tma(const __grid_constant__ CUtensorMap tl, const __grid_constant__
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * RTX + tx;
     const int x0 = blockIdx.x * RTX, y0 = blockIdx.y * RTY;
     const int z0 = blockIdx.z * zchunk, z1 = min(z0 + zchunk, L.nz);
+    scafes::step_wait();
     if (__syncthreads_or(tid == 0 && *(volatile int*)status != 0)) return;
     if (tid == 0) {
         for (int b = 0; b < RNS; ++b) scafes::mbar_init(&bar[b], 1);
@@ -607,6 +615,7 @@ k_adjoint_x2_tma(const __grid_constant__ CUtensorMap tl, const __grid_constant__
         plc = pla;
         puc = pua;
     }
+    scafes::step_next();
     if (!__syncthreads_and(ok)) fail(issued);
 }
 
@@ -785,8 +794,8 @@ int fwd_x2_tma(scafes_adj* a, const double* src, double* dst) {
     if (int rc = state_map(a, src, BOX_HALO, &mu)) return rc;
     const int zc = chunk_planes(a->L, (int)(227 * 1024 / FSMEM));
     const dim3 grid((a->L.nx + FTX - 1) / FTX, (a->L.ny + FTY - 1) / FTY, (a->L.nz + zc - 1) / zc);
-    k_forward_x2_tma<<<grid, dim3(FTX, FTY), FSMEM, a->stream>>>(mu, a->cmaps[0], a->cmaps[1], a->cmaps[2],
-                                                                  a->cmaps[3], P2(dst), a->L, zc, a->status);
+    ATRY(a, launch_step(k_forward_x2_tma, grid, dim3(FTX, FTY), FSMEM, a->stream, mu, a->cmaps[0], a->cmaps[1],
+                        a->cmaps[2], a->cmaps[3], P2(dst), a->L, zc, a->status));
     return SCAFES_OK;
 }
 
@@ -808,8 +817,9 @@ int fwd(scafes_adj* a, const double* src, double* dst) {
     } else if ((long long)a->L.nx * a->L.ny * a->L.nz < (1LL << 31)) {
         const NodeOrder o = make_node_order(a->L.nx, a->L.ny, a->L.nz, 1);
         const uint32_t inner = (o.n_inner + MARCH_THREADS - 1) / MARCH_THREADS;
-        k_forward<<<inner + (o.n_border + MARCH_THREADS - 1) / MARCH_THREADS, MARCH_THREADS, 0, a->stream>>>(
-            src, dst, a->kx, a->ky, a->kz, a->dg, a->L, o, inner);
+        const uint32_t border = (o.n_border + MARCH_THREADS - 1) / MARCH_THREADS;
+        ATRY(a, launch_step(k_forward, dim3(inner + border), dim3(MARCH_THREADS), 0, a->stream, src, dst, a->kx, a->ky,
+                            a->kz, a->dg, a->L, o, inner));
     } else {
         k_forward_big<<<grid3(a->L), dim3(AX, AY), 0, a->stream>>>(src, dst, a->kx, a->ky, a->kz, a->dg, a->L);
     }
@@ -923,13 +933,13 @@ int adj_step(Rev& R, const double* u_t) {
         return make_float2(p.hi, p.lo);
     };
     if (pairs(a))
-        k_adjoint_x2_tma<float2><<<grid, dim3(RTX, RTY), RSMEM, a->stream>>>(
+        ATRY(a, launch_step(k_adjoint_x2_tma<float2>, grid, dim3(RTX, RTY), RSMEM, a->stream,
             ml, mu, a->cmaps[0], a->cmaps[1], a->cmaps[2], a->cmaps[3], P2(a->lam[R.cur ^ 1]), P2(a->gx),
-            P2(a->bnd), half(a->w[0]), half(a->w[1]), half(a->w[2]), a->L, zc, a->status);
+            P2(a->bnd), half(a->w[0]), half(a->w[1]), half(a->w[2]), a->L, zc, a->status));
     else
-        k_adjoint_x2_tma<double><<<grid, dim3(RTX, RTY), RSMEM_F64, a->stream>>>(
+        ATRY(a, launch_step(k_adjoint_x2_tma<double>, grid, dim3(RTX, RTY), RSMEM_F64, a->stream,
             ml, mu, a->cmaps[0], a->cmaps[1], a->cmaps[2], a->cmaps[3], a->lam[R.cur ^ 1], P2(a->gx), a->bnd,
-            half(a->w[0]), half(a->w[1]), half(a->w[2]), a->L, zc, a->status);
+            half(a->w[0]), half(a->w[1]), half(a->w[2]), a->L, zc, a->status));
     ATRY(a, cudaGetLastError());
     R.cur ^= 1;
     ++a->adj_steps;

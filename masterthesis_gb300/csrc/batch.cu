@@ -92,6 +92,8 @@ __global__ void __launch_bounds__(MARCH_THREADS, MINB)
 batch_march(const BatchInst* __restrict__ inst, const NodeOrder* __restrict__ order,
             const MarchItem* __restrict__ items, typename P::T* __restrict__ pool, int cur,
             const int* __restrict__ status) {
+    step_wait();
+    after_wait(pool);
     if (*(const volatile int*)status != 0) return;
     const MarchItem w = items[blockIdx.x];
     const BatchInst& I = inst[w.inst];
@@ -110,6 +112,7 @@ batch_march(const BatchInst* __restrict__ inst, const NodeOrder* __restrict__ or
     const Star7Coeffs c = I.c;
     march_rows_of<P, SRC_A, false, R>(L, c, pool + I.off_u[cur], pool + I.off_u[cur ^ 1], pool + I.off_f, nullptr,
                                       nullptr, nullptr, Split{0.0, 0.f, 0.f}, x, y, w.z0, w.z1);
+    step_next();
 }
 
 // The persistent loop: pull work items until the step's queue is empty.
@@ -310,20 +313,20 @@ int grid_size(scafes_batch* b, const KernelInfo& k) {
 }
 
 template <class P>
-void launch_march(scafes_batch* b, int cur) {
-    batch_march<P, march_rows<P>(), march_ctas<P, SRC_A, false>()><<<(unsigned)b->hmarch.size(), MARCH_THREADS, 0, b->stream>>>(
-        b->dinst, b->dorder, b->dmarch, (typename P::T*)b->pool, cur, b->status);
+cudaError_t launch_march(scafes_batch* b, int cur) {
+    return launch_step(batch_march<P, march_rows<P>(), march_ctas<P, SRC_A, false>()>, dim3((unsigned)b->hmarch.size()),
+                       dim3(MARCH_THREADS), 0, b->stream, b->dinst, b->dorder, b->dmarch, (typename P::T*)b->pool, cur,
+                       b->status);
 }
 
 // Enqueues one step of the whole ensemble (one launch).
 int enqueue_step(scafes_batch* b, int cur, int* counter) {
     if (b->tile == STAR7_MARCH) {
         switch (b->precision) {
-            case SCAFES_PREC_F32: launch_march<PolF32>(b, cur); break;
-            case SCAFES_PREC_F32X2: launch_march<PolF32x2>(b, cur); break;
-            default: launch_march<PolF64>(b, cur); break;
+            case SCAFES_PREC_F32: BTRY(b, launch_march<PolF32>(b, cur)); break;
+            case SCAFES_PREC_F32X2: BTRY(b, launch_march<PolF32x2>(b, cur)); break;
+            default: BTRY(b, launch_march<PolF64>(b, cur)); break;
         }
-        BTRY(b, cudaGetLastError());
         return SCAFES_OK;
     }
     const KernelInfo k = kinfo(b->precision, b->tile);

@@ -24,6 +24,7 @@
 
 #include "node_order.cuh"
 #include "scafes_common.cuh"
+#include "step_launch.cuh"
 #include "../../include/scafes_gb300.h"
 
 using namespace scafes;
@@ -91,12 +92,14 @@ struct LinArgs {
 
 __global__ void __launch_bounds__(MARCH_THREADS) k_linear(const __grid_constant__ LinArgs A) {
     const Layout& L = A.L;
+    step_wait();
     int x, y, z;
     if (blockIdx.x < A.inner_ctas) {
         const uint32_t m = blockIdx.x * MARCH_THREADS + threadIdx.x;
         if (m >= A.o.n_inner) return;
         inner_node(A.o, m, x, y, z);
-        const long long o = L.idx(x, y, z);
+        long long o = L.idx(x, y, z);
+        after_wait(o);
         for (int f = 0; f < A.n_written; ++f) {
             const LinArgs::Written& w = A.written[f];
             int k = w.first;
@@ -106,6 +109,7 @@ __global__ void __launch_bounds__(MARCH_THREADS) k_linear(const __grid_constant_
             for (; k < w.end; ++k) v = fma(A.term[k].w, __ldg(A.term[k].p + o), v);
             w.out[o] = v;
         }
+        step_next();
         return;
     }
     const uint32_t m = (blockIdx.x - A.inner_ctas) * MARCH_THREADS + threadIdx.x;
@@ -392,7 +396,7 @@ extern "C" int scafes_lin_step(scafes_lin* h, int n_steps) {
                     A.written[A.n_written++] = {P.out[f], cst, first, n,
                                                 !tl.empty() && cst == 0.0 && tl[0].w == 1.0};
                 }
-                k_linear<<<inner_ctas + border_ctas, MARCH_THREADS, 0, h->stream>>>(A);
+                LTRY(h, launch_step(k_linear, dim3(inner_ctas + border_ctas), dim3(MARCH_THREADS), 0, h->stream, A));
             } else {
                 k_linear_big<<<grid, block, 0, h->stream>>>(P, rules, h->terms, h->n_fields, L);
             }

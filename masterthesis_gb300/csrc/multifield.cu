@@ -30,6 +30,7 @@
 #include "node_order.cuh"
 #include "scafes_common.cuh"
 #include "star7.cuh"
+#include "step_launch.cuh"
 #include "tma.cuh"
 #include "../../include/scafes_gb300.h"
 
@@ -172,6 +173,7 @@ constexpr int LSX = MARCH_THREADS + 2 * 16, LSY = MARCH_THREADS + 2 * 64;  // S 
 __global__ void __launch_bounds__(MARCH_THREADS, 3) k_lame_march(const __grid_constant__ LameMarch A) {
     __shared__ double sx[2][LSX], sy[2][LSY];
     const Layout& L = A.L;
+    step_wait();
     if (blockIdx.x < A.border_ctas) {
         const uint32_t m = blockIdx.x * MARCH_THREADS + threadIdx.x;
         if (m >= A.o.n_border) return;
@@ -264,6 +266,7 @@ __global__ void __launch_bounds__(MARCH_THREADS, 3) k_lame_march(const __grid_co
         szb = szc;
         szc = sza;
     }
+    step_next();
 }
 
 // Yee steps in FP64 (see orc_yee for the staggering): one node per thread
@@ -298,10 +301,12 @@ __global__ void __launch_bounds__(MARCH_THREADS, 6)
 k_yee_h(const double* __restrict__ ex, const double* __restrict__ ey, const double* __restrict__ ez,
         double* __restrict__ hx, double* __restrict__ hy, double* __restrict__ hz,
         const __grid_constant__ YeeFlat A) {
+    step_wait();
     int x, y, z;
     if (!yee_node(A, x, y, z)) return;
     const Layout& L = A.L;
-    const long long m = L.idx(x, y, z);
+    long long m = L.idx(x, y, z);
+    after_wait(m);
     const bool xi = x + 1 < L.nx, yi = y + 1 < L.ny, zi = z + 1 < L.nz;
     // A neighbour beyond the grid reads the node itself; nothing is stored there.
     const long long mx = m + (xi ? 1 : 0), my = m + (yi ? L.pitch : 0), mz = m + (zi ? L.plane : 0);
@@ -315,6 +320,7 @@ k_yee_h(const double* __restrict__ ex, const double* __restrict__ ey, const doub
     if (yi && zi) hx[m] = fma(c, fsub(d[0], d[1], mone), hx[m]);
     if (xi && zi) hy[m] = fma(c, fsub(d[2], d[4], mone), hy[m]);
     if (xi && yi) hz[m] = fma(c, fsub(d[5], d[3], mone), hz[m]);
+    step_next();
 }
 
 // Out of line: inline, the compiler would predicate the one node's
@@ -326,10 +332,12 @@ __global__ void __launch_bounds__(MARCH_THREADS, 6)
 k_yee_e(double* __restrict__ ex, double* __restrict__ ey, double* __restrict__ ez, const double* __restrict__ hx,
         const double* __restrict__ hy, const double* __restrict__ hz, const __grid_constant__ YeeFlat A,
         long long src, double src_val) {
+    step_wait();
     int x, y, z;
     if (!yee_node(A, x, y, z)) return;
     const Layout& L = A.L;
-    const long long m = L.idx(x, y, z);
+    long long m = L.idx(x, y, z);
+    after_wait(m);
     const bool xin = x > 0 && x + 1 < L.nx, yin = y > 0 && y + 1 < L.ny, zin = z > 0 && z + 1 < L.nz;
     const long long mx = m - (x > 0 ? 1 : 0), my = m - (y > 0 ? L.pitch : 0), mz = m - (z > 0 ? L.plane : 0);
     const double c = A.ch, mone = -A.one;
@@ -345,6 +353,7 @@ k_yee_e(double* __restrict__ ex, double* __restrict__ ey, double* __restrict__ e
         if (m == src) v = yee_source(v, src_val);
         ez[m] = v;
     }
+    step_next();
 }
 
 // ---- compensated FP32 pairs (SCAFES_PREC_F32X2) -----------------------------
@@ -514,6 +523,7 @@ k_lame_x2_tma(const __grid_constant__ CUtensorMap t0, const __grid_constant__ CU
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * LX + tx;
     const int x0 = blockIdx.x * LX, y0 = blockIdx.y * LY;
     const int z0 = blockIdx.z * zchunk, z1 = min(z0 + zchunk, L.nz);
+    step_wait();
     if (__syncthreads_or(tid == 0 && *(volatile int*)status != 0)) return;
     if (tid == 0) {
         for (int b = 0; b < LNS; ++b) mbar_init(&bar[b], 1);
@@ -628,6 +638,7 @@ k_lame_x2_tma(const __grid_constant__ CUtensorMap t0, const __grid_constant__ CU
             if (live1) up[o + L.pitch + c * comp] = (colb1 || zb) ? zero : out1[c];
         }
     }
+    step_next();
     if (!__syncthreads_and(ok)) fail(issued);
 }
 
@@ -723,6 +734,7 @@ k_yee_tma(const __grid_constant__ CUtensorMap tex, const __grid_constant__ CUten
     const int zs = z0 > 0 ? z0 - 1 : 0;  // plane z0-1 only gives the new H below z0
     const int np = z1 - zs;              // planes whose new H is computed
 
+    step_wait();
     // A sweep after one that timed out has nothing valid to work on.
     if (__syncthreads_or(tid == 0 && *(volatile int*)status != 0)) return;
     if (tid == 0) {
@@ -857,6 +869,7 @@ k_yee_tma(const __grid_constant__ CUtensorMap tex, const __grid_constant__ CUten
         s1 = s2;
         s2 = t;
     }
+    step_next();
 }
 
 template <class T>
@@ -1189,12 +1202,13 @@ extern "C" int scafes_mf_step(scafes_mf* h, int n_steps) {
             void* up = field_ptr(h, 3 * (h->cur ^ 1));
             if (x2) {
                 const CUtensorMap* t = h->ltm[h->cur];
-                k_lame_x2_tma<<<lgrid, dim3(LX, LY / 2), LAME_SMEM, h->stream>>>(t[0], t[1], t[2], (float2*)up, K2,
-                                                                                L, comp, lzc, h->status);
+                MTRY(h, launch_step(k_lame_x2_tma, lgrid, dim3(LX, LY / 2), LAME_SMEM, h->stream, t[0], t[1], t[2],
+                                    (float2*)up, K2, L, comp, lzc, h->status));
             } else {
                 F.u = (const double*)u;
                 F.up = (double*)up;
-                if (lame_ctas) k_lame_march<<<lame_ctas, MARCH_THREADS, 0, h->stream>>>(F);
+                if (lame_ctas)
+                    MTRY(h, launch_step(k_lame_march, dim3(lame_ctas), dim3(MARCH_THREADS), 0, h->stream, F));
                 else k_lame<<<mgrid(L), dim3(MX, MY), 0, h->stream>>>((const double*)u, (double*)up, K, L, comp);
             }
             MTRY(h, cudaGetLastError());
@@ -1227,9 +1241,9 @@ extern "C" int scafes_mf_step(scafes_mf* h, int n_steps) {
                 const int zc = yee_zchunk(L);
                 const dim3 grid((L.nx + YX - 1) / YX, (L.ny + YY - 1) / YY, (L.nz + zc - 1) / zc);
                 const f2 sp = split_double(sv);
-                k_yee_tma<YeeF32x2><<<grid, dim3(YX, YY), yee_smem(8), h->stream>>>(
+                MTRY(h, launch_step(k_yee_tma<YeeF32x2>, grid, dim3(YX, YY), yee_smem(8), h->stream,
                     t[0], t[1], t[2], t[3], t[4], t[5], g[0], g[1], g[2], g[3], g[4], g[5], L, split3(ch), src,
-                    make_float2(sp.hi, sp.lo), zc, h->status);
+                    make_float2(sp.hi, sp.lo), zc, h->status));
                 h->cur ^= 1;
             } else if (h->esz == 8) {
                 double* f[6];
@@ -1239,10 +1253,11 @@ extern "C" int scafes_mf_step(scafes_mf* h, int n_steps) {
                         Y.nodes = (uint32_t)((long long)L.nx * L.ny * std::min(slab, L.nz - Y.z0));
                         const unsigned ctas = (Y.nodes + MARCH_THREADS - 1) / MARCH_THREADS;
                         if (half == 0)
-                            k_yee_h<<<ctas, MARCH_THREADS, 0, h->stream>>>(f[0], f[1], f[2], f[3], f[4], f[5], Y);
+                            MTRY(h, launch_step(k_yee_h, dim3(ctas), dim3(MARCH_THREADS), 0, h->stream, f[0], f[1],
+                                                f[2], f[3], f[4], f[5], Y));
                         else
-                            k_yee_e<<<ctas, MARCH_THREADS, 0, h->stream>>>(f[0], f[1], f[2], f[3], f[4], f[5], Y, src,
-                                                                           sv);
+                            MTRY(h, launch_step(k_yee_e, dim3(ctas), dim3(MARCH_THREADS), 0, h->stream, f[0], f[1],
+                                                f[2], f[3], f[4], f[5], Y, src, sv));
                     }
             } else {
                 const int rc = yee_maps(h);
@@ -1252,9 +1267,9 @@ extern "C" int scafes_mf_step(scafes_mf* h, int n_steps) {
                 const CUtensorMap* t = h->ytm[h->cur];
                 const int zc = yee_zchunk(L);
                 const dim3 grid((L.nx + YX - 1) / YX, (L.ny + YY - 1) / YY, (L.nz + zc - 1) / zc);
-                k_yee_tma<YeeF32><<<grid, dim3(YX, YY), yee_smem(4), h->stream>>>(
+                MTRY(h, launch_step(k_yee_tma<YeeF32>, grid, dim3(YX, YY), yee_smem(4), h->stream,
                     t[0], t[1], t[2], t[3], t[4], t[5], g[0], g[1], g[2], g[3], g[4], g[5], L, (float)ch, src,
-                    (float)sv, zc, h->status);
+                    (float)sv, zc, h->status));
                 h->cur ^= 1;
             }
             MTRY(h, cudaGetLastError());

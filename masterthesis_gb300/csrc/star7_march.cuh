@@ -23,6 +23,7 @@
 
 #include "node_order.cuh"
 #include "star7_border.cuh"
+#include "step_launch.cuh"
 
 namespace scafes {
 
@@ -64,6 +65,7 @@ __device__ __forceinline__ void march_rows_of(const Layout& L, const Star7Coeffs
     constexpr bool has_fb = SRC == SRC_AB;
     const long long py = L.pitch, pz = L.plane;
     long long o = L.idx(x, y, z0);
+    after_wait(o);
     // Rows that are border rows are computed but not stored; a row beyond the
     // grid reads the last one.
     unsigned skip = 0u;
@@ -119,6 +121,7 @@ __global__ void __launch_bounds__(MARCH_THREADS, MINB)
 star7_march(const __grid_constant__ MarchArgs<typename P::T> A) {
     using T = typename P::T;
     const Layout& L = A.L;
+    step_wait();
     if (*(const volatile int*)A.status != 0) return;  // an earlier sweep gave up
     if (blockIdx.x < A.border_ctas) {
         const uint32_t m = blockIdx.x * (MARCH_THREADS) + threadIdx.x;
@@ -128,7 +131,9 @@ star7_march(const __grid_constant__ MarchArgs<typename P::T> A) {
         J.nodes = A.nodes;
         int x, y, z;
         border_node(A.o, m, x, y, z);
-        A.un[L.idx(x, y, z)] = border_value<P, SRC, BORDER>(J, A.uo, x, y, z);
+        const T* uo = A.uo;
+        after_wait(uo);
+        A.un[L.idx(x, y, z)] = border_value<P, SRC, BORDER>(J, uo, x, y, z);
         return;
     }
     const uint32_t q = blockIdx.x - A.border_ctas;
@@ -139,6 +144,7 @@ star7_march(const __grid_constant__ MarchArgs<typename P::T> A) {
     if ((int)row >= A.ct.h || x >= L.nx - L.nl || y >= L.ny - L.nl) return;
     const int z0 = (int)k * A.zchunk + L.nl, z1 = min(z0 + A.zchunk, L.nz - L.nl);
     march_rows_of<P, SRC, VC, R>(L, A.c, A.uo, A.un, A.fa, A.fb, A.c0, A.ca, A.t.t_old, x, y, z0, z1);
+    step_next();
 }
 
 // ---- host side ---------------------------------------------------------------
@@ -206,8 +212,8 @@ static cudaError_t launch_march_typed(const Star7Launch& a, cudaStream_t stream)
     A.txy = make_fastdiv((uint32_t)std::max(1LL, tx * ty));
     const long long ctas = A.border_ctas + (A.o.n_inner ? tx * ty * tz : 0);
     if (ctas > 0x7fffffffLL) return cudaErrorInvalidValue;
-    star7_march<P, SRC, BORDER, VC, R, march_ctas<P, SRC, VC>()><<<(unsigned)ctas, MARCH_THREADS, 0, stream>>>(A);
-    return cudaGetLastError();
+    return launch_step(star7_march<P, SRC, BORDER, VC, R, march_ctas<P, SRC, VC>()>, dim3((unsigned)ctas),
+                       dim3(MARCH_THREADS), 0, stream, A);
 }
 
 template <class P, int BORDER>

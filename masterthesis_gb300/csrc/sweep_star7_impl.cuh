@@ -5,6 +5,7 @@
 
 #include "star7_tb.cuh"
 #include "star7_tile.cuh"
+#include "step_launch.cuh"
 
 namespace scafes {
 
@@ -37,6 +38,11 @@ star7_tma(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtens
     extern __shared__ __align__(128) unsigned char smem_raw[];
     T* st = reinterpret_cast<T*>(smem_raw);
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + (size_t)NS * G::STRIDE * G::ESZ);
+    step_wait();
+    after_wait(fa);
+    after_wait(fb);
+    after_wait(ga);
+    after_wait(gb);
     // After a sweep gave up on a TMA load (status set), the results are
     // invalid until the host reads the status: later sweeps return at once
     // instead of each waiting out its own limit.
@@ -47,6 +53,7 @@ star7_tma(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtens
     const int z1 = min(z0 + zchunk, L.nz);
     uint32_t base = 0;
     star7_tile<P, SRC, BORDER, BY, R, NS, FS, ML>(J, c, blockIdx.x * BX, blockIdx.y * BY, z0, z1, st, bar, base, status);
+    step_next();
 }
 
 // Per-node border rules (FP64 and FP32 sweeps) leave the x-face nodes
@@ -66,6 +73,8 @@ constexpr bool XFACE_PASS =
 template <typename T>
 static __global__ void k_xface_node_rules(const T* __restrict__ uo, T* __restrict__ un,
                                           const scafes_border_node_rule* __restrict__ nodes, Layout L) {
+    step_wait();
+    after_wait(uo);
     const long long rows = (long long)(L.ny - 2) * (L.nz - 2);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < 2 * rows;
          i += (long long)gridDim.x * blockDim.x) {
@@ -97,6 +106,7 @@ static __global__ void k_xface_node_rules(const T* __restrict__ uo, T* __restric
             un[o] = v;
         }
     }
+    step_next();
 }
 
 // The variable-coefficient sweep: as star7_tma, with the coefficient fields
@@ -125,6 +135,9 @@ star7_vc_tma(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUt
     extern __shared__ __align__(128) unsigned char smem_raw[];
     T* st = reinterpret_cast<T*>(smem_raw);
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + (size_t)NS * G::STRIDE * G::ESZ);
+    step_wait();
+    after_wait(fa);
+    after_wait(ga);
     if (__syncthreads_or(threadIdx.x == 0 && threadIdx.y == 0 && *(volatile int*)status != 0)) return;
     ring_init<NS>(bar);
     TileJob<T> J{&tm, &tmf, un, fa, nullptr, ga, nullptr, gval, L, time_old, time_new, Split{0.0, 0.f, 0.f}, table,
@@ -134,6 +147,7 @@ star7_vc_tma(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUt
     uint32_t base = 0;
     star7_tile<P, SRC, BORDER, BY, R, NS, FS, false, true>(J, c, blockIdx.x * BX, blockIdx.y * BY, z0, z1, st,
                                                            bar, base, status);
+    step_next();
 }
 
 // ---- host side ---------------------------------------------------------------
@@ -193,11 +207,10 @@ static cudaError_t launch_typed(const Star7Launch& a, cudaStream_t stream) {
     const int zchunk = choose_zchunk(L, BY, std::is_same<P, PolF32>::value && BY == 16 && R == 4 ? 8 : 16);
     dim3 block(BX, BY / R, 1);
     dim3 grid((L.nx + BX - 1) / BX, (L.ny + BY - 1) / BY, (L.nz + zchunk - 1) / zchunk);
-    kern<<<grid, block, G::SMEM, stream>>>(*a.tm_uo, FS ? *a.tm_f : *a.tm_uo, (T*)a.un, (const T*)a.fa, (const T*)a.fb, (const T*)a.ga,
-                                           (const T*)a.gb, gval, L,
-                                           a.c, make_split(a.time_old), make_split(a.time_new),
-                                           make_split(a.mirror_corr), a.table, zchunk, a.status);
-    return cudaGetLastError();
+    return launch_step(kern, grid, block, G::SMEM, stream, *a.tm_uo, FS ? *a.tm_f : *a.tm_uo, (T*)a.un,
+                       (const T*)a.fa, (const T*)a.fb, (const T*)a.ga, (const T*)a.gb, gval, L, a.c,
+                       make_split(a.time_old), make_split(a.time_new), make_split(a.mirror_corr), a.table, zchunk,
+                       a.status);
 }
 
 template <class P, int SRC, int BORDER>
@@ -244,17 +257,17 @@ static cudaError_t launch_vc_typed(const Star7Launch& a, cudaStream_t stream) {
     const int zchunk = choose_zchunk(L, BY);
     dim3 block(BX, BY / R, 1);
     dim3 grid((L.nx + BX - 1) / BX, (L.ny + BY - 1) / BY, (L.nz + zchunk - 1) / zchunk);
-    kern<<<grid, block, G::SMEM, stream>>>(*a.tm_uo, FS ? *a.tm_f : *a.tm_uo, *a.tm_c0, *a.tm_ca, (T*)a.un,
-                                           (const T*)a.fa, (const T*)a.ga, gval, L, a.c, make_split(a.time_old),
-                                           make_split(a.time_new), a.table, a.nodes, zchunk, a.status);
+    cudaError_t e = launch_step(kern, grid, block, G::SMEM, stream, *a.tm_uo, FS ? *a.tm_f : *a.tm_uo, *a.tm_c0,
+                                *a.tm_ca, (T*)a.un, (const T*)a.fa, (const T*)a.ga, gval, L, a.c,
+                                make_split(a.time_old), make_split(a.time_new), a.table, a.nodes, zchunk, a.status);
     if constexpr (XFACE_PASS<P, BORDER>) {
-        const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         const long long work = 2LL * (L.ny - 2) * (L.nz - 2);
         const int blocks = (int)std::min<long long>((work + 255) / 256, (long long)num_sms() * 8);
-        k_xface_node_rules<T><<<blocks, 256, 0, stream>>>((const T*)a.uo, (T*)a.un, a.nodes, L);
+        e = launch_step(k_xface_node_rules<T>, dim3(blocks), dim3(256), 0, stream, (const T*)a.uo, (T*)a.un, a.nodes,
+                        L);
     }
-    return cudaGetLastError();
+    return e;
 }
 
 template <class P, int SRC, int BORDER>
