@@ -1,16 +1,17 @@
-// The new value of one border node, from the old iterate in global memory:
-// for the kernels that deal with the border nodes apart from the inner ones
-// (star7_loop.cuh, star7_march.cuh), in full warps.  Same operations in the
-// same order as the tile engine's border paths.
+// The new value of one border node, for the kernels that deal with the border
+// nodes apart from the inner ones (star7_loop.cuh, star7_march.cuh), in full
+// warps.  Same operations in the same order as the tile engine's border paths.
 #pragma once
 
 #include "star7_tile.cuh"
 
 namespace scafes {
 
-template <class P, int SRC, int BORDER>
-__device__ __forceinline__ typename P::T border_value(const TileJob<typename P::T>& J, const typename P::T* uo, int x,
-                                                      int y, int z) {
+// `at(dx, dy, dz)` gives the old iterate at the node (0, 0, 0) and at its
+// neighbours; it is called for nodes of the grid only.
+template <class P, int SRC, int BORDER, class At>
+__device__ __forceinline__ typename P::T border_value_at(const TileJob<typename P::T>& J, int x, int y, int z,
+                                                         const At& at) {
     using T = typename P::T;
     const Layout& L = J.L;
     const long long o = L.idx(x, y, z);
@@ -19,10 +20,10 @@ __device__ __forceinline__ typename P::T border_value(const TileJob<typename P::
         return J.gb ? P::src(v, J.gb[o], J.time_new, true) : v;
     } else {
         // A neighbour outside the grid reads 0, as from the TMA halo.
-        const T u = uo[o];
-        const T w = x > 0 ? uo[o - 1] : P::zero(), e = x < L.nx - 1 ? uo[o + 1] : P::zero();
-        const T s = y > 0 ? uo[o - L.pitch] : P::zero(), n = y < L.ny - 1 ? uo[o + L.pitch] : P::zero();
-        const T b = z > 0 ? uo[o - L.plane] : P::zero(), t = z < L.nz - 1 ? uo[o + L.plane] : P::zero();
+        const T u = at(0, 0, 0);
+        const T w = x > 0 ? at(-1, 0, 0) : P::zero(), e = x < L.nx - 1 ? at(1, 0, 0) : P::zero();
+        const T s = y > 0 ? at(0, -1, 0) : P::zero(), n = y < L.ny - 1 ? at(0, 1, 0) : P::zero();
+        const T b = z > 0 ? at(0, 0, -1) : P::zero(), t = z < L.nz - 1 ? at(0, 0, 1) : P::zero();
         if constexpr (BORDER == SCAFES_BORDER_NODES) {
             return node_rule<P>(J, x, y, z, u, w, e, s, n, b, t);
         } else if constexpr (BORDER == SCAFES_BORDER_TABLE) {
@@ -43,6 +44,17 @@ __device__ __forceinline__ typename P::T border_value(const TileJob<typename P::
             return P::mirror(u, opp, minus ? negated(J.corr) : J.corr);
         }
     }
+}
+
+// The same from the old iterate in global memory.
+template <class P, int SRC, int BORDER>
+__device__ __forceinline__ typename P::T border_value(const TileJob<typename P::T>& J, const typename P::T* uo, int x,
+                                                      int y, int z) {
+    const Layout& L = J.L;
+    const long long o = L.idx(x, y, z);
+    return border_value_at<P, SRC, BORDER>(J, x, y, z, [&](int dx, int dy, int dz) {
+        return uo[o + dx + dy * (long long)L.pitch + dz * L.plane];
+    });
 }
 
 }  // namespace scafes

@@ -24,32 +24,9 @@
 
 #include <algorithm>
 
-#include "node_order.cuh"
-#include "star7_border.cuh"
+#include "star7_cluster.cuh"
 
 namespace scafes {
-
-template <class T>
-struct LoopArgs {
-    T* u[2];                 // iterates; u[first] is the old one of the first step
-    int first, n_steps;
-    const T* fa;
-    const T* fb;
-    const T* ga;
-    const T* gb;
-    T gval;
-    const T* c0;             // variable coefficients
-    const T* ca;
-    Layout L;
-    NodeOrder o;
-    Star7Coeffs c;
-    const BorderTable* table;
-    const scafes_border_node_rule* nodes;
-    const StepTimes* times;  // n_steps entries, or null when nothing reads the time
-    uint32_t in_cta, bd_cta; // inner and border nodes per CTA
-    unsigned* arrivals;      // barrier counter, 0 at launch
-    int* status;
-};
 
 // Ends a step for the whole grid: returns false (status set) when the other
 // CTAs did not arrive in time.  The release of thread 0 after the block
@@ -166,6 +143,11 @@ static cudaError_t launch_loop_typed(const Star7Loop& q, cudaStream_t stream) {
     A.times = q.times;
     A.arrivals = q.arrivals;
     A.status = a.status;
+    {
+        bool done = false;
+        const cudaError_t ce = launch_cluster<P, SRC, BORDER, VC>(A, stream, &done);
+        if (ce != cudaSuccess || done) return ce;
+    }
     // Two warps per CTA at least: fewer CTAs make the barrier cheaper, more
     // spread the FP64 pipe's work; all SMs from 2 * 32 * SMs nodes on.
     const uint32_t wi = (A.o.n_inner + 31) / 32, wb = (A.o.n_border + 31) / 32;

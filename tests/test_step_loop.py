@@ -1,7 +1,7 @@
 """The one-launch time loop of small grids (star7_loop.cuh).
 
 CPU: the numbering of inner and border nodes against plain loops.  GPU: the
-loop, the sweep by plain loads (star7_march.cuh) and the tile sweeps give the
+loop (inside one cluster on the smallest grids), the sweep by plain loads (star7_march.cuh) and the tile sweeps give the
 same bits (an explicitly set depth or tile keeps one launch per step) for every border kind, source, element type and layer count it
 accepts, on grids with no inner node, one node, and remainders of warps and
 CTAs, over more steps than one launch takes.
@@ -73,7 +73,7 @@ CASES = [(prec, border, source, layers)
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("prec,border,source,layers", CASES)
-@pytest.mark.parametrize("n,steps", [((4, 4, 4), 3), ((5, 7, 4), 1030), ((33, 18, 11), 5), ((70, 66, 68), 4)])
+@pytest.mark.parametrize("n,steps", [((4, 4, 4), 3), ((5, 7, 4), 1030), ((9, 8, 21), 6), ((33, 18, 11), 5), ((70, 66, 68), 4)])
 def test_loop_and_sweeps_give_the_same_bits(gpu, prec, border, source, layers, n, steps):
     M = gpu
     got = []
