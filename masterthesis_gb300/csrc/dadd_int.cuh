@@ -108,4 +108,56 @@ SCAFES_HD uint64_t dadd_bits(uint64_t a, uint64_t b, bool& ok) {
     return mag ? ((uint64_t)hi << 32) | (uint32_t)r : 0u;
 }
 
+// A constant factor prepared for dmul_bits: its significand's 53 bits at the
+// top of 64, what its exponent and sign add to the high word of the other
+// factor, and the exponent fields (in place) for which the product and both
+// factors are normal numbers: [lo, lo + range].
+struct IntFactor {
+    uint32_t ch, cl, k, lo, range;
+};
+
+inline IntFactor make_int_factor(double c) {
+    uint64_t b;
+    __builtin_memcpy(&b, &c, 8);
+    const int ec = (int)(b >> 52 & 0x7ff);
+    const uint64_t m = ((b & 0xfffffffffffffull) | (1ull << 52)) << 11;
+    IntFactor f;
+    f.ch = (uint32_t)(m >> 32);
+    f.cl = (uint32_t)m;
+    f.k = ((uint32_t)(ec - 1023) << 20) + (uint32_t)(b >> 63 << 31);
+    const int lo = 1025 - ec > 1 ? 1025 - ec : 1, hi = 3067 - ec < 2046 ? 3067 - ec : 2046;
+    const bool normal = ec >= 1 && ec <= 2046 && lo <= hi;
+    f.lo = normal ? (uint32_t)lo << 20 : 0xfff00000u;  // never matched
+    f.range = normal ? (uint32_t)(hi - lo) << 20 : 0u;
+    return f;
+}
+
+// c * u, rounded to nearest even as by the FP64 multiplier, where `ok` (u,
+// c and the product normal numbers).  The 53 x 53 bit product is formed
+// exactly in four 32 x 32 multiplications (the FMA pipe); its top 53 bits are
+// rounded with the rest.
+SCAFES_HD uint64_t dmul_bits(const IntFactor& c, uint64_t u, bool& ok) {
+    const uint32_t uh = (uint32_t)(u >> 32), ul = (uint32_t)u;
+    const uint32_t mh = (uh & 0x000fffffu) | 0x00100000u;
+    const uint64_t p0 = (uint64_t)ul * c.cl;
+    const uint64_t p1 = (uint64_t)ul * c.ch + (p0 >> 32);
+    const uint64_t p2 = (uint64_t)mh * c.cl + (uint32_t)p1;
+    const uint64_t p3 = (uint64_t)mh * c.ch + (p1 >> 32) + (p2 >> 32);  // the top 52 or 53 bits
+    const uint32_t r1 = (uint32_t)p2, r0 = (uint32_t)p0;                // the rest
+    const uint32_t th = (uint32_t)(p3 >> 32), tl = (uint32_t)p3;
+    const uint32_t s = 1u - (th >> 20);  // one bit short: shift in the next
+#if defined(__CUDA_ARCH__)
+    const uint32_t nh = __funnelshift_l(tl, th, s), nl = __funnelshift_l(r1, tl, s), nr = __funnelshift_l(r0, r1, s);
+#else
+    const uint32_t nh = s ? th << 1 | tl >> 31 : th, nl = s ? tl << 1 | r1 >> 31 : tl, nr = s ? r1 << 1 | r0 >> 31 : r1;
+#endif
+    // Round half to even; a bit of r0 breaks a tie (where its top bit moved
+    // into nr, nr is no tie).
+    const uint32_t rest = nr | (r0 != 0u ? 1u : 0u);
+    const uint32_t up = rest > 0x80000000u - (nl & 1u) ? 1u : 0u;
+    const uint64_t m = (((uint64_t)nh << 32) | nl) + up;
+    ok = (uh & 0x7ff00000u) - c.lo <= c.range;
+    return m + ((uint64_t)((uh & 0xfff00000u) + c.k - (s << 20)) << 32);
+}
+
 }  // namespace scafes

@@ -4,6 +4,7 @@
 
 #include <cuda.h>
 
+#include "dadd_int.cuh"
 #include "scafes_common.cuh"
 #include "../../include/scafes_gb300.h"
 
@@ -27,6 +28,7 @@ constexpr int BX = 32;
 
 struct Star7Coeffs {
     double c0, cx, cy, cz, cf;
+    IntFactor m0, mx;  // c0 and cx for products on the integer pipe
     float c0h, c0l, c0ll, cxh, cxl, cxll, cyh, cyl, cyll, czh, czl, czll, cfh, cfl, cfll;
 };
 

@@ -76,35 +76,47 @@ __device__ __forceinline__ void march_rows_of(const Layout& L, const Star7Coeffs
         if (y + i >= L.ny - L.nl) skip |= 1u << i;
     }
     const long long rn = (min(y + R, L.ny - 1) - y) * py;
-    T below[R], cur[R];
+    // With a source or node coefficients, what streams from memory (they and
+    // the plane above) is loaded a plane before it is used: FP64 ensemble 311
+    // -> 303 us, 256^3 with a source 160 -> 156; without, it costs 141 -> 145.
+    constexpr bool AHEAD = R == 1 && (HAS_F || VC);
+    T below[R], cur[R], above[R], f[R], c0[R], ca[R];
+    auto fetch = [&](long long m, T (&fo)[R], T (&c0o)[R], T (&cao)[R]) {
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            fo[i] = P::zero();
+            if (HAS_F) fo[i] = P::src(fa[m + ro[i]], has_fb ? fb[m + ro[i]] : P::zero(), t_old, has_fb);
+            if constexpr (VC) {
+                c0o[i] = c0f[m + ro[i]];
+                cao[i] = caf[m + ro[i]];
+            }
+        }
+    };
 #pragma unroll
     for (int i = 0; i < R; ++i) {
         below[i] = uo[o + ro[i] - pz];
         cur[i] = uo[o + ro[i]];
+        if (AHEAD) above[i] = uo[o + ro[i] + pz];
     }
+    if (AHEAD) fetch(o, f, c0, ca);
 #pragma unroll 2
     for (int z = z0; z < z1; ++z, o += pz) {
-        T above[R], w[R], e[R], f[R], v[R];
+        T w[R], e[R], v[R], next[R], fn[R], c0n[R], can[R];
+        const long long on = z + 1 < z1 ? o + pz : o;  // the last plane loads its own again
         const T ym = uo[o - py], yp = uo[o + rn];
 #pragma unroll
         for (int i = 0; i < R; ++i) {
-            above[i] = uo[o + ro[i] + pz];
+            if (AHEAD) next[i] = uo[on + ro[i] + pz];
+            else above[i] = uo[o + ro[i] + pz];
             w[i] = uo[o + ro[i] - 1];
             e[i] = uo[o + ro[i] + 1];
-            f[i] = P::zero();
-            if (HAS_F) f[i] = P::src(fa[o + ro[i]], has_fb ? fb[o + ro[i]] : P::zero(), t_old, has_fb);
         }
-        if constexpr (VC) {
-            T c0[R], ca[R];
-#pragma unroll
-            for (int i = 0; i < R; ++i) {
-                c0[i] = c0f[o + ro[i]];
-                ca[i] = caf[o + ro[i]];
-            }
+        if (AHEAD) fetch(on, fn, c0n, can);
+        else fetch(o, f, c0, ca);
+        if constexpr (VC)
             P::template star_vc_rows<HAS_F, R>(c, below, cur, above, ym, yp, w, e, f, c0, ca, 1, v, skip);
-        } else {
+        else
             P::template star_rows<HAS_F, R>(c, below, cur, above, ym, yp, w, e, f, v, skip);
-        }
 #pragma unroll
         for (int i = 0; i < R; ++i)
             if (R == 1 || !((skip >> i) & 1u)) un[o + i * py] = v[i];
@@ -112,6 +124,12 @@ __device__ __forceinline__ void march_rows_of(const Layout& L, const Star7Coeffs
         for (int i = 0; i < R; ++i) {
             below[i] = cur[i];
             cur[i] = above[i];
+            if (AHEAD) {
+                above[i] = next[i];
+                f[i] = fn[i];
+                c0[i] = c0n[i];
+                ca[i] = can[i];
+            }
         }
     }
 }

@@ -71,9 +71,42 @@ struct PolF64 {
 #pragma unroll
         for (int k = 0; k < R; ++k) out[k] = r.v[k];
     }
+    // out[k] = c * a[k] on the integer pipe (dmul_bits: the FP64 multiplier's
+    // bits), with the same fallback as the sums.  Without a source it is even
+    // (256^3 142 / 141 us, both pipes 60 - 80 % busy), with one, five FP64
+    // operations to four, it pays: 256^3 175 -> 160, the ensemble 325 -> 303
+    // (both with star7_march.cuh's loads ahead), the loop at 64^3 5.06 -> 4.78.
+    template <int R>
+    static __device__ __noinline__ Nodes<R> fp64_mul(double c, Nodes<R> a) {
+        Nodes<R> r;
+#pragma unroll
+        for (int k = 0; k < R; ++k) r.v[k] = c * a.v[k];
+        return r;
+    }
+    template <int R>
+    static __device__ __forceinline__ void products(const IntFactor& m, double c, const T (&a)[R], T (&out)[R],
+                                                    unsigned skip) {
+        bool ok = true;
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            bool o;
+            const uint64_t r = dmul_bits(m, (uint64_t)__double_as_longlong(a[k]), o);
+            out[k] = __longlong_as_double((long long)r);
+            ok = ok && (o || ((skip >> k) & 1u));
+        }
+        if (__any_sync(__activemask(), !ok)) {
+            Nodes<R> x;
+#pragma unroll
+            for (int k = 0; k < R; ++k) x.v[k] = a[k];
+            const Nodes<R> r = fp64_mul<R>(c, x);
+#pragma unroll
+            for (int k = 0; k < R; ++k) out[k] = r.v[k];
+        }
+    }
+    // c0u = c0 * u.
     template <bool HAS_F>
-    static __device__ __forceinline__ T star_of_sums(const Star7Coeffs& c, T u, T sx, T sy, T sz, T f) {
-        double v = c.c0 * u;
+    static __device__ __forceinline__ T star_of_sums(const Star7Coeffs& c, T c0u, T sx, T sy, T sz, T f) {
+        double v = c0u;
         v = fma(c.cx, sx, v);
         v = fma(c.cy, sy, v);
         v = fma(c.cz, sz, v);
@@ -83,10 +116,11 @@ struct PolF64 {
     template <bool HAS_F>
     static __device__ __forceinline__ T star(const Star7Coeffs& c, T u, T w, T e,
                                              T s, T n, T b, T t, T f) {
-        T sx[1], sy[1], sz[1];
-        const T w1[1] = {w}, e1[1] = {e}, s1[1] = {s}, n1[1] = {n}, b1[1] = {b}, t1[1] = {t};
+        T sx[1], sy[1], sz[1], c0u[1];
+        const T u1[1] = {u}, w1[1] = {w}, e1[1] = {e}, s1[1] = {s}, n1[1] = {n}, b1[1] = {b}, t1[1] = {t};
         sums<1>(w1, e1, s1, n1, b1, t1, sx, sy, sz, 0u);
-        return star_of_sums<HAS_F>(c, u, sx[0], sy[0], sz[0], f);
+        products<1>(c.m0, c.c0, u1, c0u, 0u);
+        return star_of_sums<HAS_F>(c, c0u[0], sx[0], sy[0], sz[0], f);
     }
     static __device__ __forceinline__ T mirror(T u, T uo, const Split& corr) {
         return (u + uo) - corr.d;
@@ -97,11 +131,12 @@ struct PolF64 {
 
     // Variable coefficients: c0x * u + cax * (cx (w+e) + cy (s+n) + cz (b+t))
     // + f, with the node's own C0 and CA and the source with weight 1
-    // (8 FP64 operations, the three sums on the integer pipe as in sums()).
+    // (8 FP64 operations, the three sums and cxsx = cx (w+e) on the integer
+    // pipe).
     template <bool HAS_F>
-    static __device__ __forceinline__ T star_vc_of_sums(const Star7Coeffs& c, T u, T sx, T sy, T sz, T f, T c0x,
+    static __device__ __forceinline__ T star_vc_of_sums(const Star7Coeffs& c, T u, T cxsx, T sy, T sz, T f, T c0x,
                                                         T cax) {
-        double l = c.cx * sx;
+        double l = cxsx;
         l = fma(c.cy, sy, l);
         l = fma(c.cz, sz, l);
         const double v = HAS_F ? fma(c0x, u, f) : c0x * u;
@@ -113,7 +148,9 @@ struct PolF64 {
         T sx[1], sy[1], sz[1];
         const T w1[1] = {w}, e1[1] = {e}, s1[1] = {s}, n1[1] = {n}, b1[1] = {b}, t1[1] = {t};
         sums<1>(w1, e1, s1, n1, b1, t1, sx, sy, sz, 0u);
-        return star_vc_of_sums<HAS_F>(c, u, sx[0], sy[0], sz[0], f, c0x, cax);
+        T cxsx[1];
+        products<1>(c.mx, c.cx, sx, cxsx, 0u);
+        return star_vc_of_sums<HAS_F>(c, u, cxsx[0], sy[0], sz[0], f, c0x, cax);
     }
     // All R rows of one thread with the coefficients c0[k * stride],
     // ca[k * stride] of row k; `skip` as for star_rows.
@@ -130,9 +167,11 @@ struct PolF64 {
             n[k] = k == R - 1 ? yp : cur[k + 1];
         }
         sums<R>(w, e, s, n, below, above, sx, sy, sz, skip);
+        T cxsx[R];
+        products<R>(c.mx, c.cx, sx, cxsx, skip);
 #pragma unroll
         for (int k = 0; k < R; ++k)
-            v[k] = star_vc_of_sums<HAS_F>(c, cur[k], sx[k], sy[k], sz[k], f[k], c0[k * stride], ca[k * stride]);
+            v[k] = star_vc_of_sums<HAS_F>(c, cur[k], cxsx[k], sy[k], sz[k], f[k], c0[k * stride], ca[k * stride]);
     }
     // All R rows of one thread (row k's s/n neighbours are rows k-1/k+1,
     // ym/yp beyond the ends).  Bit k of `skip`: row k's result is replaced
@@ -149,8 +188,10 @@ struct PolF64 {
             n[k] = k == R - 1 ? yp : cur[k + 1];
         }
         sums<R>(w, e, s, n, below, above, sx, sy, sz, skip);
+        T c0u[R];
+        products<R>(c.m0, c.c0, cur, c0u, skip);
 #pragma unroll
-        for (int k = 0; k < R; ++k) v[k] = star_of_sums<HAS_F>(c, cur[k], sx[k], sy[k], sz[k], f[k]);
+        for (int k = 0; k < R; ++k) v[k] = star_of_sums<HAS_F>(c, c0u[k], sx[k], sy[k], sz[k], f[k]);
     }
 };
 

@@ -17,6 +17,8 @@ namespace scafes {
 Star7Coeffs make_star7_coeffs(double c0, const double cp[3], double cf) {
     Star7Coeffs c;
     c.c0 = c0; c.cx = cp[0]; c.cy = cp[1]; c.cz = cp[2]; c.cf = cf;
+    c.m0 = make_int_factor(c0);
+    c.mx = make_int_factor(cp[0]);
     auto split3 = [](double v, float& h, float& l, float& ll) {
         h = (float)v;
         double r = v - (double)h;

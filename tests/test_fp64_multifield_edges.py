@@ -31,6 +31,14 @@ def test_any_sign_adder_equals_the_fp64_adder(tmp_path, seed):
     assert handed_back < pairs // 3
 
 
+@pytest.mark.parametrize("seed", [5, 13])
+def test_constant_factor_multiplier_equals_the_fp64_multiplier(tmp_path, seed):
+    exe = tmp_path / "dmul_int_check"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-o", str(exe), str(NATIVE / "dmul_int_check.cpp")], check=True)
+    res = subprocess.run([str(exe), str(seed), "4000000"], capture_output=True, text=True)
+    assert res.returncode == 0, res.stdout
+
+
 def _field(kind, shape, rng):
     if kind == "smooth":
         z, y, x = np.meshgrid(*(np.linspace(0.1, 0.9, m) for m in shape), indexing="ij")
