@@ -394,7 +394,10 @@ k_forward_x2_tma(const __grid_constant__ CUtensorMap tu, const __grid_constant__
 // node instead of 104).  A face to a node outside the grid or between two
 // border nodes contributes nothing: lambda is zero there.
 // The operands are staged through TMA on the forward step's tile (RTX x
-// RTY columns, a chunk of planes, a ring of four planes on four mbarriers).  Per
+// RTY columns, a chunk of planes, a ring of three planes on three mbarriers: z
+// and z+1 in use, z+2 in flight; a fourth would cost one of four resident CTAs
+// per SM, FP64 200 steps of 97 x 90 x 83 with 16 snapshots 10.0 against 9.2
+// ms).  Per
 // plane one mbarrier covers six boxes: lambda and u with a one-node halo
 // (x from x0-2), the x faces from x0-2, the y faces from row y0-1, the z
 // faces and the diagonal.  lambda, u and the z face of the plane below and
@@ -402,7 +405,7 @@ k_forward_x2_tma(const __grid_constant__ CUtensorMap tu, const __grid_constant__
 // read with plain loads one plane ahead and written in place.
 // Out-of-range box elements read as zero.  Every wait is bounded (status
 // word, drain, return).
-constexpr int RTX = FTX, RTY = FTY, RNS = FNS;
+constexpr int RTX = FTX, RTY = FTY, RNS = 3;
 constexpr int RLW = FUW, RLH = FUH;                       // lambda and u boxes: the forward's u box
 constexpr int RO_L = 0, RO_U = pad16(RLW * RLH), RO_X = RO_U + pad16(RLW * RLH);
 constexpr int RO_Y = RO_X + pad16(FXW * FXH), RO_Z = RO_Y + pad16(FYW * FYH), RO_D = RO_Z + pad16(FKW * FKH);
@@ -475,7 +478,7 @@ k_adjoint_x2_tma(const __grid_constant__ CUtensorMap tl, const __grid_constant__
     // Input plane j is z0-1+j (j = 0 .. n_in-1), in ring slot j % RNS.
     const int n_in = z1 - z0 + 2;
     auto issue = [&](int j) {
-        const int s = j & (RNS - 1), z = z0 - 1 + j;
+        const int s = j % RNS, z = z0 - 1 + j;
         E* d = rsm + s * RSLOT;
         scafes::mbar_arrive_expect_tx(&bar[s], RTX_BYTES);
         scafes::tma_load_3d(d + RO_L, &tl, x0 - 2, y0 - 1, z, &bar[s]);
@@ -487,13 +490,13 @@ k_adjoint_x2_tma(const __grid_constant__ CUtensorMap tl, const __grid_constant__
     };
     if (tid == 0)
         for (int j = 0; j < RNS && j < n_in; ++j) issue(j);
-    auto wait = [&](int j) { return scafes::bounded_wait(&bar[j & (RNS - 1)], (uint32_t)(j >> 2) & 1u); };
+    auto wait = [&](int j) { return scafes::bounded_wait(&bar[j % RNS], (uint32_t)(j / RNS) & 1u); };
     auto fail = [&](int last_issued) {
         if (tid == 0) {
             atomicExch(status, SCAFES_ERR_TIMEOUT);
             for (int j = last_issued - (RNS - 1); j <= last_issued; ++j)
                 if (j >= 0 && j < n_in)
-                    scafes::bounded_wait(&bar[j & (RNS - 1)], (uint32_t)(j >> 2) & 1u, scafes::kWaitLimitNs / 16);
+                    scafes::bounded_wait(&bar[j % RNS], (uint32_t)(j / RNS) & 1u, scafes::kWaitLimitNs / 16);
         }
     };
     const int x = x0 + tx, y = y0 + ty;
@@ -507,7 +510,7 @@ k_adjoint_x2_tma(const __grid_constant__ CUtensorMap tl, const __grid_constant__
     // F64: input plane j's lambda and u boxes as pairs into ring slot j & 1.
     auto to_pairs = [&](int j) {
         if constexpr (F64) {
-            const E* sj = rsm + (j & (RNS - 1)) * RSLOT;
+            const E* sj = rsm + (j % RNS) * RSLOT;
             float2* pj = pring + (j & 1) * 2 * RPAIR;
             for (int i = tid; i < RLW * RLH; i += NT) {
                 pj[i] = pview(sj[RO_L + i]);
@@ -534,17 +537,18 @@ k_adjoint_x2_tma(const __grid_constant__ CUtensorMap tl, const __grid_constant__
             fail(issued);
             return;
         }
-        if (tid == 0 && jc + 3 < n_in && jc + 3 > issued) {
+        constexpr int AHEAD = RNS - 1;
+        if (tid == 0 && jc + AHEAD < n_in && jc + AHEAD > issued) {
             scafes::fence_proxy_async_smem();
-            issue(jc + 3);
-            issued = jc + 3;
+            issue(jc + AHEAD);
+            issued = jc + AHEAD;
         }
         const float2 gc = gn;
         if (live && z + 1 < z1) gn = g[o + L.plane];
         ok = wait(jc + 1) && ok;  // plane z+1
         to_pairs(jc + 1);         // read from the next iteration on (after its barrier)
-        const E* sc = rsm + (jc & (RNS - 1)) * RSLOT;
-        const E* sa = rsm + ((jc + 1) & (RNS - 1)) * RSLOT;
+        const E* sc = rsm + (jc % RNS) * RSLOT;
+        const E* sa = rsm + ((jc + 1) % RNS) * RSLOT;
         const float2* ppl = pring + (jc & 1) * 2 * RPAIR;  // F64: plane z's pairs
         const float2* ppu = ppl + RPAIR;
         auto PL = [&](int i) -> float2 {
