@@ -267,6 +267,8 @@ static bool slot_is_double(int field) {
 // Copies the host image of the border table (rules, higher time orders of
 // G, time basis) to the device, once the rules exist there.
 static int sync_table(scafes_handle* h) {
+    BorderTable& t = h->table_host;
+    t.affine = !t.g_hi[0] && !t.g_hi[1] && !t.g_hi[2] && t.t_center == 0.0 && t.t_rate == 1.0;
     if (!h->table) return SCAFES_OK;
     CUDA_TRY(h, cudaMemcpyAsync(h->table, &h->table_host, sizeof(BorderTable), cudaMemcpyHostToDevice, h->stream));
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));

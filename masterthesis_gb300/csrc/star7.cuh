@@ -73,6 +73,7 @@ struct BorderTable {
     scafes_border_form rule[SCAFES_BORDER_CLASSES];
     const double* g_hi[3] = {nullptr, nullptr, nullptr};  // G_C, G_D, G_E (FP64) or null
     double t_center = 0.0, t_rate = 1.0;
+    bool affine = true;  // no higher orders and the default basis
 };
 
 // Border nodes (within nl of a face) of an nx x ny x nz grid.

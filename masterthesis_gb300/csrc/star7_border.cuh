@@ -1,6 +1,8 @@
 // The new value of one border node, for the kernels that deal with the border
 // nodes apart from the inner ones (star7_loop.cuh, star7_march.cuh), in full
-// warps.  Same operations in the same order as the tile engine's border paths.
+// warps.  Same operations in the same order as the tile engine's border paths,
+// inline: a call would pass the job through local memory, which each step of
+// a loop finds flushed from L1.
 #pragma once
 
 #include "star7_tile.cuh"
@@ -25,11 +27,11 @@ __device__ __forceinline__ typename P::T border_value_at(const TileJob<typename 
         const T s = y > 0 ? at(0, -1, 0) : P::zero(), n = y < L.ny - 1 ? at(0, 1, 0) : P::zero();
         const T b = z > 0 ? at(0, 0, -1) : P::zero(), t = z < L.nz - 1 ? at(0, 0, 1) : P::zero();
         if constexpr (BORDER == SCAFES_BORDER_NODES) {
-            return node_rule<P>(J, x, y, z, u, w, e, s, n, b, t);
+            return node_rule_value<P>(J, x, y, z, u, w, e, s, n, b, t);
         } else if constexpr (BORDER == SCAFES_BORDER_TABLE) {
             const int mask = (x == 0) | ((x == L.nx - 1) << 1) | ((y == 0) << 2) | ((y == L.ny - 1) << 3) |
                              ((z == 0) << 4) | ((z == L.nz - 1) << 5);
-            return table_rule<P, SRC != SRC_NONE, SRC == SRC_AB>(J, mask, o, u, w, e, s, n, b, t);
+            return table_rule_value<P, SRC != SRC_NONE, SRC == SRC_AB>(J, mask, o, u, w, e, s, n, b, t);
         } else {
             // Mirror border: the last face (in direction order x-, x+, y-,
             // y+, z-, z+) the node lies on decides.

@@ -10,8 +10,8 @@
 // barrier (a counter in global memory) ends the step.  The inner nodes and
 // the border nodes are numbered separately, so a warp holds one kind and the
 // border rules (a chain of FP64 operations) run in full warps instead of in
-// one or two lanes of every warp at a face.  A step now takes 2.15, 3.5 and
-// 5.2 us on those three; of the 2.1 us of an almost empty step, most is the
+// one or two lanes of every warp at a face.  A step now takes 2.1, 2.7 and
+// 4.6 us on those three; of the 2.1 us of an almost empty step, most is the
 // round trips to L2 (neighbours, store and release, counter, acquire).  Two
 // warps per CTA and up to one CTA per SM: 1, 2 and 4 warps measure the same
 // within 2 %, 16 warps 20 % slower at 17 x 15 x 16.

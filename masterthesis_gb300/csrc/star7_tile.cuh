@@ -83,10 +83,10 @@ struct TileJob {
 // one or two lanes, and a warp's FP64 instructions (and FP32<->FP64
 // conversions) hold GB300's narrow FP64 pipe whatever the active lanes.
 template <class P>
-__device__ __noinline__ typename P::T node_rule(const TileJob<typename P::T>& J, int x, int y, int z,
-                                                 typename P::T u, typename P::T w, typename P::T e,
-                                                 typename P::T s, typename P::T n, typename P::T b,
-                                                 typename P::T t) {
+__device__ __forceinline__ typename P::T node_rule_value(const TileJob<typename P::T>& J, int x, int y, int z,
+                                                         typename P::T u, typename P::T w, typename P::T e,
+                                                         typename P::T s, typename P::T n, typename P::T b,
+                                                         typename P::T t) {
     if constexpr (std::is_same<P, PolF32>::value) {
         const float* Rf = reinterpret_cast<const float*>(J.nodes) + 8 * border_node_index(J.L, x, y, z);
         float v = fmaf(Rf[0], u, Rf[7]);
@@ -109,14 +109,23 @@ __device__ __noinline__ typename P::T node_rule(const TileJob<typename P::T>& J,
     return P::from_double(v);
 }
 
+// Out of line for the tiles, whose hot loop must not carry its registers.
+template <class P>
+__device__ __noinline__ typename P::T node_rule(const TileJob<typename P::T>& J, int x, int y, int z,
+                                                 typename P::T u, typename P::T w, typename P::T e,
+                                                 typename P::T s, typename P::T n, typename P::T b,
+                                                 typename P::T t) {
+    return node_rule_value<P>(J, x, y, z, u, w, e, s, n, b, t);
+}
+
 // The table rule of a border node, in FP64 whatever the element type (border
 // nodes are a thin layer; the rule needs the reference's rounding, not
 // speed).  mask: faces the node lies on; off: its element offset.
 template <class P, bool HAS_F, bool HAS_FB>
-__device__ __noinline__ typename P::T table_rule(const TileJob<typename P::T>& J, int mask, long long off,
-                                                  typename P::T u, typename P::T w, typename P::T e,
-                                                  typename P::T s, typename P::T n, typename P::T b,
-                                                  typename P::T t) {
+__device__ __forceinline__ typename P::T table_rule_value(const TileJob<typename P::T>& J, int mask, long long off,
+                                                          typename P::T u, typename P::T w, typename P::T e,
+                                                          typename P::T s, typename P::T n, typename P::T b,
+                                                          typename P::T t) {
     const BorderTable& B = *J.table;
     const scafes_border_form& R = B.rule[mask];
     const double ud = P::to_double(u);
@@ -133,26 +142,40 @@ __device__ __noinline__ typename P::T table_rule(const TileJob<typename P::T>& J
         v = fma(R.cf, f, v);
     }
     // G(t) = G_A + s (G_B + s (G_C + s (G_D + s G_E))), s = (time - tc) * rate;
-    // with the default basis and no higher orders this is G_A + time * G_B.
+    // with the default basis and no higher orders (`affine`, 4 instead of 14
+    // FP64 operations, the same value) this is G_A + time * G_B.
     const double g0 = J.ga ? P::to_double(J.ga[off]) : P::to_double(J.gval);
     const double g1 = J.gb ? P::to_double(J.gb[off]) : 0.0;
-    double gh[3];
+    if (B.affine) {
+        v = fma(R.cg_old, fma(g1, J.time_old.d, g0), v);
+        v = fma(R.cg_new, fma(g1, J.time_new.d, g0), v);
+    } else {
+        double gh[3];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) gh[k] = B.g_hi[k] ? B.g_hi[k][off] : 0.0;
-    auto G = [&](double time) {
-        const double s = __dmul_rn(__dsub_rn(time, B.t_center), B.t_rate);
-        double g = fma(gh[2], s, gh[1]);
-        g = fma(g, s, gh[0]);
-        g = fma(g, s, g1);
-        return fma(g, s, g0);
-    };
-    v = fma(R.cg_old, G(J.time_old.d), v);
-    v = fma(R.cg_new, G(J.time_new.d), v);
+        for (int k = 0; k < 3; ++k) gh[k] = B.g_hi[k] ? B.g_hi[k][off] : 0.0;
+        auto G = [&](double time) {
+            const double s = __dmul_rn(__dsub_rn(time, B.t_center), B.t_rate);
+            double g = fma(gh[2], s, gh[1]);
+            g = fma(g, s, gh[0]);
+            g = fma(g, s, g1);
+            return fma(g, s, g0);
+        };
+        v = fma(R.cg_old, G(J.time_old.d), v);
+        v = fma(R.cg_new, G(J.time_new.d), v);
+    }
     if (R.cu4 != 0.0) {
         const double u2 = ud * ud;
         v = fma(R.cu4, u2 * u2, v);
     }
     return P::from_double(v);
+}
+
+template <class P, bool HAS_F, bool HAS_FB>
+__device__ __noinline__ typename P::T table_rule(const TileJob<typename P::T>& J, int mask, long long off,
+                                                  typename P::T u, typename P::T w, typename P::T e,
+                                                  typename P::T s, typename P::T n, typename P::T b,
+                                                  typename P::T t) {
+    return table_rule_value<P, HAS_F, HAS_FB>(J, mask, off, u, w, e, s, n, b, t);
 }
 
 // Initialises the ring's mbarriers (thread 0) -- once per CTA.
