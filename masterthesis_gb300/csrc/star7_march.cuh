@@ -6,14 +6,18 @@
 // inner nodes only, so every border kind, source and layer count is one
 // kernel and no warp at a face runs a rule for one or two lanes.
 //
-// The FP64 sweep is bound by the FP64 pipe (16 clocks of an SM per warp
-// instruction, 4 per node) and by the integer sums; the tile engine
+// The FP64 sweep is bound by the FP64 pipe (16 to 19 clocks of an SM per warp
+// instruction) and the integer ALU, which takes the neighbour sums and half
+// or all of the centre's products (star7_policies.cuh).  The tile engine
 // (star7_tile.cuh) spends as many instructions again on its ring -- barrier
 // waits, block barriers, addresses -- as on the node: 268 issued per 32
-// nodes against 175 here, which the memory path does not need, since FP64
-// asks it for 2 TB/s.  512^3: 1178 -> 1077 us (124.6 GLUP/s, FP64 pipe 82 %
-// busy, integer ALU 55 %); 256^3: 175 -> 145 us.  Six CTAs of 256 threads (40
-// registers, nothing spilled): 4, 5 and 8 CTAs measure 2 % to 0.2 % slower.
+// nodes, where this loop took 175 with the same arithmetic, and the memory
+// path does not need the ring, since FP64 asks it for 2 TB/s.  us per step at
+// 512^3 / 256^3: tile 1178 / 175; this loop 1093 / 150, with the adder of
+// dadd_int.cuh as it is now 1077 / 145, with overlapped launches 1072 / 141, with
+// every second plane's products on the integer pipe 1015 / 135 (132 GLUP/s).
+// Six CTAs of 256 threads (40 registers, nothing spilled): 4, 5 and 8 CTAs
+// measured 2 % to 0.2 % slower.
 // FP32 and pairs are bound by the memory path, where the tile engine's ring
 // keeps more bytes in flight (f32 400^3 89 against 123 us); they come here
 // with rule tables and several border layers only.
@@ -99,8 +103,12 @@ __device__ __forceinline__ void march_rows_of(const Layout& L, const Star7Coeffs
         if (AHEAD) above[i] = uo[o + ro[i] + pz];
     }
     if (AHEAD) fetch(o, f, c0, ca);
-#pragma unroll 2
-    for (int z = z0; z < z1; ++z, o += pz) {
+    // Without a source the FP64 update is short of either pipe by turns:
+    // bound by the integer ALU (76 % busy, FP64 61 %) with every c0 u there, by
+    // FP64 (82 %, ALU 55 %) with none, 141 us at 256^3 both ways.  Every second
+    // plane's goes to the FP64 pipe: 135 us, at 512^3 1072 -> 1015.
+    constexpr bool HALF = std::is_same<P, PolF64>::value && !HAS_F && !VC;
+    auto plane = [&](int z, auto int_mul) {
         T w[R], e[R], v[R], next[R], fn[R], c0n[R], can[R];
         const long long on = z + 1 < z1 ? o + pz : o;  // the last plane loads its own again
         const T ym = uo[o - py], yp = uo[o + rn];
@@ -116,7 +124,7 @@ __device__ __forceinline__ void march_rows_of(const Layout& L, const Star7Coeffs
         if constexpr (VC)
             P::template star_vc_rows<HAS_F, R>(c, below, cur, above, ym, yp, w, e, f, c0, ca, 1, v, skip);
         else
-            P::template star_rows<HAS_F, R>(c, below, cur, above, ym, yp, w, e, f, v, skip);
+            P::template star_rows<HAS_F, R, decltype(int_mul)::value>(c, below, cur, above, ym, yp, w, e, f, v, skip);
 #pragma unroll
         for (int i = 0; i < R; ++i)
             if (R == 1 || !((skip >> i) & 1u)) un[o + i * py] = v[i];
@@ -131,7 +139,15 @@ __device__ __forceinline__ void march_rows_of(const Layout& L, const Star7Coeffs
                 ca[i] = can[i];
             }
         }
+        o += pz;
+    };
+    int z = z0;
+#pragma unroll 1
+    for (; z + 1 < z1; z += 2) {
+        plane(z, std::true_type{});
+        plane(z + 1, std::integral_constant<bool, !HALF>{});
     }
+    if (z < z1) plane(z, std::true_type{});
 }
 
 template <class P, int SRC, int BORDER, bool VC, int R, int MINB>

@@ -72,10 +72,10 @@ struct PolF64 {
         for (int k = 0; k < R; ++k) out[k] = r.v[k];
     }
     // out[k] = c * a[k] on the integer pipe (dmul_bits: the FP64 multiplier's
-    // bits), with the same fallback as the sums.  Without a source it is even
-    // (256^3 142 / 141 us, both pipes 60 - 80 % busy), with one, five FP64
-    // operations to four, it pays: 256^3 175 -> 160, the ensemble 325 -> 303
-    // (both with star7_march.cuh's loads ahead), the loop at 64^3 5.06 -> 4.78.
+    // bits), with the same fallback as the sums.  Without a source the large
+    // sweep wants it for half of the nodes (star7_march.cuh), with one, five
+    // FP64 operations to four, for all: 256^3 175 -> 160, the ensemble 325 ->
+    // 303 (with star7_march.cuh's loads ahead), the loop at 64^3 5.06 -> 4.78.
     template <int R>
     static __device__ __noinline__ Nodes<R> fp64_mul(double c, Nodes<R> a) {
         Nodes<R> r;
@@ -175,8 +175,8 @@ struct PolF64 {
     }
     // All R rows of one thread (row k's s/n neighbours are rows k-1/k+1,
     // ym/yp beyond the ends).  Bit k of `skip`: row k's result is replaced
-    // by the caller.
-    template <bool HAS_F, int R>
+    // by the caller.  INT_MUL: c0 u on the integer pipe, else on the FP64 pipe.
+    template <bool HAS_F, int R, bool INT_MUL = true>
     static __device__ __forceinline__ void star_rows(const Star7Coeffs& c, const T (&below)[R], const T (&cur)[R],
                                                      const T (&above)[R], T ym, T yp, const T (&w)[R],
                                                      const T (&e)[R], const T (&f)[R], T (&v)[R],
@@ -189,7 +189,12 @@ struct PolF64 {
         }
         sums<R>(w, e, s, n, below, above, sx, sy, sz, skip);
         T c0u[R];
-        products<R>(c.m0, c.c0, cur, c0u, skip);
+        if constexpr (INT_MUL) {
+            products<R>(c.m0, c.c0, cur, c0u, skip);
+        } else {
+#pragma unroll
+            for (int k = 0; k < R; ++k) c0u[k] = c.c0 * cur[k];
+        }
 #pragma unroll
         for (int k = 0; k < R; ++k) v[k] = star_of_sums<HAS_F>(c, c0u[k], sx[k], sy[k], sz[k], f[k]);
     }
@@ -238,7 +243,7 @@ struct PolF32 {
     }
     // All R rows of one thread (row k's s/n neighbours are rows k-1/k+1,
     // ym/yp beyond the ends).
-    template <bool HAS_F, int R>
+    template <bool HAS_F, int R, bool = true>
     static __device__ __forceinline__ void star_rows(const Star7Coeffs& c, const T (&below)[R], const T (&cur)[R],
                                                      const T (&above)[R], T ym, T yp, const T (&w)[R],
                                                      const T (&e)[R], const T (&f)[R], T (&v)[R],
@@ -397,7 +402,7 @@ struct PolF32x2 {
         o1 = make_float2(-S.y, -E.y);
     }
 
-    template <bool HAS_F, int R>
+    template <bool HAS_F, int R, bool = true>
     static __device__ __forceinline__ void star_rows(const Star7Coeffs& c, const T (&below)[R], const T (&cur)[R],
                                                      const T (&above)[R], T ym, T yp, const T (&w)[R],
                                                      const T (&e)[R], const T (&f)[R], T (&v)[R],
