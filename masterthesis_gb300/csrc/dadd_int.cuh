@@ -103,7 +103,8 @@ SCAFES_HD uint64_t dadd_bits(uint64_t a, uint64_t b, bool& ok) {
     r += (uint64_t)(0x1ffu + (((uint32_t)r >> 10) & 1u));
     r >>= 10;
     const uint32_t top = e - 0x04000000u;  // exponent field - 64
-    ok = (e - m <= 0x00900000u || m == 0u) && (top <= 0x7bd00000u || mag == 0u);
+    // A zero sum is right at any exponent but that of infinities and NaNs.
+    ok = (e - m <= 0x00900000u || m == 0u) && (top <= 0x7bd00000u || (mag == 0u && e < 0x7ff00000u));
     const uint32_t hi = ((uint32_t)(r >> 32) + e + ((uint32_t)(1 - lz) << 20)) | ((ah ^ (uint32_t)n) & 0x80000000u);
     return mag ? ((uint64_t)hi << 32) | (uint32_t)r : 0u;
 }

@@ -33,6 +33,7 @@ int main(int argc, char** argv) {
             if (kind == 1) b = (a ^ (1ull << 63)) + (rnd() % 9) - 4;      // almost cancels
             if (kind == 2) a &= ~0xffffffull, b &= ~0xffffffull;          // ties
             if (kind == 3) a |= 0xfffffffffffffull, b |= rnd() & 0xfffffffffffffull;
+            if (kind == 5 && i % 16 == 5) b = a ^ (1ull << 63);            // cancels, infinities and NaNs too
         } else if (kind == 6) {
             if (rnd() & 1) a &= 1ull << 63;
             if (rnd() & 1) b &= 1ull << 63;
