@@ -86,7 +86,8 @@ struct MarchItem {
 // to 60 11.9 / 63; pairs 226 / 163 and 9.8 / 30, FP32 155 / 76 and 7.9 / 14:
 // the memory-bound types keep the TMA ring (and its {16,4} tile) from
 // kMarchNodes nodes on, about where the fields outgrow L2.  FP64 takes 5 CTAs
-// per SM (48 registers): 4 (64, no spills) 350, 6 (40) 338.
+// per SM (48 registers): 4 (64, no spills) 350, 6 (40) 338.  With the
+// centre's product on the integer pipe too the FP64 case went 327 -> 298.
 template <class P, int R, int MINB>
 __global__ void __launch_bounds__(MARCH_THREADS, MINB)
 batch_march(const BatchInst* __restrict__ inst, const NodeOrder* __restrict__ order,
