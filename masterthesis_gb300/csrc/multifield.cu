@@ -12,7 +12,7 @@
 // schemes here follow the textbook forms written out in the oracle
 // (orc_lame, orc_yee), which the tests use as the reference.
 //
-// Both are bound by the FP64 pipe on GB300 in FP64 (Lame: 44 operations per
+// Both are bound by the FP64 pipe on GB300 in FP64 (Lame: 45 operations per
 // node, Yee: 24 per cell and step), so the kernels read neighbours straight
 // from global memory through L1 instead of staging tiles, and move part of
 // the sums to the integer pipe (dadd_int.cuh).  The FP32-pair Lame kernel
@@ -135,30 +135,32 @@ __device__ __forceinline__ void combine(const double (&a)[N], const double (&b)[
     }
 }
 
-// The FP64 step.  Written out per node it takes 54 FP64 operations, 24 of
-// them for the six mixed derivatives; but with D_q v = v(+q) - v(-q), the
-// mixed terms of component c are one difference along c of
-//   S_c = sum over q != c of k_q D_q u_q,
-// and the D_q are shared between the components: 14 operations (three D, two
-// products, S_x, S_y, S_z, and a difference and an FMA per component), 44 in
-// all.  S_z stays with its column; S_x and S_y go through shared memory, the
-// tile's threads also computing the S of the nodes around it.  The nine
-// second differences' sums u(+p) + u(-p) go to the integer pipe, which leaves
-// 35; the other sums and differences are FMAs with a one in a register: GB300
-// issues a DFMA in 16 clocks of an SM and a DADD or DMUL in 19.
+// The FP64 step.  Written out per node (k_lame) it takes 54 FP64 operations,
+// 18 of them for the differences of the six mixed derivatives; but with
+// D_q v = v(+q) - v(-q), d_cq u_q is D_q u_q(+c) - D_q u_q(-c), the same bits,
+// and the D_q are shared between nodes and components: three of them and a
+// difference and an FMA per mixed term, 45 operations in all.  D of the planes
+// above and below stays with its column; D of the neighbours in x and y goes
+// through shared memory, the tile's threads also computing it for the nodes
+// around the tile.  The nine second differences' sums u(+p) + u(-p) go to the
+// integer pipe, which leaves 36; the other sums and differences are FMAs with
+// a one in a register: GB300 issues a DFMA in 16 clocks of an SM and a DADD or
+// DMUL in 19.  Every rounding is the written-out form's, so are the results.
 // A CTA marches a few planes of a column tile that fits the grid's width
 // (make_column_tile); CTAs in front zero the border nodes of u^{n+1}.
 // us per step at 129 x 111 x 101: columns of 16 planes, written out per node
-// 252; this split 141; with 3, 6, 9 integer sums 134, 127, 119 (FP64 pipe 79 %
-// busy, ALU 35 %); with integer D as well 119 - 124.  Error against a
-// 113-bit run (60 - 120 steps, three grids): 0.96 of the written-out form's.
+// 252; this split 115 (FP64 pipe 77 % busy, ALU 38 %, 36.3 FP64 instructions
+// per node).  Before, with the products summed per component first (35 on the
+// pipe, other roundings): 118; that form with 0, 3, 6 of the integer sums took
+// 141, 134, 127, and with integer D as well 119 - 124.  u + ((u - u_prev) +
+// increments) errs 4.6 times less against a 113-bit run, but is slower (the
+// pass of 400 steps 54.3 ms against 49.3) and no longer the scheme's roundings.
 struct LameMarch {
     const double* u;
     double* up;
     long long comp;
     double a[3][3];  // as LameCoef
-    double k[3];     // k_q = tau^2/rho (lambda + mu) / (4 h_q)
-    double ih[3];    // 1 / h_c
+    double b[3][3];
     double one;
     Layout L;
     NodeOrder o;
@@ -168,10 +170,12 @@ struct LameMarch {
     int zchunk;
 };
 
-constexpr int LSX = MARCH_THREADS + 2 * 16, LSY = MARCH_THREADS + 2 * 64;  // S with its halo: h <= 16, w <= 64
+constexpr int LSX = MARCH_THREADS + 2 * 16, LSY = MARCH_THREADS + 2 * 64;  // a tile with its halo: h <= 16, w <= 64
 
 __global__ void __launch_bounds__(MARCH_THREADS, 3) k_lame_march(const __grid_constant__ LameMarch A) {
-    __shared__ double sx[2][LSX], sy[2][LSY];
+    // D_y u_y and D_z u_z with the columns left and right of the tile, D_x u_x
+    // and D_z u_z with the rows before and after it.
+    __shared__ double yx[2][LSX], zx[2][LSX], xy[2][LSY], zy[2][LSY];
     const Layout& L = A.L;
     step_wait();
     if (blockIdx.x < A.border_ctas) {
@@ -190,15 +194,15 @@ __global__ void __launch_bounds__(MARCH_THREADS, 3) k_lame_march(const __grid_co
     const int row = (int)fastdiv(threadIdx.x, A.ct.w), col = (int)threadIdx.x - row * W;
     const bool main = row < H;
     // Threads beyond the grid compute on its last nodes and write nothing;
-    // those on its last column and row provide S only.
+    // those on its last column and row provide D only.
     const int x = min(x0 + col, L.nx - 1), y = min(y0 + row, L.ny - 1);
     const bool live = main && x0 + col < L.nx - 1 && y0 + row < L.ny - 1;
     const int z0 = (int)kz * A.zchunk + 1, z1 = min(z0 + A.zchunk, L.nz - 1);
     const long long py = L.pitch, pz = L.plane;
     const int xp = x < L.nx - 1 ? 1 : 0;
     const long long yp = y < L.ny - 1 ? py : 0;
-    // One S node around the tile per thread: columns -1 and W of its rows
-    // (S_x), then rows -1 and H of its columns (S_y).
+    // One node around the tile per thread: columns -1 and W of its rows,
+    // then rows -1 and H of its columns.
     const int h = (int)threadIdx.x;
     const bool hx = h < 2 * H, hy = !hx && h < 2 * H + 2 * W;
     const int g = h - 2 * H;
@@ -211,33 +215,30 @@ __global__ void __launch_bounds__(MARCH_THREADS, 3) k_lame_march(const __grid_co
     const double* u1 = A.u + A.comp;
     const double* u2 = A.u + 2 * A.comp;
     long long o = L.idx(x, y, z0), ho = (hx || hy) ? L.idx(hxx, hyy, z0) : 0;
-    // k_x D_x u, k_y D_y v and their sum S_z at a node.
-    auto dxy = [&](long long m, double& qx, double& qy) {
-        qx = A.k[0] * fsub(u0[m + xp], u0[m - 1], mone);
-        qy = A.k[1] * fsub(u1[m + yp], u1[m - py], mone);
-        return fadd(qx, qy, one);
-    };
-    double qx, qy, szb, szc, wb = u2[o - pz], wc = u2[o];
-    szb = dxy(o - pz, qx, qy);
-    szc = dxy(o, qx, qy);
+    auto dx = [&](long long m) { return fsub(u0[m + xp], u0[m - 1], mone); };
+    auto dy = [&](long long m) { return fsub(u1[m + yp], u1[m - py], mone); };
+    // D_x u_x and D_y u_y below, at and above the plane.
+    double wb = u2[o - pz], wc = u2[o];
+    double dxb = dx(o - pz), dyb = dy(o - pz), dxc = dx(o), dyc = dy(o);
     int p = 0;
     for (int z = z0; z < z1; ++z, o += pz, ho += pz, p ^= 1) {
         const double wa = u2[o + pz];
         const double dz = fsub(wa, wb, mone);
         if (main) {
-            sx[p][row * (W + 2) + col + 1] = fma(A.k[2], dz, qy);
-            sy[p][(row + 1) * W + col] = fma(A.k[2], dz, qx);
+            const int a = row * (W + 2) + col + 1, b = (row + 1) * W + col;
+            yx[p][a] = dyc, zx[p][a] = dz;
+            xy[p][b] = dxc, zy[p][b] = dz;
         }
         if (hx) {
-            const double d = fsub(u2[ho + pz], u2[ho - pz], mone);
-            const double e = fsub(u1[ho + hdy], u1[ho - hdy], mone);
-            sx[p][hrow * (W + 2) + hcol + 1] = fma(A.k[2], d, A.k[1] * e);
+            const int a = hrow * (W + 2) + hcol + 1;
+            yx[p][a] = fsub(u1[ho + hdy], u1[ho - hdy], mone);
+            zx[p][a] = fsub(u2[ho + pz], u2[ho - pz], mone);
         } else if (hy) {
-            const double d = fsub(u2[ho + pz], u2[ho - pz], mone);
-            const double e = fsub(u0[ho + hdx], u0[ho - hdx], mone);
-            sy[p][(hrow + 1) * W + hcol] = fma(A.k[2], d, A.k[0] * e);
+            const int b = (hrow + 1) * W + hcol;
+            xy[p][b] = fsub(u0[ho + hdx], u0[ho - hdx], mone);
+            zy[p][b] = fsub(u2[ho + pz], u2[ho - pz], mone);
         }
-        const double sza = dxy(o + pz, qx, qy);
+        const double dxa = dx(o + pz), dya = dy(o + pz);
         double acc[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -253,18 +254,22 @@ __global__ void __launch_bounds__(MARCH_THREADS, 3) k_lame_march(const __grid_co
             acc[c] = fma(A.a[c][1], ly, acc[c]);
             acc[c] = fma(A.a[c][2], lz, acc[c]);
         }
-        __syncthreads();  // S of plane z is complete; the other buffer is free
+        __syncthreads();  // D of plane z is complete; the other buffer is free
         if (live) {
-            const double* a = &sx[p][row * (W + 2) + col + 1];
-            const double* b = &sy[p][(row + 1) * W + col];
-            A.up[o] = fma(A.ih[0], fsub(a[1], a[-1], mone), acc[0]);
-            A.up[o + A.comp] = fma(A.ih[1], fsub(b[W], b[-W], mone), acc[1]);
-            A.up[o + 2 * A.comp] = fma(A.ih[2], fsub(sza, szb, mone), acc[2]);
+            const int a = row * (W + 2) + col + 1, b = (row + 1) * W + col;
+            acc[0] = fma(A.b[0][1], fsub(yx[p][a + 1], yx[p][a - 1], mone), acc[0]);
+            acc[1] = fma(A.b[1][0], fsub(xy[p][b + W], xy[p][b - W], mone), acc[1]);
+            acc[2] = fma(A.b[2][0], fsub(dxa, dxb, mone), acc[2]);
+            A.up[o] = fma(A.b[0][2], fsub(zx[p][a + 1], zx[p][a - 1], mone), acc[0]);
+            A.up[o + A.comp] = fma(A.b[1][2], fsub(zy[p][b + W], zy[p][b - W], mone), acc[1]);
+            A.up[o + 2 * A.comp] = fma(A.b[2][1], fsub(dya, dyb, mone), acc[2]);
         }
         wb = wc;
         wc = wa;
-        szb = szc;
-        szc = sza;
+        dxb = dxc;
+        dxc = dxa;
+        dyb = dyc;
+        dyc = dya;
     }
     step_next();
 }
@@ -1177,10 +1182,7 @@ extern "C" int scafes_mf_step(scafes_mf* h, int n_steps) {
         if (!x2 && (long long)L.nx * L.ny * L.nz <= kMaxNumbered) {
             F.comp = comp;
             memcpy(F.a, K.a, sizeof(F.a));
-            for (int p = 0; p < 3; ++p) {
-                F.k[p] = s * (lam + mu) / (4.0 * hh[p]);
-                F.ih[p] = 1.0 / hh[p];
-            }
+            memcpy(F.b, K.b, sizeof(F.b));
             F.one = 1.0;
             F.L = L;
             F.o = make_node_order(L.nx, L.ny, L.nz, 1);
