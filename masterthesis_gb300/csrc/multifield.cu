@@ -91,8 +91,7 @@ k_lame(const double* __restrict__ u, double* __restrict__ up, LameCoef K, Layout
     }
 }
 
-// a + b and a - b as FMAs (same rounding).
-__device__ __forceinline__ double fadd(double a, double b, double one) { return fma(a, one, b); }
+// a - b as an FMA (same rounding).
 __device__ __forceinline__ double fsub(double a, double b, double mone) { return fma(b, mone, a); }
 
 // N sums (NEG: differences) of a[i] and b[i]: the first NI on the integer pipe
