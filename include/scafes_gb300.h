@@ -313,13 +313,16 @@ int scafes_gpu_synchronize(scafes_handle* h);
 
 /* No counterpart in the reference (its node loop has no tunables): times
  * n_steps sweeps with each tile variant of the sweep kernel (32 x BY CTA
- * tile, R rows per thread) on the uploaded problem, keeps the fastest for
- * later scafes_gpu_step calls and returns it (1-based) in *chosen and the
- * per-variant ms per step in ms_per_tile[4] (may be NULL); a sweep by plain
- * loads is timed too and takes the tile's place if it is faster; then times
- * temporal blocking depth 2 where the problem allows it and keeps it if it
- * is faster per step (scafes_gpu_temporal_depth).  The iterate and the step
- * counter are restored afterwards.  Allocates one temporary copy of the
+ * tile, R rows per thread) on the uploaded problem and returns the fastest
+ * variant (1-based) in *chosen and the per-variant ms per step in
+ * ms_per_tile[4] (may be NULL); a sweep by plain loads is timed too and takes
+ * the tile's place if it is faster; then times temporal blocking depth 2 where
+ * the problem allows it and takes it if it is faster per step
+ * (scafes_gpu_temporal_depth); and then, where the caller fixed no tile or
+ * depth and the grid is small enough, the one-launch loop against these, over
+ * 64 steps or n_steps if that is more.  What was fastest serves the later
+ * scafes_gpu_step calls.  The iterate and the step counter are restored
+ * afterwards.  Allocates one temporary copy of the
  * iterate. */
 int scafes_gpu_autotune(scafes_handle* h, int n_steps, int* chosen,
                         float* ms_per_tile);

@@ -336,8 +336,8 @@ class Plain:
         return gk, gu
 
     def autotune(self, n_steps: int = 20):
-        """Picks the fastest sweep tile variant on this problem; returns
-        (chosen 1-based variant, ms per step of each variant)."""
+        """Picks the fastest schedule on this problem for later steps; returns
+        (fastest 1-based sweep tile variant, ms per step of each variant)."""
         chosen = C.c_int()
         ms = (C.c_float * 4)()
         _check(lib().scafes_gpu_autotune(self.h, n_steps, C.byref(chosen), ms), self.h)

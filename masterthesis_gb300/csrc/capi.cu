@@ -40,6 +40,11 @@ int fail(std::string* where, int code, const char* fmt, ...) {
 // memory takes without waiting for the stream.
 constexpr int kLoopSteps = 1024;
 
+// Fewest steps over which the autotuner compares the loop with the sweeps: in
+// a handful of steps the loop's own launch and copies (some 10 us) weigh as
+// much as the steps, in the hundreds of a solve they do not.
+constexpr int kLoopTrial = 64;
+
 // Bytes of host staging used for precision conversions (per slab).
 constexpr size_t kStageBytes = 64ull << 20;
 
@@ -60,6 +65,8 @@ struct scafes_handle {
     int tile = -1;                        // schedule of the sweep (tile variant or STAR7_MARCH), -1 the default
     int depth = 1;                        // temporal blocking depth (1 or 2)
     bool schedule_set = false;            // the caller chose the tile or the depth: one launch per pass
+    bool sweeps_tuned = false;            // the autotuner measured the sweeps faster than the one-launch loop
+    bool loop_too_large = false;          // the device cannot hold the loop's CTAs at once
     // One-launch time loop of small grids: the grid barrier's counter and
     // the times of up to kLoopSteps steps (made on first use).
     unsigned* arrivals = nullptr;
@@ -536,7 +543,7 @@ static const CUtensorMap* tb_map(scafes_handle* h, int buf) {
 // schedule, several steps, and not under stream capture (the step times are
 // copied from host memory that a replay would find gone).
 static bool takes_loop(scafes_handle* h, const Star7Launch& a, int n_steps) {
-    if (h->schedule_set || n_steps < 3) return false;
+    if (h->schedule_set || h->sweeps_tuned || h->loop_too_large || n_steps < 3) return false;
     if ((long long)n_nodes(h) > star7_loop_max_nodes(a)) return false;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     return cudaStreamIsCapturing(h->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
@@ -550,7 +557,7 @@ static void step_times(const scafes_handle* h, int t, double& t_old, double& t_n
 }
 
 // Runs the steps as one-launch loops; *done counts them (fewer than n_steps,
-// and h->schedule_set from then on, where the device cannot hold the loop's
+// and h->loop_too_large from then on, where the device cannot hold the loop's
 // CTAs at once).
 static int loop_steps(scafes_handle* h, const Star7Launch& a, int n_steps, int* done, int* launches) {
     const bool timed = a.fb || a.gb || a.border == SCAFES_BORDER_TABLE || a.border == SCAFES_BORDER_MIRROR_POW2;
@@ -580,7 +587,7 @@ static int loop_steps(scafes_handle* h, const Star7Launch& a, int n_steps, int* 
         const cudaError_t e = launch_star7_loop(q, h->stream);
         if (e == cudaErrorCooperativeLaunchTooLarge) {
             cudaGetLastError();
-            h->schedule_set = true;
+            h->loop_too_large = true;
             return SCAFES_OK;
         }
         if (e != cudaSuccess)
@@ -1092,6 +1099,28 @@ extern "C" int scafes_gpu_autotune(scafes_handle* h, int n_steps, int* chosen, f
         }
         h->depth = keep;
     }
+    // The one-launch loop, where it applies (the caller set no tile or depth),
+    // against the best sweeps.
+    const bool tuned_before = h->sweeps_tuned;
+    bool sweeps_tuned = false;
+    if (!h->schedule_set) {
+        const int n = n_steps > kLoopTrial ? n_steps : kLoopTrial;
+        float ms[2] = {0.f, 0.f};
+        bool looped = false;
+        h->sweeps_tuned = false;
+        for (int k = 0; k < 2 && e == cudaSuccess && rc == SCAFES_OK; ++k) {
+            rc = step_impl(h, n, best, false, best_depth, k == 0);  // warm-up
+            if (rc == SCAFES_OK) rc = step_impl(h, n, best, true, best_depth, k == 0);
+            if (rc != SCAFES_OK) break;
+            if (k == 0) looped = h->launches < n / best_depth;
+            if (!looped) break;
+            e = cudaEventSynchronize(h->ev1);
+            if (e == cudaSuccess) e = cudaEventElapsedTime(&ms[k], h->ev0, h->ev1);
+        }
+        sweeps_tuned = looped && ms[1] < ms[0];
+        if (looped && !sweeps_tuned) best_depth = 1;
+        h->sweeps_tuned = tuned_before;
+    }
     if (e == cudaSuccess) e = cudaMemcpyAsync(h->u[cur_save], save, bytes, cudaMemcpyDeviceToDevice, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     cudaFree(save);
@@ -1105,6 +1134,7 @@ extern "C" int scafes_gpu_autotune(scafes_handle* h, int n_steps, int* chosen, f
     if (rc) return rc;
     h->tile = best;
     h->depth = best_depth;
+    h->sweeps_tuned = sweeps_tuned;
     if (chosen) *chosen = best_tile + 1;
     return SCAFES_OK;
 }

@@ -1,0 +1,49 @@
+"""What the schedules choose on the GPU: the autotuner's choice is what later
+steps run.  Times are compared between schedules of the same problem, measured
+one after the other; the margins are far below what a wrong choice costs."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def heat(M, n, prec, tile=0, seed=1):
+    rng = np.random.default_rng(seed)
+    shape = (n[2], n[1], n[0])
+    tau = 0.4 / (2.0 * sum((m - 1) ** 2 for m in n))
+    p = M.Plain(M.make_cfg(n, tau=tau, precision=prec, tile=tile, heat=(1.0, 1.0, 0.3)))
+    p.upload(M.FIELD_U, rng.uniform(0.5, 1.5, shape))
+    return p
+
+
+def us_per_step(p, steps=60):
+    """Best of four step calls, by the device's clock."""
+    best = np.inf
+    for _ in range(4):
+        p.step(steps)
+        p.synchronize()
+        best = min(best, p.last_step_ms())
+    return 1e3 * best / steps
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32", "f32x2"])
+@pytest.mark.parametrize("n", [(17, 15, 16), (64, 48, 40), (160, 160, 160)])
+def test_autotuned_steps_run_what_was_fastest(gpu, prec, n):
+    M = gpu
+    with heat(M, n, prec) as p:
+        for _ in range(2):  # a second call chooses anew
+            _, ms = p.autotune(20)
+            t = us_per_step(p)
+            assert t <= 1.15 * 1e3 * min(ms)
+            launches = p.last_step_launches()
+            assert launches == 30 if p.temporal_depth == 2 else launches in (1, 60)
+
+
+def test_autotune_keeps_one_launch_per_step_of_a_set_tile(gpu):
+    M = gpu
+    with heat(M, (17, 15, 16), "f64", tile=2) as p:
+        p.autotune(5)
+        p.step(8)
+        assert p.last_step_launches() in (4, 8)
