@@ -68,7 +68,9 @@ struct scafes_handle {
     bool sweeps_tuned = false;            // the autotuner measured the sweeps faster than the one-launch loop
     bool loop_too_large = false;          // the device cannot hold the loop's CTAs at once
     // One-launch time loop of small grids: the grid barrier's counter and
-    // the times of up to kLoopSteps steps (made on first use).
+    // the times of up to kLoopSteps steps, behind the partial sums of `red`.
+    // Made with the handle: an allocation in a step call would be refused
+    // while another stream of the program is being captured.
     unsigned* arrivals = nullptr;
     StepTimes* times = nullptr;
     int sms = 1;
@@ -194,8 +196,6 @@ extern "C" void scafes_gpu_destroy(scafes_handle* h) {
     cudaFree(h->stage);
     cudaFree(h->table);
     cudaFree(h->nodes);
-    cudaFree(h->arrivals);
-    cudaFree(h->times);
     cudaFree(h->snap_dev);
     for (int i = 0; i < 2; ++i) {
         if (h->snap_host[i]) cudaFreeHost(h->snap_host[i]);
@@ -255,8 +255,11 @@ extern "C" int scafes_gpu_create(const scafes_cfg* cfg, scafes_handle** out) {
     h->red_blocks = sms * 4;
     h->sms = sms;
     h->schedule_set = cfg->tile > 0;
-    if ((e = cudaMalloc(&h->red, sizeof(double) * 2 * (h->red_blocks + 1))) != cudaSuccess)
+    const size_t partials = sizeof(double) * 2 * (h->red_blocks + 1);
+    if ((e = cudaMalloc(&h->red, partials + sizeof(StepTimes) * kLoopSteps + sizeof(unsigned))) != cudaSuccess)
         return bail(SCAFES_ERR_NOMEM, "cudaMalloc(scratch)", e);
+    h->times = reinterpret_cast<StepTimes*>(reinterpret_cast<char*>(h->red) + partials);
+    h->arrivals = reinterpret_cast<unsigned*>(h->times + kLoopSteps);
     if ((e = cudaMallocHost(&h->red_host, sizeof(double) * 2)) != cudaSuccess)
         return bail(SCAFES_ERR_NOMEM, "cudaMallocHost", e);
     if ((e = cudaStreamSynchronize(h->stream)) != cudaSuccess) return bail(SCAFES_ERR_CUDA, "sync", e);
@@ -561,8 +564,6 @@ static void step_times(const scafes_handle* h, int t, double& t_old, double& t_n
 // CTAs at once).
 static int loop_steps(scafes_handle* h, const Star7Launch& a, int n_steps, int* done, int* launches) {
     const bool timed = a.fb || a.gb || a.border == SCAFES_BORDER_TABLE || a.border == SCAFES_BORDER_MIRROR_POW2;
-    if (!h->arrivals) CUDA_TRY(h, cudaMalloc(&h->arrivals, sizeof(unsigned)));
-    if (timed && !h->times) CUDA_TRY(h, cudaMalloc(&h->times, sizeof(StepTimes) * kLoopSteps));
     std::vector<StepTimes> st;
     Star7Loop q;
     q.step = a;
