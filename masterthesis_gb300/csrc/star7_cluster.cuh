@@ -14,6 +14,7 @@
 // nodes in warps of their own; same operations per node, same bits.
 #pragma once
 
+#include "per_device.cuh"
 #include "star7_loop_args.cuh"
 
 namespace scafes {
@@ -160,9 +161,11 @@ static cudaError_t launch_cluster(const LoopArgs<typename P::T>& A, cudaStream_t
     using T = typename P::T;
     auto kern = star7_cluster<P, SRC, BORDER, VC>;
     *done = false;
-    static int most = -1;  // largest cluster the device holds, 0 none
-    if (most < 0) {
-        most = 0;
+    static PerDevice largest;  // cluster the device holds, 0 none
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const int most = largest.get(dev, [&] {
+        int most = 0;
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) == cudaSuccess &&
             cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
             for (int n = CLUSTER_MAX; n >= 1 && most == 0; n >>= 1) {
@@ -180,7 +183,8 @@ static cudaError_t launch_cluster(const LoopArgs<typename P::T>& A, cudaStream_t
             }
         }
         cudaGetLastError();
-    }
+        return most;
+    });
     const int n = most > 0 ? cluster_ctas<P, BORDER, VC>(A.L, most) : 0;
     if (n == 0) return cudaSuccess;
     const uint32_t planes = (A.L.nz + n - 1) / n, np = (uint32_t)A.L.nx * A.L.ny;
@@ -196,8 +200,15 @@ static cudaError_t launch_cluster(const LoopArgs<typename P::T>& A, cudaStream_t
     attr.val.clusterDim = {(unsigned)n, 1, 1};
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, A);
+    // A cluster that the device will not place has not run: the loop over all
+    // SMs takes the steps.
+    if (e == cudaErrorInvalidClusterSize || e == cudaErrorInvalidConfiguration || e == cudaErrorLaunchOutOfResources) {
+        cudaGetLastError();
+        return cudaSuccess;
+    }
     *done = true;
-    return cudaLaunchKernelEx(&cfg, kern, A);
+    return e;
 }
 
 }  // namespace scafes

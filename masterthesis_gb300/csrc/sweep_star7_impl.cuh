@@ -3,6 +3,7 @@
 // so that the instantiations compile in parallel.
 #pragma once
 
+#include "per_device.cuh"
 #include "star7_tb.cuh"
 #include "star7_tile.cuh"
 #include "step_launch.cuh"
@@ -152,6 +153,12 @@ star7_vc_tma(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUt
 
 // ---- host side ---------------------------------------------------------------
 
+static int device() {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return dev;
+}
+
 static int num_sms() {
     static int n = 0;
     if (n == 0) {
@@ -193,15 +200,15 @@ static cudaError_t launch_typed(const Star7Launch& a, cudaStream_t stream) {
     const Layout& L = a.L;
     if (FS && a.tm_f == nullptr) return cudaErrorInvalidValue;
     auto kern = star7_tma<P, SRC, BORDER, BY, R, NS, FS, ML>;
-    static bool attr = false;
-    if (!attr) {
+    static PerDevice attr;
+    attr.get(device(), [&] {
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::SMEM);
         // The ring lives in shared memory: ask for the largest carveout so
         // that occupancy is not capped by a small L1/shared split.
         cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                              cudaSharedmemCarveoutMaxShared);
-        attr = true;
-    }
+        return 1;
+    });
     T gval;
     to_elem(a.gconst, gval);
     const int zchunk = choose_zchunk(L, BY, std::is_same<P, PolF32>::value && BY == 16 && R == 4 ? 8 : 16);
@@ -246,12 +253,12 @@ static cudaError_t launch_vc_typed(const Star7Launch& a, cudaStream_t stream) {
     const Layout& L = a.L;
     if ((FS && a.tm_f == nullptr) || a.tm_c0 == nullptr || a.tm_ca == nullptr) return cudaErrorInvalidValue;
     auto kern = star7_vc_tma<P, SRC, BORDER, BY, R, NS>;
-    static bool attr = false;
-    if (!attr) {
+    static PerDevice attr;
+    attr.get(device(), [&] {
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::SMEM);
         cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-        attr = true;
-    }
+        return 1;
+    });
     T gval;
     to_elem(a.gconst, gval);
     const int zchunk = choose_zchunk(L, BY);
