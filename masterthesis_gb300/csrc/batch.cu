@@ -39,6 +39,11 @@ namespace {
 
 constexpr int kZChunk = 32;  // planes per work item
 constexpr long long kMarchNodes = 4000000;  // FP32 and pairs: larger ensembles take the persistent kernel
+// Its tile there: {16,4}, for pairs {16,2} while too few items of 16 rows fill
+// the SMs.  us per step, tiles {16,2} / {16,4}: pairs 4.1 M nodes 46.4 / 56.6,
+// 5.9 M 47.4 / 57.3, 7.6 M 60.4 / 58.8, 11.3 M 83.1 / 76.9; FP32 4.1 M 25.9 /
+// 23.6, 11.3 M 40.8 / 37.6.
+constexpr long long kWideTileNodes = 7000000;
 constexpr int kSideStreams = 16;  // parallel launch chains of a depth-2 step
 
 struct BatchInst {
@@ -657,13 +662,14 @@ extern "C" int scafes_batch_create(const scafes_batch_instance* in, int n_inst, 
         most = std::max(most, n);
     }
     const bool f64 = precision == SCAFES_PREC_F64;
-    b->tile = f64 || nodes <= kMarchNodes ? STAR7_MARCH : 3;
+    const int persistent = f64 ? 0 : precision == SCAFES_PREC_F32X2 && nodes < kWideTileNodes ? 1 : 3;
+    b->tile = f64 || nodes <= kMarchNodes ? STAR7_MARCH : persistent;
     build_march_items(b);
     // The steps by plain loads number an instance's nodes, and the items, in
     // 32 bits.
     if (most >= (1LL << 31) || b->hmarch.size() >= (1ull << 31)) {
         b->hmarch.clear();
-        if (b->tile == STAR7_MARCH) b->tile = f64 ? 0 : 3;
+        if (b->tile == STAR7_MARCH) b->tile = persistent;
     }
     std::vector<NodeOrder> order;
     for (const BatchInst& I : b->hinst) order.push_back(make_node_order(I.L.nx, I.L.ny, I.L.nz, 1));

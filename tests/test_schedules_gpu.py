@@ -47,3 +47,31 @@ def test_autotune_keeps_one_launch_per_step_of_a_set_tile(gpu):
         p.autotune(5)
         p.step(8)
         assert p.last_step_launches() in (4, 8)
+
+
+@pytest.mark.parametrize("prec", ["f32", "f32x2"])
+@pytest.mark.parametrize("instances,side", [(5, 94), (8, 90), (13, 95)])
+def test_default_ensemble_schedule_is_near_the_best(gpu, prec, instances, side):
+    M = gpu
+    rng = np.random.default_rng(instances)
+    n = (side + 3, side, side - 3)
+    shape = (n[2], n[1], n[0])
+    tau = 0.3 / sum((m - 1) ** 2 for m in n)
+    with M.Batch([M.batch_instance(n, tau, 0.5, 1.0, 1e-3, 37.0)] * instances, prec) as b:
+        for i in range(instances):
+            b.upload(i, M.FIELD_F_A, rng.uniform(0.0, 10.0, shape))
+            b.upload(i, M.FIELD_U, 37.0 + rng.uniform(0.0, 1.0, shape))
+
+        def best():
+            ms = []
+            for _ in range(4):
+                b.step(30)
+                ms.append(b.last_ms())
+            return min(ms)
+
+        default = best()
+        persistent = []
+        for tile in (1, 2, 3, 4):
+            b.set_schedule(tile)
+            persistent.append(best())
+    assert default <= 1.12 * min(persistent)
