@@ -43,23 +43,38 @@ int star7_box_height(int tile) {
 
 // Measured in us per step (cubes unless given):
 //   FP64: the march (star7_march.cuh) at every size;
-//   rule tables, several border layers: the march, whose border rules run in
-//     full warps (256^3 with a rule table: f64 226 against 500 with the best
-//     tile, f32 85 / 369, pairs 144 / 586);
-//   pairs: with a source the {32,4} tile (201 x 181 x 163: 40.5, {8,1} 41.9;
-//     300 x 280 x 260: 104.7, {16,4} 108.5), without one the {16,4} tile
-//     (256^3: 64.7, {32,4} 81.2);
+//   rule tables: the march, whose border rules run in full warps (256^3 with a
+//     rule table: f64 226 against 500 with the best tile, f32 85 / 369, pairs
+//     144 / 586);
+//   pairs with a source affine in time: the march, in whose registers its
+//     second field costs no staging (64^3 4.5 against 5.2 with the best tile,
+//     130^3 14.5 / 22.3, 201 x 181 x 163 44 / 52, 300 x 280 x 260 146 / 157);
+//   pairs with a static source: the {16,2} tile (130^3 17.9, {32,4} 20.0; 201
+//     x 181 x 163 37.9 / 39.2; 250 x 240 x 230 68.1 / 73.1) up to 256 x 256
+//     columns, then {32,4} (300 x 280 x 260: 105.4 against 107.4; {16,4} 105.3,
+//     with a mirror border 109.5 against 106.7);
+//   pairs without a source: the {16,4} tile (256^3: 64.7, {32,4} 81.2);
 //   FP32: the {16,4} tile (400^3 89 - 94, {32,4} 94 - 95, {8,1} 154; with
 //     node coefficients 256^3 88, {32,4} 95, the march 96; 448^3 345, 354, 439);
 //   FP32 and pairs below 128 x 128 columns: the {8,1} tile, which has the
-//     most CTAs (several steps of these grids run as a one-launch loop).
+//     most CTAs (several steps of these grids run as a one-launch loop);
+//   several border layers (Dirichlet): one tile is built for them.  FP32 takes
+//     it from 128 x 128 columns on (march / tile: 112^3 7.9 / 7.5, 130^3 10.2 /
+//     9.5, 160^3 13.5 / 11.6, 250 x 240 x 230 38.5 / 31.2), pairs from 8 M nodes
+//     on (201 x 181 x 163 28.9 / 33.1, with a source 36.9 / 39.0; 224^3 50.7 /
+//     49.1 and 62.1 / 57.8, 300 x 280 x 260 95.5 / 93.0 and 116 / 110); with a
+//     source affine in time the march stays (FP32 201 x 181 x 163 25.7 / 28.3,
+//     300 x 280 x 260 80.8 / 85.0).
 int star7_default_tile(const Star7Launch& a) {
-    // The march numbers nodes in 32 bits.
-    const bool march = (long long)a.L.nx * a.L.ny * a.L.nz < (1LL << 31);
-    if (march && (a.precision == SCAFES_PREC_F64 || a.L.nl != 1 || a.border == SCAFES_BORDER_TABLE))
+    const long long cols = (long long)a.L.nx * a.L.ny, nodes = cols * a.L.nz;
+    const bool pairs = a.precision == SCAFES_PREC_F32X2, small = cols < 128LL * 128LL;
+    const bool march = nodes < (1LL << 31);  // the march numbers nodes in 32 bits
+    if (march && (a.precision == SCAFES_PREC_F64 || a.border == SCAFES_BORDER_TABLE || (pairs && a.fb)))
         return STAR7_MARCH;
-    if (a.precision == SCAFES_PREC_F64 || (long long)a.L.nx * a.L.ny < 128LL * 128LL) return 0;
-    return a.precision == SCAFES_PREC_F32X2 && a.fa ? 2 : 3;
+    if (a.L.nl != 1) return march && (a.fb || (pairs ? nodes < 8000000 : small)) ? STAR7_MARCH : STAR7_MULTI_LAYER_TILE;
+    if (a.precision == SCAFES_PREC_F64 || small) return 0;
+    if (pairs && a.fa) return cols < 256LL * 256LL ? 1 : 2;
+    return 3;
 }
 
 cudaError_t launch_star7_f64(const Star7Launch& a, cudaStream_t stream);

@@ -9,11 +9,15 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-def heat(M, n, prec, tile=0, seed=1):
+def heat(M, n, prec, tile=0, seed=1, source="none", layers=1):
     rng = np.random.default_rng(seed)
     shape = (n[2], n[1], n[0])
     tau = 0.4 / (2.0 * sum((m - 1) ** 2 for m in n))
-    p = M.Plain(M.make_cfg(n, tau=tau, precision=prec, tile=tile, heat=(1.0, 1.0, 0.3)))
+    p = M.Plain(M.make_cfg(n, tau=tau, precision=prec, n_layers=layers, tile=tile, heat=(1.0, 1.0, 0.3)))
+    if source != "none":
+        p.upload(M.FIELD_F_A, rng.uniform(0.5, 1.0, shape))
+    if source == "affine":
+        p.upload(M.FIELD_F_B, rng.uniform(0.5, 1.0, shape))
     p.upload(M.FIELD_U, rng.uniform(0.5, 1.5, shape))
     return p
 
@@ -75,3 +79,17 @@ def test_default_ensemble_schedule_is_near_the_best(gpu, prec, instances, side):
             b.set_schedule(tile)
             persistent.append(best())
     assert default <= 1.12 * min(persistent)
+
+
+@pytest.mark.parametrize("prec,source,layers,n", [
+    ("f32x2", "affine", 1, (150, 140, 145)), ("f32x2", "affine", 1, (260, 258, 120)), ("f32x2", "static", 1, (140, 150, 145)),
+    ("f32x2", "static", 2, (240, 230, 220)), ("f32", "none", 2, (224, 220, 200)), ("f32", "static", 2, (150, 140, 145)),
+    ("f32", "affine", 2, (201, 181, 163)), ("f32x2", "none", 2, (130, 129, 131))])
+def test_default_sweep_is_near_the_best(gpu, prec, source, layers, n):
+    M = gpu
+    us = []
+    for tile in (0, 1, 2, 3, 4):
+        with heat(M, n, prec, tile, source=source, layers=layers) as p:
+            p.set_temporal_depth(1)
+            us.append(us_per_step(p))
+    assert us[0] <= 1.12 * min(us[1:])
