@@ -11,7 +11,7 @@
 // the border nodes are numbered separately, so a warp holds one kind and the
 // border rules (a chain of FP64 operations) run in full warps instead of in
 // one or two lanes of every warp at a face.  A step now takes 2.1, 2.7 and
-// 4.6 us on those three; of the 2.1 us of an almost empty step, most is the
+// 5.1 us on those three; of the 2.1 us of an almost empty step, most is the
 // round trips to L2 (neighbours, store and release, counter, acquire).  Two
 // warps per CTA and up to one CTA per SM: 1, 2 and 4 warps measure the same
 // within 2 %, 16 warps 20 % slower at 17 x 15 x 16.
@@ -56,11 +56,28 @@ __device__ __forceinline__ bool grid_barrier(unsigned* arrivals, unsigned target
     return __syncthreads_and(ok);
 }
 
-constexpr int LOOP_MAX_THREADS = 1024;
 constexpr uint32_t LOOP_MIN_WARPS = 2;
 
+// Registers and threads of a CTA leave room for a second loop on every SM where
+// that costs little: with 1024 threads of 44 to 64 registers the loops of
+// handles on several streams ran one after the other, each alone with its
+// barriers (12 loops at 64^3, us per step and handle: FP64 4.8, FP32 2.6,
+// pairs 3.0, where tile sweeps had taken 3.5, 1.6 and 1.8).  FP32 and pairs fit
+// 32 registers (at most 16 bytes spilled), FP64 48 (none); a loop by itself is
+// as fast (64^3 4.81 -> 4.76, 2.60 -> 2.56, 3.00 -> 2.94).  In FP64 two such CTAs fit
+// with 640 threads: 12 loops 4.8 -> 3.3, one 4.76 -> 5.05; from LOOP_FULL_NODES
+// nodes on a loop by itself needs all 1024 (80^3 7.3, 640 threads 8.0) and
+// several gain less.  Rule tables and node rules keep 64 registers: their
+// tile sweeps are slower than a loop that waits its turn (64^3 FP64 15.4, 5.6).
+template <class P, int BORDER>
+constexpr int loop_registers() {
+    if (BORDER != SCAFES_BORDER_DIRICHLET && BORDER != SCAFES_BORDER_MIRROR_POW2) return 64;
+    return std::is_same<P, PolF64>::value ? 48 : 32;
+}
+constexpr uint32_t LOOP_MAX_THREADS = 1024, LOOP_PAIR_THREADS = 640, LOOP_FULL_NODES = 320000;
+
 template <class P, int SRC, int BORDER, bool VC>
-__global__ void __launch_bounds__(LOOP_MAX_THREADS, 1)
+__global__ void __maxnreg__((loop_registers<P, BORDER>()))
 star7_loop(const __grid_constant__ LoopArgs<typename P::T> A) {
     using T = typename P::T;
     constexpr bool HAS_F = SRC != SRC_NONE;
@@ -155,7 +172,9 @@ static cudaError_t launch_loop_typed(const Star7Loop& q, cudaStream_t stream) {
     A.in_cta = (A.o.n_inner + ctas - 1) / ctas;
     A.bd_cta = (A.o.n_border + ctas - 1) / ctas;
     const uint32_t want = ((A.in_cta + 31) / 32 + (A.bd_cta + 31) / 32) * 32;
-    const uint32_t rounds = (want + LOOP_MAX_THREADS - 1) / LOOP_MAX_THREADS;
+    const bool pair = loop_registers<P, BORDER>() == 48 && A.o.n_inner < LOOP_FULL_NODES;
+    const uint32_t most = pair ? LOOP_PAIR_THREADS : LOOP_MAX_THREADS;
+    const uint32_t rounds = (want + most - 1) / most;
     const uint32_t threads = ((want / 32 + rounds - 1) / rounds) * 32;
     cudaError_t e = cudaMemsetAsync(q.arrivals, 0, sizeof(unsigned), stream);
     if (e != cudaSuccess) return e;

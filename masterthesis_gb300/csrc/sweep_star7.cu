@@ -119,22 +119,31 @@ cudaError_t launch_star7_loop_f64(const Star7Loop& q, cudaStream_t stream);
 cudaError_t launch_star7_loop_f32(const Star7Loop& q, cudaStream_t stream);
 cudaError_t launch_star7_loop_f32x2(const Star7Loop& q, cudaStream_t stream);
 
-// Largest grid whose steps run faster as a one-launch loop than as sweeps
-// (both measured, us per step, loop / default sweep):
-//   FP64, and rule tables in any type: f64 96^3 11.4 / 14.4, 201 x 181 x 163
-//     60 / 64, 256^3 161 / 148; node coefficients 96^3 12 / 16, 201 x 181 x
-//     163 75 / 78, 256^3 221 / 178; rule table 96^3 16 / 21, 201 x 181 x 163
-//     95 / 98, 256^3 270 / 226; f32 rule table 201 x 181 x 163 40 / 39, 256^3
-//     122 / 85; pairs 63 / 66, 169 / 144;
-//   FP32 and pairs: while the iterates and the source (and the coefficients)
-//     stay in the 126 MB L2, since the loop reads neighbours through L1 only:
-//     f32 201 x 181 x 163 19 / 23, 224^3 (90 MB) 35 / 34.5, with a source
-//     (135 MB) 52 / 39; pairs 201 x 181 x 163 (106 MB) 32 / 35, 224^3 (180
-//     MB) 75 / 55; f32 node coefficients 201 x 181 x 163 (122 MB) 37 / 47.
+// Largest grid whose steps run faster as a one-launch loop than as sweeps, in
+// nodes (both measured, us per step, loop / default sweep; the loop reads its
+// neighbours through L1 only and falls behind where the sweep's pipes or HBM
+// are busy, while the grid barrier is the smaller share):
+//   FP64: 96^3 10.3 / 11.1, 112^3 15.4 / 15.4, 128^3 21.0 / 20.6, 201 x 181 x
+//     163 54 / 53, with a source 69.6 / 63.4; node coefficients 128^3 23.7 /
+//     26.8, 160 x 150 x 140 43.7 / 42.7; node rules and rule tables 201 x 181 x
+//     163 63 / 69 and 70 / 74 (256^3 270 / 226);
+//   FP32: 112^3 6.3 / 7.7, 128^3 8.3 / 6.8, 160^3 13.9 / 9.8, 250 x 240 x 230
+//     53.8 / 26.2; node coefficients 112^3 6.6 / 8.2, 128^3 8.6 / 8.1; with a
+//     source affine in time 145^3 11.4 / 11.7, 160 x 150 x 140 12.5 / 11.2;
+//   pairs: 145^3 16.0 / 17.9, 160^3 20.7 / 19.1; with a source 160^3 22.9 / 24.2,
+//     180^3 no faster; with one affine in time 97^3 7.1 / 7.9, 112^3 10.5 / 10.4,
+//     130^3 15.5 / 13.8;
+//   rule tables in FP32 and pairs: 80^3 5.7 / 6.0 and 8.6 / 10.0, 96^3 7.5 / 6.4
+//     and 12.2 / 10.6;
+//   node rules in FP32 (160^3 16.7 / 30.9, 201 x 181 x 163 36 / 42): while the
+//     fields stay in the 126 MB L2.
 long long star7_loop_max_nodes(const Star7Launch& a) {
-    if (a.precision == SCAFES_PREC_F64 || a.border == SCAFES_BORDER_TABLE) return 200LL * 200 * 200;
-    const int fields = 2 + (a.fa ? 1 : 0) + (a.fb ? 1 : 0) + (a.vc ? 2 : 0);
-    return 120000000LL / (fields * (long long)element_size(a.precision));
+    const bool table = a.border == SCAFES_BORDER_TABLE, rules = a.border == SCAFES_BORDER_NODES;
+    switch (a.precision) {
+        case SCAFES_PREC_F64: return table || rules ? 8000000 : a.vc ? 3000000 : 2000000;
+        case SCAFES_PREC_F32X2: return table ? 600000 : a.fb ? 1500000 : a.fa ? 4200000 : 3200000;
+        default: return table ? 600000 : rules ? 120000000 / ((a.fa ? 5 : 4) * 4) : a.fb ? 3000000 : 1500000;
+    }
 }
 
 cudaError_t launch_star7_loop(const Star7Loop& q, cudaStream_t stream) {

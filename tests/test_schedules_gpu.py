@@ -3,6 +3,8 @@ steps run.  Times are compared between schedules of the same problem, measured
 one after the other; the margins are far below what a wrong choice costs."""
 from __future__ import annotations
 
+import time
+
 import numpy as np
 import pytest
 
@@ -93,3 +95,53 @@ def test_default_sweep_is_near_the_best(gpu, prec, source, layers, n):
             p.set_temporal_depth(1)
             us.append(us_per_step(p))
     assert us[0] <= 1.12 * min(us[1:])
+
+
+@pytest.mark.parametrize("prec,source,n", [("f32", "none", (160, 160, 160)), ("f32", "none", (250, 240, 230)),
+                                           ("f32", "static", (201, 181, 163)), ("f32x2", "affine", (130, 140, 120)),
+                                           ("f64", "static", (201, 181, 163)), ("f64", "none", (80, 80, 80))])
+def test_default_steps_are_near_the_faster_of_loop_and_sweeps(gpu, prec, source, n):
+    M = gpu
+    with heat(M, n, prec, source=source) as p:
+        default = us_per_step(p)
+        p.set_temporal_depth(1)
+        assert default <= 1.1 * us_per_step(p)
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32", "f32x2"])
+@pytest.mark.parametrize("n", [(50, 50, 50), (64, 64, 64)])
+def test_loops_of_several_handles_share_the_gpu(gpu, prec, n):
+    """Four handles on streams of their own: their loops overlap (in turn they
+    would take four times as long as one), and give the bits of loops run
+    alone."""
+    M = gpu
+    steps = 400
+    alone = []
+    seconds = [np.inf, np.inf]
+    for k in range(4):
+        with heat(M, n, prec, seed=k) as p:
+            for _ in range(3):
+                p.synchronize()
+                t0 = time.perf_counter()
+                p.step(steps)
+                p.synchronize()
+                seconds[0] = min(seconds[0], time.perf_counter() - t0)
+                assert p.last_step_launches() == 1
+            alone.append(p.download())
+    handles = [heat(M, n, prec, seed=k) for k in range(4)]
+    try:
+        for _ in range(3):
+            for p in handles:
+                p.synchronize()
+            t0 = time.perf_counter()
+            for p in handles:
+                p.step(steps)
+            for p in handles:
+                p.synchronize()
+            seconds[1] = min(seconds[1], time.perf_counter() - t0)
+        for p, want in zip(handles, alone):
+            assert np.array_equal(p.download(), want)
+    finally:
+        for p in handles:
+            p.close()
+    assert seconds[1] <= 3.2 * seconds[0]
