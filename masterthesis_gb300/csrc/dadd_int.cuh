@@ -70,7 +70,8 @@ SCAFES_HD uint64_t dadd_same_sign_bits(uint64_t a, uint64_t b, bool& ok) {
 // neighbours in fields that change sign.  The significands are aligned to the
 // larger exponent with 9 guard bits (so nothing is shifted out), added as
 // signed 64-bit numbers, and the magnitude is normalised by its leading
-// zeros and rounded half to even.  (-0) + (-0) gives +0.
+// zeros and rounded half to even.  A zero sum has the FP64 adder's sign: -0
+// only where both operands are -0.
 SCAFES_HD uint64_t dadd_bits(uint64_t a, uint64_t b, bool& ok) {
     const uint32_t ah = (uint32_t)(a >> 32), al = (uint32_t)a;
     const uint32_t bh = (uint32_t)(b >> 32), bl = (uint32_t)b;
@@ -106,7 +107,7 @@ SCAFES_HD uint64_t dadd_bits(uint64_t a, uint64_t b, bool& ok) {
     // A zero sum is right at any exponent but that of infinities and NaNs.
     ok = (e - m <= 0x00900000u || m == 0u) && (top <= 0x7bd00000u || (mag == 0u && e < 0x7ff00000u));
     const uint32_t hi = ((uint32_t)(r >> 32) + e + ((uint32_t)(1 - lz) << 20)) | ((ah ^ (uint32_t)n) & 0x80000000u);
-    return mag ? ((uint64_t)hi << 32) | (uint32_t)r : 0u;
+    return mag ? ((uint64_t)hi << 32) | (uint32_t)r : (uint64_t)(ah & bh & 0x80000000u) << 32;
 }
 
 // A constant factor prepared for dmul_bits: its significand's 53 bits at the
