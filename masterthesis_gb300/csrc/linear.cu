@@ -16,6 +16,7 @@
 // rule the identity) is neither copied nor swapped in that phase.
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -65,7 +66,7 @@ struct FieldPtrs {
 // of the Yee cavity at 96 x 81 x 73: the table in memory, read by every node,
 // 52.8, in shared memory 51, this 37.7); and a rule that starts with a field's own
 // value, weight 1 and no constant, starts from that value instead of
-// multiplying it.
+// multiplying it (as fma(1, x, +0) it would give +0 for -0, hence plus_zero).
 struct Resolved {
     const double* p;  // the source's buffer, moved by the term's offset
     double w;
@@ -90,6 +91,12 @@ struct LinArgs {
     Resolved term[SCAFES_LIN_MAX_FIELDS * SCAFES_LIN_MAX_TERMS];
 };
 
+// x + 0 on the integer pipe: x, but +0 for -0.
+__device__ __forceinline__ double plus_zero(double x) {
+    const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+    return __hiloint2double((int)(((hi ^ 0x80000000u) | lo) == 0u ? 0u : hi), (int)lo);
+}
+
 __global__ void __launch_bounds__(MARCH_THREADS) k_linear(const __grid_constant__ LinArgs A) {
     const Layout& L = A.L;
     step_wait();
@@ -104,7 +111,7 @@ __global__ void __launch_bounds__(MARCH_THREADS) k_linear(const __grid_constant_
             const LinArgs::Written& w = A.written[f];
             int k = w.first;
             double v = w.cst;
-            if (w.own) v = __ldg(A.term[k++].p + o);
+            if (w.own) v = plus_zero(__ldg(A.term[k++].p + o));
 #pragma unroll 4
             for (; k < w.end; ++k) v = fma(A.term[k].w, __ldg(A.term[k].p + o), v);
             w.out[o] = v;
@@ -394,7 +401,7 @@ extern "C" int scafes_lin_step(scafes_lin* h, int n_steps) {
                     const int first = n;
                     for (const auto& t : tl) A.term[n++] = Resolved{P.in[t.src] + L.idx(t.dx, t.dy, t.dz), t.w};
                     A.written[A.n_written++] = {P.out[f], cst, first, n,
-                                                !tl.empty() && cst == 0.0 && tl[0].w == 1.0};
+                                                !tl.empty() && cst == 0.0 && !std::signbit(cst) && tl[0].w == 1.0};
                 }
                 LTRY(h, launch_step(k_linear, dim3(inner_ctas + border_ctas), dim3(MARCH_THREADS), 0, h->stream, A));
             } else {

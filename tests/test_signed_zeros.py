@@ -1,6 +1,6 @@
 """Signs of zeros: the integer adder's (CPU, bit for bit against the host's
-FP64 adder) and one Yee step's on fields of zeros of both signs, where every
-operation is exact and numpy gives the bits."""
+FP64 adder), and those of a Yee step and of recorded linear rules on fields of
+zeros of both signs, where every operation is exact and numpy gives the bits."""
 from __future__ import annotations
 
 import subprocess
@@ -52,3 +52,26 @@ def test_yee_step_of_signed_zeros(gpu, n):
     got[2][at] = ez[at] = 0.0
     for k, want in enumerate((ex, ey, ez, hx, hy, hz)):
         assert np.array_equal(bits(got[k]), bits(want)), k
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cst", [0.0, -0.0])
+def test_linear_rules_of_signed_zeros(gpu, cst):
+    """A rule is a chain of fma from its constant on: a copy of -0 with the
+    constant +0 gives +0, with -0 it stays."""
+    M = gpu
+    n = (6, 5, 4)
+    shape = (n[2], n[1], n[0])
+    rng = np.random.default_rng(3)
+    f = [np.where(rng.random(shape) < 0.5, -0.0, 0.0) for _ in range(2)]
+    with M.Linear(n, 2) as h:
+        for cls in range(64):
+            h.set_rule(1, 0, cls, [(1, 0, 0, 0, 1.0)], cst)
+            h.set_rule(1, 1, cls, [(0, 0, 0, 0, 1.0), (1, 0, 0, 0, 0.5)], cst)
+        for i, a in enumerate(f):
+            h.upload(i, a)
+        h.step(1)
+        got = [h.download(i) for i in range(2)]
+    want = [f[1] + cst, 0.5 * f[1] + (f[0] + cst)]
+    for a, b in zip(got, want):
+        assert np.array_equal(bits(a), bits(b))
