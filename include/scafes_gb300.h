@@ -429,7 +429,9 @@ int scafes_batch_step_looped(scafes_batch* b, int n_steps);
  * schedule. */
 int scafes_batch_autotune(scafes_batch* b, int n_steps, int* tile,
                           int* ctas_per_sm);
-/* Sets the schedule directly: tile 1..4, ctas_per_sm 0 (= occupancy) .. 16. */
+/* Sets the schedule directly: tile 1..4 of the persistent kernel, or 0, the
+ * sweep by plain loads (as scafes_batch_info reports them); ctas_per_sm 0
+ * (= occupancy) .. 16, of the persistent kernel. */
 int scafes_batch_set_schedule(scafes_batch* b, int tile, int ctas_per_sm);
 /* Temporal-blocking depth of scafes_batch_step: 1 or 2 (an odd last step
  * of a depth-2 call runs at depth 1). */

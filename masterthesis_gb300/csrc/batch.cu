@@ -745,7 +745,7 @@ extern "C" int scafes_batch_step(scafes_batch* b, int n_steps) {
     int rc = ensure_counters(b, n_steps);
     if (rc) return rc;
     if (b->tile != STAR7_MARCH) grid_size(b, kinfo(b->precision, b->tile));  // sets the smem attribute outside any capture
-    // Depth 2: n_steps / 2 passes, an odd last step by the persistent kernel.
+    // Depth 2: n_steps / 2 passes, an odd last step by the depth-1 schedule.
     const int pairs = b->depth == 2 ? n_steps / 2 : 0;
     const int singles = n_steps - 2 * pairs;
     if (pairs > 0) {
@@ -940,9 +940,11 @@ extern "C" int scafes_batch_autotune(scafes_batch* b, int n_steps, int* tile_out
 
 extern "C" int scafes_batch_set_schedule(scafes_batch* b, int tile, int ctas_per_sm) {
     if (!b) return bfail(nullptr, SCAFES_ERR_ARG, "scafes_batch_set_schedule: batch is NULL");
-    if (tile < 1 || tile > STAR7_NUM_TILES || ctas_per_sm < 0 || ctas_per_sm > 16)
+    // 0 as scafes_batch_info reports it: the step by plain loads, where the
+    // instances' node numbers allow it.
+    if (tile < (b->hmarch.empty() ? 1 : 0) || tile > STAR7_NUM_TILES || ctas_per_sm < 0 || ctas_per_sm > 16)
         return bfail(b, SCAFES_ERR_ARG, "scafes_batch_set_schedule: tile %d / ctas %d out of range", tile, ctas_per_sm);
-    b->tile = tile - 1;
+    b->tile = tile == 0 ? STAR7_MARCH : tile - 1;
     b->ctas_per_sm = ctas_per_sm;
     return SCAFES_OK;
 }

@@ -145,3 +145,32 @@ def test_loops_of_several_handles_share_the_gpu(gpu, prec, n):
         for p in handles:
             p.close()
     assert seconds[1] <= 3.2 * seconds[0]
+
+
+@pytest.mark.parametrize("prec,side", [("f64", 20), ("f32", 20), ("f32", 170)])
+def test_a_reported_ensemble_schedule_can_be_set_again(gpu, prec, side):
+    M = gpu
+    n = (side, side, side)
+    tau = 0.3 / (3.0 * (side - 1) ** 2)
+    u0 = np.random.default_rng(side).uniform(37.0, 38.0, n)
+    got = []
+    for again in (False, True):
+        with M.Batch([M.batch_instance(n, tau, 0.5, 1.0, 0.0, 37.0)], prec) as b:
+            b.upload(0, M.FIELD_U, u0)
+            b.step(2)
+            info = b.info()
+            if again:
+                b.set_schedule(2)
+                b.step(2)
+                b.set_schedule(info["tile"], info["ctas_per_sm"])
+                assert {k: b.info()[k] for k in ("tile", "ctas_per_sm", "items")} == \
+                    {k: info[k] for k in ("tile", "ctas_per_sm", "items")}
+                b.step(2)
+            else:
+                b.step(4)
+            got.append(b.download(0))
+    assert np.array_equal(got[0], got[1])
+    with M.Batch([M.batch_instance(n, tau, 0.5, 1.0, 0.0, 37.0)], prec) as b:
+        for tile in (-1, 5):
+            with pytest.raises(M.ScafesError):
+                b.set_schedule(tile)
