@@ -96,9 +96,10 @@ constexpr int MARCH_THREADS = 256;
 // FP64 pays for every warp whatever its active lanes, and 32 columns at a
 // time leave up to a quarter of them idle (98 inner columns: 98 of 128), so
 // the width follows the grid: the (w, h) with the fewest idle threads, w
-// at most 64 and at
-// least 16 where the grid has them, h at most 16 (sectors; rows that share
-// their y neighbours in L1; the halos that callers keep in shared memory).
+// at most 64 and at least 16 where the grid has them, h at most 16 (sectors;
+// rows that share their y neighbours in L1; the halos that callers keep in
+// shared memory).  Launches call it, so the search is over the 49 widths,
+// whatever the grid's.
 struct ColumnTile {
     FastDiv w;
     int h, nx, ny;  // rows of threads; tiles along x and y
@@ -106,11 +107,16 @@ struct ColumnTile {
 inline ColumnTile make_column_tile(int ix, int iy, int rows) {
     ColumnTile t;
     t.h = t.nx = t.ny = 0;
+    if (ix <= 0 || iy <= 0) return t;
     long long best = 0;
     const int ty = (iy + rows - 1) / rows;  // rows of threads
-    for (int n = (ix + 63) / 64; n <= (ix + 15) / 16 || n == (ix + 63) / 64; ++n) {
-        if (n == 0) break;
-        const int w = (ix + n - 1) / n, h = MARCH_THREADS / w < 16 ? MARCH_THREADS / w : 16, m = (ty + h - 1) / h;
+    const int least = ix < 16 ? ix : 16;
+    int last = 0;
+    for (int k = ix < 64 ? ix : 64; k >= least; --k) {
+        const int n = (ix + k - 1) / k, w = (ix + n - 1) / n;
+        if (n == last || w < least) continue;
+        last = n;
+        const int h = MARCH_THREADS / w < 16 ? MARCH_THREADS / w : 16, m = (ty + h - 1) / h;
         const long long threads = (long long)n * m * MARCH_THREADS;
         if (t.h == 0 || threads < best || (threads == best && h > t.h)) {
             best = threads;
