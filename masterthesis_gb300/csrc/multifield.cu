@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(MARCH_THREADS, 3) k_lame_march(const __grid_co
     const Layout& L = A.L;
     step_wait();
     if (blockIdx.x < A.border_ctas) {
-        const uint32_t m = blockIdx.x * MARCH_THREADS + threadIdx.x;
+        const uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
         if (m >= A.o.n_border) return;
         int x, y, z;
         border_node(A.o, m, x, y, z);
@@ -1177,7 +1177,7 @@ extern "C" int scafes_mf_step(scafes_mf* h, int n_steps) {
             if (rc) return rc;
         }
         LameMarch F{};
-        unsigned lame_ctas = 0;
+        unsigned lame_ctas = 0, lame_threads = 0;
         if (!x2 && (long long)L.nx * L.ny * L.nz <= kMaxNumbered) {
             F.comp = comp;
             memcpy(F.a, K.a, sizeof(F.a));
@@ -1188,13 +1188,20 @@ extern "C" int scafes_mf_step(scafes_mf* h, int n_steps) {
             F.ct = make_column_tile(L.nx - 2, L.ny - 2, 1);
             F.tx = make_fastdiv((uint32_t)F.ct.nx);
             F.txy = make_fastdiv((uint32_t)(F.ct.nx * F.ct.ny));
-            F.border_ctas = (F.o.n_border + MARCH_THREADS - 1) / MARCH_THREADS;
             // 8 planes per CTA, fewer while that leaves under two rounds of
             // resident CTAs (us per step at 129 x 111 x 101 with 4, 6, 8
             // planes: 123, 119, 123).
             const long long lt = (long long)F.ct.nx * F.ct.ny, want = 2LL * 3 * sm_count();
             F.zchunk = (int)std::max(1LL, std::min(8LL, (L.nz - 2) * lt / want));
-            lame_ctas = F.border_ctas + F.ct.nx * F.ct.ny * ((L.nz - 2 + F.zchunk - 1) / F.zchunk);
+            const long long tile_ctas = lt * ((L.nz - 2 + F.zchunk - 1) / F.zchunk);
+            // Where the tiles fill the SMs, no more threads than a tile and its
+            // halo need, since all do the arithmetic (4 x 5 x 60000 859 -> 286 us
+            // a step, 5 x 30000 x 4 86 -> 44); else all, for the border nodes
+            // (6 x 9 x 14 5.5, with 32 threads 5.9).
+            const int cols = (int)F.ct.w.d, rows = F.ct.h;
+            lame_threads = tile_ctas < want / 2 ? MARCH_THREADS : (std::max(cols * rows, 2 * (cols + rows)) + 31) / 32 * 32;
+            F.border_ctas = (F.o.n_border + lame_threads - 1) / lame_threads;
+            lame_ctas = (unsigned)(F.border_ctas + tile_ctas);
         }
         const int lzc = lame_zchunk(L);
         const dim3 lgrid((L.nx + LX - 1) / LX, (L.ny + LY - 1) / LY, (L.nz + lzc - 1) / lzc);
@@ -1209,7 +1216,7 @@ extern "C" int scafes_mf_step(scafes_mf* h, int n_steps) {
                 F.u = (const double*)u;
                 F.up = (double*)up;
                 if (lame_ctas)
-                    MTRY(h, launch_step(k_lame_march, dim3(lame_ctas), dim3(MARCH_THREADS), 0, h->stream, F));
+                    MTRY(h, launch_step(k_lame_march, dim3(lame_ctas), dim3(lame_threads), 0, h->stream, F));
                 else k_lame<<<mgrid(L), dim3(MX, MY), 0, h->stream>>>((const double*)u, (double*)up, K, L, comp);
             }
             MTRY(h, cudaGetLastError());
