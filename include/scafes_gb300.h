@@ -700,11 +700,14 @@ int scafes_probe_dadd_int(const unsigned long long* a, const unsigned long long*
  * runs the bounded device wait of the sweep kernels on an mbarrier that
  * never completes, with a limit of limit_us (1 .. 1e6): *status receives
  * the status the kernel recorded (SCAFES_ERR_TIMEOUT) and *waited_ms the
- * time it waited.  scafes_gpu_inject_status writes `code` (<= 0) into a
+ * time it waited; _grid_barrier_timeout the same for the barrier of the
+ * one-launch time loop, with a CTA that never arrives.
+ * scafes_gpu_inject_status writes `code` (<= 0) into a
  * handle's device status word, as a sweep that gave up does: later sweeps
  * of the handle skip their work and the next download reports the status
  * (and clears it). */
 int scafes_probe_wait_timeout(unsigned limit_us, int* status, double* waited_ms);
+int scafes_probe_grid_barrier_timeout(unsigned limit_us, int* status, double* waited_ms);
 int scafes_gpu_inject_status(scafes_handle* h, int code);
 /* The same for an adjoint handle: its FP32-pair forward and adjoint steps
  * skip their work while the word is set, and the next scafes_adj_forward /

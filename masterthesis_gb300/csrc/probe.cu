@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "dadd_int.cuh"
+#include "grid_barrier.cuh"
 #include "tma.cuh"
 #include "../../include/scafes_gb300.h"
 
@@ -53,6 +54,15 @@ __global__ void k_wait_probe(unsigned long long limit_ns, int* status, unsigned 
     }
 }
 
+// The same for the barrier of the one-launch time loop: one CTA at a barrier
+// that expects two.
+__global__ void k_grid_barrier_probe(unsigned long long limit_ns, unsigned* arrivals, int* status,
+                                     unsigned long long* waited_ns) {
+    const unsigned long long t0 = scafes::global_timer_ns();
+    if (!scafes::grid_barrier(arrivals, 2u, status, limit_ns) && threadIdx.x == 0)
+        *waited_ns = scafes::global_timer_ns() - t0;
+}
+
 // The integer-pipe addition of the FP64 sweep, element by element.
 __global__ void k_dadd_int(const uint64_t* a, const uint64_t* b, uint64_t* sum, unsigned char* ok, long long n) {
     const long long stride = (long long)gridDim.x * blockDim.x;
@@ -89,6 +99,29 @@ extern "C" int scafes_probe_dadd_int(const unsigned long long* a, const unsigned
     return e == cudaSuccess ? SCAFES_OK : SCAFES_ERR_CUDA;
 }
 
+// Runs `launch(status, waited_ns, zero)` (device words, all zero) and reads
+// the status and the time waited back; synchronises the device.
+template <class Launch>
+static int probe_timeout(int* status, double* waited_ms, const Launch& launch) {
+    unsigned long long* d = nullptr;  // time waited, status, a counter
+    if (cudaMalloc(&d, 3 * sizeof(*d)) != cudaSuccess) return SCAFES_ERR_CUDA;
+    int st = 0;
+    unsigned long long w = 0;
+    cudaError_t e = cudaMemset(d, 0, 3 * sizeof(*d));
+    if (e == cudaSuccess) {
+        launch(reinterpret_cast<int*>(d + 1), d, reinterpret_cast<unsigned*>(d + 2));
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (e == cudaSuccess) e = cudaMemcpy(&st, d + 1, sizeof(int), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(&w, d, sizeof(w), cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    if (e != cudaSuccess) return SCAFES_ERR_CUDA;
+    *status = st;
+    *waited_ms = (double)w * 1e-6;
+    return SCAFES_OK;
+}
+
 // No counterpart in the reference: exercises the timeout path of the
 // bounded device waits without any fault (no load is ever issued; the
 // barrier simply never completes).  limit_us in [1, 1e6].  Writes the
@@ -96,30 +129,17 @@ extern "C" int scafes_probe_dadd_int(const unsigned long long* a, const unsigned
 // waited; synchronises the device.
 extern "C" int scafes_probe_wait_timeout(unsigned limit_us, int* status, double* waited_ms) {
     if (!status || !waited_ms || limit_us < 1 || limit_us > 1000000) return SCAFES_ERR_ARG;
-    int* d_status = nullptr;
-    unsigned long long* d_waited = nullptr;
-    if (cudaMalloc(&d_status, sizeof(int)) != cudaSuccess) return SCAFES_ERR_CUDA;
-    if (cudaMalloc(&d_waited, sizeof(unsigned long long)) != cudaSuccess) {
-        cudaFree(d_status);
-        return SCAFES_ERR_CUDA;
-    }
-    int st = 0;
-    unsigned long long w = 0;
-    cudaError_t e = cudaMemset(d_status, 0, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(d_waited, 0, sizeof(unsigned long long));
-    if (e == cudaSuccess) {
-        k_wait_probe<<<1, 64>>>((unsigned long long)limit_us * 1000ull, d_status, d_waited);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    if (e == cudaSuccess) e = cudaMemcpy(&st, d_status, sizeof(int), cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess) e = cudaMemcpy(&w, d_waited, sizeof(w), cudaMemcpyDeviceToHost);
-    cudaFree(d_status);
-    cudaFree(d_waited);
-    if (e != cudaSuccess) return SCAFES_ERR_CUDA;
-    *status = st;
-    *waited_ms = (double)w * 1e-6;
-    return SCAFES_OK;
+    return probe_timeout(status, waited_ms, [&](int* st, unsigned long long* waited, unsigned*) {
+        k_wait_probe<<<1, 64>>>((unsigned long long)limit_us * 1000ull, st, waited);
+    });
+}
+
+// The same for the grid barrier of the one-launch time loop.
+extern "C" int scafes_probe_grid_barrier_timeout(unsigned limit_us, int* status, double* waited_ms) {
+    if (!status || !waited_ms || limit_us < 1 || limit_us > 1000000) return SCAFES_ERR_ARG;
+    return probe_timeout(status, waited_ms, [&](int* st, unsigned long long* waited, unsigned* arrivals) {
+        k_grid_barrier_probe<<<1, 64>>>((unsigned long long)limit_us * 1000ull, arrivals, st, waited);
+    });
 }
 
 // No counterpart in the reference: a measurement utility for the roofline.
