@@ -41,9 +41,10 @@ constexpr int kZChunk = 32;  // planes per work item
 constexpr long long kMarchNodes = 4000000;  // FP32 and pairs: larger ensembles take the persistent kernel
 // Its tile there: {16,4}, for pairs {16,2} while too few items of 16 rows fill
 // the SMs.  us per step, tiles {16,2} / {16,4}: pairs 4.1 M nodes 46.4 / 56.6,
-// 5.9 M 47.4 / 57.3, 7.6 M 60.4 / 58.8, 11.3 M 83.1 / 76.9; FP32 4.1 M 25.9 /
-// 23.6, 11.3 M 40.8 / 37.6.
-constexpr long long kWideTileNodes = 7000000;
+// 5.9 M 47.4 / 57.3, 7.3 M in equal instances 47.8 / 58.0, 7.6 M in uneven
+// ones 60.4 / 58.8, 11.3 M 83.1 / 76.9; FP32 4.1 M 25.9 / 23.6, 11.3 M 40.8 /
+// 37.6.
+constexpr long long kWideTileNodes = 8500000;
 constexpr int kSideStreams = 16;  // parallel launch chains of a depth-2 step
 
 struct BatchInst {

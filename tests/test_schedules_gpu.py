@@ -1,6 +1,8 @@
 """What the schedules choose on the GPU: the autotuner's choice is what later
-steps run.  Times are compared between schedules of the same problem, measured
-one after the other; the margins are far below what a wrong choice costs."""
+steps run, the defaults are near the best schedule, loops of several handles
+overlap.  Times are compared between schedules of the same problem, measured
+one after the other, best of several; the margins are far below what a wrong
+choice costs, and a comparison that a disturbance spoils is made again."""
 from __future__ import annotations
 
 import time
@@ -34,17 +36,30 @@ def us_per_step(p, steps=60):
     return 1e3 * best / steps
 
 
+def assert_no_slower(margin, measure, tries=4):
+    """measure() -> (time, time of what it is compared with)."""
+    for _ in range(tries):
+        t, reference = measure()
+        if t <= margin * reference:
+            return
+    assert t <= margin * reference
+
+
 @pytest.mark.parametrize("prec", ["f64", "f32", "f32x2"])
 @pytest.mark.parametrize("n", [(17, 15, 16), (64, 48, 40), (160, 160, 160)])
 def test_autotuned_steps_run_what_was_fastest(gpu, prec, n):
     M = gpu
     with heat(M, n, prec) as p:
-        for _ in range(2):  # a second call chooses anew
+
+        def measure():  # a second call chooses anew
             _, ms = p.autotune(20)
             t = us_per_step(p)
-            assert t <= 1.15 * 1e3 * min(ms)
             launches = p.last_step_launches()
             assert launches == 30 if p.temporal_depth == 2 else launches in (1, 60)
+            return t, 1e3 * min(ms)
+
+        assert_no_slower(1.15, measure)
+        assert_no_slower(1.15, measure)
 
 
 def test_autotune_keeps_one_launch_per_step_of_a_set_tile(gpu):
@@ -55,32 +70,29 @@ def test_autotune_keeps_one_launch_per_step_of_a_set_tile(gpu):
         assert p.last_step_launches() in (4, 8)
 
 
-@pytest.mark.parametrize("prec", ["f32", "f32x2"])
-@pytest.mark.parametrize("instances,side", [(5, 94), (8, 90), (13, 95)])
-def test_default_ensemble_schedule_is_near_the_best(gpu, prec, instances, side):
+@pytest.mark.parametrize("instances,side", [(5, 94), (8, 90), (10, 90), (13, 95)])
+def test_default_pair_ensemble_schedule_is_near_the_best(gpu, instances, side):
     M = gpu
     rng = np.random.default_rng(instances)
     n = (side + 3, side, side - 3)
     shape = (n[2], n[1], n[0])
     tau = 0.3 / sum((m - 1) ** 2 for m in n)
-    with M.Batch([M.batch_instance(n, tau, 0.5, 1.0, 1e-3, 37.0)] * instances, prec) as b:
+    with M.Batch([M.batch_instance(n, tau, 0.5, 1.0, 1e-3, 37.0)] * instances, "f32x2") as b:
         for i in range(instances):
             b.upload(i, M.FIELD_F_A, rng.uniform(0.0, 10.0, shape))
             b.upload(i, M.FIELD_U, 37.0 + rng.uniform(0.0, 1.0, shape))
 
-        def best():
+        def best(tile):
+            if tile is not None:
+                b.set_schedule(tile)
             ms = []
             for _ in range(4):
                 b.step(30)
                 ms.append(b.last_ms())
             return min(ms)
 
-        default = best()
-        persistent = []
-        for tile in (1, 2, 3, 4):
-            b.set_schedule(tile)
-            persistent.append(best())
-    assert default <= 1.12 * min(persistent)
+        chosen = b.info()["tile"]
+        assert_no_slower(1.12, lambda: (best(chosen), min(best(tile) for tile in (1, 2, 3, 4))))
 
 
 @pytest.mark.parametrize("prec,source,layers,n", [
@@ -89,12 +101,16 @@ def test_default_ensemble_schedule_is_near_the_best(gpu, prec, instances, side):
     ("f32", "affine", 2, (201, 181, 163)), ("f32x2", "none", 2, (130, 129, 131))])
 def test_default_sweep_is_near_the_best(gpu, prec, source, layers, n):
     M = gpu
-    us = []
-    for tile in (0, 1, 2, 3, 4):
-        with heat(M, n, prec, tile, source=source, layers=layers) as p:
-            p.set_temporal_depth(1)
-            us.append(us_per_step(p))
-    assert us[0] <= 1.12 * min(us[1:])
+
+    def measure():
+        us = []
+        for tile in (0, 1, 2, 3, 4):
+            with heat(M, n, prec, tile, source=source, layers=layers) as p:
+                p.set_temporal_depth(1)
+                us.append(us_per_step(p))
+        return us[0], min(us[1:])
+
+    assert_no_slower(1.12, measure)
 
 
 @pytest.mark.parametrize("prec,source,n", [("f32", "none", (160, 160, 160)), ("f32", "none", (250, 240, 230)),
@@ -102,10 +118,14 @@ def test_default_sweep_is_near_the_best(gpu, prec, source, layers, n):
                                            ("f64", "static", (201, 181, 163)), ("f64", "none", (80, 80, 80))])
 def test_default_steps_are_near_the_faster_of_loop_and_sweeps(gpu, prec, source, n):
     M = gpu
-    with heat(M, n, prec, source=source) as p:
-        default = us_per_step(p)
-        p.set_temporal_depth(1)
-        assert default <= 1.1 * us_per_step(p)
+
+    def measure():
+        with heat(M, n, prec, source=source) as p:
+            default = us_per_step(p)
+            p.set_temporal_depth(1)
+            return default, us_per_step(p)
+
+    assert_no_slower(1.1, measure)
 
 
 @pytest.mark.parametrize("prec", ["f64", "f32", "f32x2"])
@@ -116,35 +136,36 @@ def test_loops_of_several_handles_share_the_gpu(gpu, prec, n):
     alone."""
     M = gpu
     steps = 400
-    alone = []
-    seconds = [np.inf, np.inf]
-    for k in range(4):
-        with heat(M, n, prec, seed=k) as p:
-            for _ in range(3):
-                p.synchronize()
-                t0 = time.perf_counter()
-                p.step(steps)
-                p.synchronize()
-                seconds[0] = min(seconds[0], time.perf_counter() - t0)
-                assert p.last_step_launches() == 1
-            alone.append(p.download())
     handles = [heat(M, n, prec, seed=k) for k in range(4)]
-    try:
+
+    def seconds(some):
+        best = np.inf
         for _ in range(3):
-            for p in handles:
+            for p in some:
                 p.synchronize()
             t0 = time.perf_counter()
-            for p in handles:
+            for p in some:
                 p.step(steps)
-            for p in handles:
+            for p in some:
                 p.synchronize()
-            seconds[1] = min(seconds[1], time.perf_counter() - t0)
+            best = min(best, time.perf_counter() - t0)
+        return best
+
+    try:
+        alone = []
+        for k in range(4):
+            with heat(M, n, prec, seed=k) as p:
+                p.step(steps)
+                assert p.last_step_launches() == 1
+                alone.append(p.download())
+        for p in handles:
+            p.step(steps)
         for p, want in zip(handles, alone):
             assert np.array_equal(p.download(), want)
+        assert_no_slower(3.2, lambda: (seconds(handles), seconds(handles[:1])))
     finally:
         for p in handles:
             p.close()
-    assert seconds[1] <= 3.2 * seconds[0]
 
 
 @pytest.mark.parametrize("prec,side", [("f64", 20), ("f32", 20), ("f32", 170)])
