@@ -75,6 +75,7 @@ SCAFES_HD uint64_t dadd_same_sign_bits(uint64_t a, uint64_t b, bool& ok) {
 SCAFES_HD uint64_t dadd_bits(uint64_t a, uint64_t b, bool& ok) {
     const uint32_t ah = (uint32_t)(a >> 32), al = (uint32_t)a;
     const uint32_t bh = (uint32_t)(b >> 32), bl = (uint32_t)b;
+    const uint32_t z0 = ah & bh & 0x80000000u;  // the high word of a zero sum
     const uint32_t ta = ah & 0x7ff00000u, tb = bh & 0x7ff00000u;
     const uint32_t e = ta > tb ? ta : tb, m = ta > tb ? tb : ta;
     const uint32_t sa = (e - ta) >> 20, sb = (e - tb) >> 20;
@@ -107,10 +108,11 @@ SCAFES_HD uint64_t dadd_bits(uint64_t a, uint64_t b, bool& ok) {
     // A zero sum is right at any exponent but that of infinities and NaNs.
     ok = (e - m <= 0x00900000u || m == 0u) && (top <= 0x7bd00000u || (mag == 0u && e < 0x7ff00000u));
     const uint32_t hi = ((uint32_t)(r >> 32) + e + ((uint32_t)(1 - lz) << 20)) | ((ah ^ (uint32_t)n) & 0x80000000u);
-    // The low word of a zero sum is zero already.  Selecting the high word alone
-    // keeps the sign in few registers: a Yee step at 128 x 120 x 113 takes 62.6
-    // us, 61.7 with the sign dropped, 66.3 selecting both words (spills).
-    return ((uint64_t)(mag ? hi : ah & bh & 0x80000000u) << 32) | (uint32_t)r;
+    // The low word of a zero sum is zero already.  Where the sign is formed
+    // decides what the compiler spills: a Yee step at 128 x 120 x 113 takes 62.5
+    // us with it formed first, 63.0 formed here, 66 with both words selected,
+    // and 62.1 with the sign dropped.
+    return ((uint64_t)(mag ? hi : z0) << 32) | (uint32_t)r;
 }
 
 // A constant factor prepared for dmul_bits: its significand's 53 bits at the
