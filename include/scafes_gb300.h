@@ -184,7 +184,8 @@ typedef struct scafes_cfg {
                                 scafes_gpu_autotune), 0 = the default
                                 schedule: one-launch loops on small grids, a
                                 sweep by plain loads for FP64, rule tables
-                                and border layers, a tile for the others */
+                                and pairs with F_B, a tile or that sweep for
+                                several border layers, a tile for the others */
     double c0;               /* centre coefficient */
     double cp[3];            /* pair coefficient per axis */
     double cf;               /* source coefficient (0 disables F) */

@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 namespace scafes {
 
 // Row pitch (in elements) of every device field: rows start on 256-byte
@@ -61,6 +63,17 @@ __host__ __device__ inline f2 split_double(double x) {
     float hi = (float)x;
     float lo = (float)(x - (double)hi);
     return {hi, lo};
+}
+
+// A double as an element of type T (host side).
+template <class T>
+T elem_of(double x) {
+    if constexpr (std::is_same<T, float2>::value) {
+        const f2 p = split_double(x);
+        return make_float2(p.hi, p.lo);
+    } else {
+        return (T)x;
+    }
 }
 
 __host__ __device__ inline double join_pair(float hi, float lo) {

@@ -99,16 +99,6 @@ star7_loop(const __grid_constant__ LoopArgs<typename P::T> A) {
 
 // ---- host side ---------------------------------------------------------------
 
-template <class T>
-static T loop_elem(double d) {
-    if constexpr (std::is_same<T, float2>::value) {
-        const f2 p = split_double(d);
-        return make_float2(p.hi, p.lo);
-    } else {
-        return (T)d;
-    }
-}
-
 template <class P, int SRC, int BORDER, bool VC>
 static cudaError_t launch_loop_typed(const Star7Loop& q, cudaStream_t stream) {
     using T = typename P::T;
@@ -122,7 +112,7 @@ static cudaError_t launch_loop_typed(const Star7Loop& q, cudaStream_t stream) {
     A.fb = (const T*)a.fb;
     A.ga = (const T*)a.ga;
     A.gb = (const T*)a.gb;
-    A.gval = loop_elem<T>(a.gconst);
+    A.gval = elem_of<T>(a.gconst);
     A.c0 = (const T*)a.c0;
     A.ca = (const T*)a.ca;
     A.L = a.L;

@@ -20,7 +20,8 @@
 // measured 2 % to 0.2 % slower.
 // FP32 and pairs are bound by the memory path, where the tile engine's ring
 // keeps more bytes in flight (f32 400^3 89 against 123 us); they come here
-// with rule tables and several border layers only.
+// with rule tables, pairs with a source affine in time, and some grids with
+// several border layers (star7_default_tile).
 #pragma once
 
 #include <algorithm>
@@ -183,16 +184,6 @@ star7_march(const __grid_constant__ MarchArgs<typename P::T> A) {
 
 // ---- host side ---------------------------------------------------------------
 
-template <class T>
-static T march_elem(double d) {
-    if constexpr (std::is_same<T, float2>::value) {
-        const f2 p = split_double(d);
-        return make_float2(p.hi, p.lo);
-    } else {
-        return (T)d;
-    }
-}
-
 // Rows per thread and resident CTAs: pairs work on two rows at once (the
 // paired FP32 instructions), the others on one.
 template <class P>
@@ -217,7 +208,7 @@ static cudaError_t launch_march_typed(const Star7Launch& a, cudaStream_t stream)
     A.fb = (const T*)a.fb;
     A.ga = (const T*)a.ga;
     A.gb = (const T*)a.gb;
-    A.gval = march_elem<T>(a.gconst);
+    A.gval = elem_of<T>(a.gconst);
     A.c0 = (const T*)a.c0;
     A.ca = (const T*)a.ca;
     A.L = a.L;

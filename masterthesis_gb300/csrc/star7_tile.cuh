@@ -143,7 +143,8 @@ __device__ __forceinline__ typename P::T table_rule_value(const TileJob<typename
     }
     // G(t) = G_A + s (G_B + s (G_C + s (G_D + s G_E))), s = (time - tc) * rate;
     // with the default basis and no higher orders (`affine`, 4 instead of 14
-    // FP64 operations, the same value) this is G_A + time * G_B.
+    // FP64 operations) this is G_A + time * G_B: the same value, up to the sign
+    // of a zero where G_A and G_B are both -0.
     const double g0 = J.ga ? P::to_double(J.ga[off]) : P::to_double(J.gval);
     const double g1 = J.gb ? P::to_double(J.gb[off]) : 0.0;
     if (B.affine) {

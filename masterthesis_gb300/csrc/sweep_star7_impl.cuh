@@ -183,14 +183,6 @@ static int choose_zchunk(const Layout& L, int by, int most = 16) {
     return zc;
 }
 
-// A double as the element type of a precision (host side).
-static inline void to_elem(double d, double& out) { out = d; }
-static inline void to_elem(double d, float& out) { out = (float)d; }
-static inline void to_elem(double d, float2& out) {
-    f2 p = split_double(d);
-    out = make_float2(p.hi, p.lo);
-}
-
 template <class P, int SRC, int BORDER, int BY, int R, int NS0, bool ML>
 static cudaError_t launch_typed(const Star7Launch& a, cudaStream_t stream) {
     using T = typename P::T;
@@ -209,8 +201,7 @@ static cudaError_t launch_typed(const Star7Launch& a, cudaStream_t stream) {
                              cudaSharedmemCarveoutMaxShared);
         return 1;
     });
-    T gval;
-    to_elem(a.gconst, gval);
+    const T gval = elem_of<T>(a.gconst);
     const int zchunk = choose_zchunk(L, BY, std::is_same<P, PolF32>::value && BY == 16 && R == 4 ? 8 : 16);
     dim3 block(BX, BY / R, 1);
     dim3 grid((L.nx + BX - 1) / BX, (L.ny + BY - 1) / BY, (L.nz + zchunk - 1) / zchunk);
@@ -259,8 +250,7 @@ static cudaError_t launch_vc_typed(const Star7Launch& a, cudaStream_t stream) {
         cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         return 1;
     });
-    T gval;
-    to_elem(a.gconst, gval);
+    const T gval = elem_of<T>(a.gconst);
     const int zchunk = choose_zchunk(L, BY);
     dim3 block(BX, BY / R, 1);
     dim3 grid((L.nx + BX - 1) / BX, (L.ny + BY - 1) / BY, (L.nz + zchunk - 1) / zchunk);
@@ -362,8 +352,7 @@ static cudaError_t launch_tb_typed(const Star7Launch& a, cudaStream_t stream) {
     auto kern = star7_tb2<P, HAS_F>;
     constexpr size_t SMEM = tb_smem(sizeof(T));
     if (const cudaError_t e = tb_attributes<P, HAS_F>()) return e;
-    T gval;
-    to_elem(a.gconst, gval);
+    const T gval = elem_of<T>(a.gconst);
     const Layout& L = a.L;
     const int zc = tb_zchunk(L);
     const dim3 grid((L.nx + TB_X - 1) / TB_X, (L.ny + TB_Y - 1) / TB_Y, (L.nz + zc - 1) / zc);
