@@ -55,26 +55,31 @@ int star7_box_height(int tile) {
 //     with a mirror border 109.5 against 106.7);
 //   pairs without a source: the {16,4} tile (256^3: 64.7, {32,4} 81.2);
 //   FP32: the {16,4} tile (400^3 89 - 94, {32,4} 94 - 95, {8,1} 154; with
-//     node coefficients 256^3 88, {32,4} 95, the march 96; 448^3 345, 354, 439);
-//   FP32 and pairs below 128 x 128 columns: the {8,1} tile, which has the
-//     most CTAs (several steps of these grids run as a one-launch loop);
+//     node coefficients 256^3 88, {32,4} 95, the march 96; 448^3 345, 354, 439),
+//     with a source affine in time {16,2} below 2 M nodes (200 x 200 x 20 5.7 /
+//     7.9, 120^3 9.2 / 9.4, 130^3 11.2 / 10.4);
+//   FP32 and pairs below 700 000 nodes: the {8,1} tile, which has the most
+//     CTAs (130 x 130 x 5 3.4, {16,4} 4.7; 80^3 4.4 / 5.2; 97^3 6.4 / 5.4; 100 x
+//     100 x 300 15.0 / 10.4; several steps of these grids run as a one-launch
+//     loop);
 //   several border layers (Dirichlet): one tile is built for them.  FP32 takes
-//     it from 128 x 128 columns on (march / tile: 112^3 7.9 / 7.5, 130^3 10.2 /
-//     9.5, 160^3 13.5 / 11.6, 250 x 240 x 230 38.5 / 31.2), pairs from 8 M nodes
+//     it from 1.2 M nodes on (march / tile: 112^3 7.9 / 7.5, 130^3 10.2 / 9.5,
+//     160^3 13.5 / 11.6, 250 x 240 x 230 38.5 / 31.2), pairs from 8 M nodes
 //     on (201 x 181 x 163 28.9 / 33.1, with a source 36.9 / 39.0; 224^3 50.7 /
 //     49.1 and 62.1 / 57.8, 300 x 280 x 260 95.5 / 93.0 and 116 / 110); with a
 //     source affine in time the march stays (FP32 201 x 181 x 163 25.7 / 28.3,
 //     300 x 280 x 260 80.8 / 85.0).
 int star7_default_tile(const Star7Launch& a) {
     const long long cols = (long long)a.L.nx * a.L.ny, nodes = cols * a.L.nz;
-    const bool pairs = a.precision == SCAFES_PREC_F32X2, small = cols < 128LL * 128LL;
+    const bool pairs = a.precision == SCAFES_PREC_F32X2;
     const bool march = nodes < (1LL << 31);  // the march numbers nodes in 32 bits
     if (march && (a.precision == SCAFES_PREC_F64 || a.border == SCAFES_BORDER_TABLE || (pairs && a.fb)))
         return STAR7_MARCH;
-    if (a.L.nl != 1) return march && (a.fb || (pairs ? nodes < 8000000 : small)) ? STAR7_MARCH : STAR7_MULTI_LAYER_TILE;
-    if (a.precision == SCAFES_PREC_F64 || small) return 0;
+    if (a.L.nl != 1)
+        return march && (a.fb || nodes < (pairs ? 8000000 : 1200000)) ? STAR7_MARCH : STAR7_MULTI_LAYER_TILE;
+    if (a.precision == SCAFES_PREC_F64 || nodes < 700000) return 0;
     if (pairs && a.fa) return cols < 256LL * 256LL ? 1 : 2;
-    return 3;
+    return !pairs && a.fb && nodes < 2000000 ? 1 : 3;
 }
 
 cudaError_t launch_star7_f64(const Star7Launch& a, cudaStream_t stream);
@@ -123,12 +128,15 @@ cudaError_t launch_star7_loop_f32x2(const Star7Loop& q, cudaStream_t stream);
 // nodes (both measured, us per step, loop / default sweep; the loop reads its
 // neighbours through L1 only and falls behind where the sweep's pipes or HBM
 // are busy, while the grid barrier is the smaller share):
-//   FP64: 96^3 10.3 / 11.1, 112^3 15.4 / 15.4, 128^3 21.0 / 20.6, 201 x 181 x
-//     163 54 / 53, with a source 69.6 / 63.4; node coefficients 128^3 23.7 /
+//   FP64: 96^3 10.3 / 11.1, 112^3 16.0 / 15.3, 128^3 21.5 / 20.6, 136^3 24.7 /
+//     24.0, 144^3 29.2 / 27.0, 201 x 181 x 163 54 / 53, with a source 71 / 63, but
+//     fields that change sign, whose sums fall back to FP64 in both, 128^3 27.8 /
+//     31.2, 144^3 37.6 / 42.0; node coefficients 128^3 23.7 /
 //     26.8, 160 x 150 x 140 43.7 / 42.7; node rules and rule tables 201 x 181 x
 //     163 63 / 69 and 70 / 74 (256^3 270 / 226);
-//   FP32: 112^3 6.3 / 7.7, 128^3 8.3 / 6.8, 160^3 13.9 / 9.8, 250 x 240 x 230
-//     53.8 / 26.2; node coefficients 112^3 6.6 / 8.2, 128^3 8.6 / 8.1; with a
+//   FP32: 112^3 6.6 / 6.5, 128^3 8.7 / 6.8, 160^3 14.7 / 9.8, 250 x 240 x 230
+//     53.8 / 26.2; node coefficients 104^3 5.7 / 6.2, 112^3 6.6 / 6.5; several
+//     border layers 128^3 8.4 / 8.0, 136^3 9.9 / 10.0, 144^3 11.3 / 10.4; with a
 //     source affine in time 145^3 11.4 / 11.7, 160 x 150 x 140 12.5 / 11.2;
 //   pairs: 145^3 16.0 / 17.9, 160^3 20.7 / 19.1; with a source 160^3 22.9 / 24.2,
 //     180^3 no faster; with one affine in time 97^3 7.1 / 7.9, 112^3 10.5 / 10.4,
@@ -140,9 +148,12 @@ cudaError_t launch_star7_loop_f32x2(const Star7Loop& q, cudaStream_t stream);
 long long star7_loop_max_nodes(const Star7Launch& a) {
     const bool table = a.border == SCAFES_BORDER_TABLE, rules = a.border == SCAFES_BORDER_NODES;
     switch (a.precision) {
-        case SCAFES_PREC_F64: return table || rules ? 8000000 : a.vc ? 3000000 : 2000000;
+        case SCAFES_PREC_F64: return table || rules ? 8000000 : a.vc ? 3000000 : 2600000;
         case SCAFES_PREC_F32X2: return table ? 600000 : a.fb ? 1500000 : a.fa ? 4200000 : 3200000;
-        default: return table ? 600000 : rules ? 120000000 / ((a.fa ? 5 : 4) * 4) : a.fb ? 3000000 : 1500000;
+        default:
+            if (table) return 600000;
+            if (rules) return 120000000 / ((a.fa ? 5 : 4) * 4);
+            return a.fb ? 3000000 : a.L.nl != 1 ? 2600000 : 1500000;
     }
 }
 

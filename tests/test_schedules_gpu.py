@@ -98,7 +98,8 @@ def test_default_pair_ensemble_schedule_is_near_the_best(gpu, instances, side):
 @pytest.mark.parametrize("prec,source,layers,n", [
     ("f32x2", "affine", 1, (150, 140, 145)), ("f32x2", "affine", 1, (260, 258, 120)), ("f32x2", "static", 1, (140, 150, 145)),
     ("f32x2", "static", 2, (240, 230, 220)), ("f32", "none", 2, (224, 220, 200)), ("f32", "static", 2, (150, 140, 145)),
-    ("f32", "affine", 2, (201, 181, 163)), ("f32x2", "none", 2, (130, 129, 131))])
+    ("f32", "affine", 2, (201, 181, 163)), ("f32x2", "none", 2, (130, 129, 131)), ("f32", "none", 1, (100, 100, 300)),
+    ("f32", "none", 1, (130, 130, 5)), ("f32", "affine", 1, (200, 200, 20)), ("f32x2", "none", 1, (64, 64, 1000))])
 def test_default_sweep_is_near_the_best(gpu, prec, source, layers, n):
     M = gpu
 
