@@ -11,7 +11,7 @@
 // the border nodes are numbered separately, so a warp holds one kind and the
 // border rules (a chain of FP64 operations) run in full warps instead of in
 // one or two lanes of every warp at a face.  A step now takes 2.1, 2.7 and
-// 5.1 us on those three; of the 2.1 us of an almost empty step, most is the
+// 4.9 us on those three; of the 2.1 us of an almost empty step, most is the
 // round trips to L2 (neighbours, store and release, counter, acquire).  Two
 // warps per CTA and up to one CTA per SM: 1, 2 and 4 warps measure the same
 // within 2 %, 16 warps 20 % slower at 17 x 15 x 16.
@@ -36,21 +36,26 @@ constexpr uint32_t LOOP_MIN_WARPS = 2;
 // handles on several streams ran one after the other, each alone with its
 // barriers (12 loops at 64^3, us per step and handle: FP64 4.8, FP32 2.6,
 // pairs 3.0, where tile sweeps had taken 3.5, 1.6 and 1.8).  FP32 and pairs fit
-// 32 registers (at most 16 bytes spilled), FP64 48 (none); a loop by itself is
-// as fast (64^3 4.81 -> 4.76, 2.60 -> 2.56, 3.00 -> 2.94).  In FP64 two such CTAs fit
-// with 640 threads: 12 loops 4.8 -> 3.3, one 4.76 -> 5.05; from LOOP_FULL_NODES
-// nodes on a loop by itself needs all 1024 (80^3 7.3, 640 threads 8.0) and
-// several gain less.  Rule tables and node rules keep 64 registers: their
-// tile sweeps are slower than a loop that waits its turn (64^3 FP64 15.4, 5.6).
+// 32 registers (at most 16 bytes spilled) and 1.6 and 1.9 us, a loop by itself
+// is as fast (64^3 2.60 -> 2.56, 3.00 -> 2.94).  FP64 takes 48 registers (none
+// spilled), with which CTAs of up to LOOP_TWO_FIT threads go two to an SM.
+// Larger ones, below LOOP_FULL_NODES inner nodes: with a Dirichlet border and no
+// or a static source 32 registers (56 bytes spilled; 12 loops at 64^3 3.4, one
+// 4.81 -> 4.94), else at most LOOP_PAIR_THREADS (3.7, 5.3 -> 5.6; 32 registers
+// 4.0 and 5.7).  From there on a loop by itself needs all of both (80^3 7.3, 32
+// registers 7.6, 640 threads 8.0) and several gain less.  Rule tables and node
+// rules keep 64 registers: their tile sweeps are slower than a loop that waits
+// its turn (64^3 FP64 15.4, 5.6).
 template <class P, int BORDER>
 constexpr int loop_registers() {
     if (BORDER != SCAFES_BORDER_DIRICHLET && BORDER != SCAFES_BORDER_MIRROR_POW2) return 64;
     return std::is_same<P, PolF64>::value ? 48 : 32;
 }
-constexpr uint32_t LOOP_MAX_THREADS = 1024, LOOP_PAIR_THREADS = 640, LOOP_FULL_NODES = 320000;
+constexpr uint32_t LOOP_MAX_THREADS = 1024, LOOP_TWO_FIT = 672, LOOP_PAIR_THREADS = 640;
+constexpr uint32_t LOOP_FULL_NODES = 320000;
 
-template <class P, int SRC, int BORDER, bool VC>
-__global__ void __maxnreg__((loop_registers<P, BORDER>()))
+template <class P, int SRC, int BORDER, bool VC, int REGISTERS>
+__global__ void __maxnreg__(REGISTERS)
 star7_loop(const __grid_constant__ LoopArgs<typename P::T> A) {
     using T = typename P::T;
     constexpr bool HAS_F = SRC != SRC_NONE;
@@ -135,15 +140,25 @@ static cudaError_t launch_loop_typed(const Star7Loop& q, cudaStream_t stream) {
     A.in_cta = (A.o.n_inner + ctas - 1) / ctas;
     A.bd_cta = (A.o.n_border + ctas - 1) / ctas;
     const uint32_t want = ((A.in_cta + 31) / 32 + (A.bd_cta + 31) / 32) * 32;
-    const bool pair = loop_registers<P, BORDER>() == 48 && A.o.n_inner < LOOP_FULL_NODES;
-    const uint32_t most = pair ? LOOP_PAIR_THREADS : LOOP_MAX_THREADS;
-    const uint32_t rounds = (want + most - 1) / most;
-    const uint32_t threads = ((want / 32 + rounds - 1) / rounds) * 32;
+    auto threads_of = [&](uint32_t most) {
+        const uint32_t rounds = (want + most - 1) / most;
+        return ((want / 32 + rounds - 1) / rounds) * 32;
+    };
+    constexpr int REGISTERS = loop_registers<P, BORDER>();
+    auto kern = star7_loop<P, SRC, BORDER, VC, REGISTERS>;
+    uint32_t threads = threads_of(LOOP_MAX_THREADS);
+    if constexpr (REGISTERS == 48) {
+        if (threads > LOOP_TWO_FIT && A.o.n_inner < LOOP_FULL_NODES) {
+            if constexpr (BORDER == SCAFES_BORDER_DIRICHLET && SRC != SRC_AB && !VC)
+                kern = star7_loop<P, SRC, BORDER, VC, 32>;
+            else
+                threads = threads_of(LOOP_PAIR_THREADS);
+        }
+    }
     cudaError_t e = cudaMemsetAsync(q.arrivals, 0, sizeof(unsigned), stream);
     if (e != cudaSuccess) return e;
     void* args[] = {&A};
-    e = cudaLaunchCooperativeKernel((const void*)star7_loop<P, SRC, BORDER, VC>, dim3(ctas), dim3(threads), args, 0,
-                                    stream);
+    e = cudaLaunchCooperativeKernel((const void*)kern, dim3(ctas), dim3(threads), args, 0, stream);
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
