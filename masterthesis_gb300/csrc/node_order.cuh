@@ -96,10 +96,11 @@ constexpr int MARCH_THREADS = 256;
 // FP64 pays for every warp whatever its active lanes, and 32 columns at a
 // time leave up to a quarter of them idle (98 inner columns: 98 of 128), so
 // the width follows the grid: the (w, h) with the fewest idle threads, w
-// at most 64 and at least 16 where the grid has them, h at most 16 (sectors;
-// rows that share their y neighbours in L1; the halos that callers keep in
-// shared memory).  Launches call it, so the search is over the 49 widths,
-// whatever the grid's.
+// at most 64, no more tiles than ceil(columns / 16) (so w is at least 9 where
+// the grid has them; 31 x 14 x 21 FP64 Lame takes 5 % longer with tiles of 29
+// columns than of 15), h at most 16 (sectors; rows that share their y
+// neighbours in L1; the halos that callers keep in shared memory).  Launches
+// call it, so the search is over the widths, whatever the grid's.
 struct ColumnTile {
     FastDiv w;
     int h, nx, ny;  // rows of threads; tiles along x and y
@@ -110,11 +111,11 @@ inline ColumnTile make_column_tile(int ix, int iy, int rows) {
     if (ix <= 0 || iy <= 0) return t;
     long long best = 0;
     const int ty = (iy + rows - 1) / rows;  // rows of threads
-    const int least = ix < 16 ? ix : 16;
     int last = 0;
-    for (int k = ix < 64 ? ix : 64; k >= least; --k) {
+    for (int k = ix < 64 ? ix : 64; k > 0; --k) {
         const int n = (ix + k - 1) / k, w = (ix + n - 1) / n;
-        if (n == last || w < least) continue;
+        if (n > (ix + 15) / 16) break;
+        if (n == last) continue;
         last = n;
         const int h = MARCH_THREADS / w < 16 ? MARCH_THREADS / w : 16, m = (ty + h - 1) / h;
         const long long threads = (long long)n * m * MARCH_THREADS;

@@ -14,7 +14,7 @@ static bool check(int ix, int iy, int rows) {
     const bool limits = w >= 1 && w <= 64 && t.h >= 1 && t.h <= 16 && w * t.h <= scafes::MARCH_THREADS;
     const bool cover = (long long)t.nx * w >= ix && (long long)(t.nx - 1) * w < ix && (long long)t.ny * t.h >= ty &&
                        (long long)(t.ny - 1) * t.h < ty;
-    const bool wide = w >= 16 || w == ix;
+    const bool wide = w >= 9 || w == ix;
     if (!(limits && cover && wide)) std::printf("%d x %d, %d rows: w %d h %d, %d x %d tiles\n", ix, iy, rows, w, t.h, t.nx, t.ny);
     return limits && cover && wide;
 }
